@@ -173,6 +173,76 @@ struct Entry {
     double W[9];
 };
 
+// The ELL entries by tensor id (ell_ntensor > 0): a lattice of cells repeats a
+// few coupling tensors, so an entry is 4 bytes (24-bit column, 8-bit id) where
+// the general form holds 76, and the tensors sit in shared memory.  Taken when
+// the matrix has at most kEllMaxTensors distinct tensors and its site indices
+// fit 24 bits; `done` is false otherwise.  `merged` is sorted by (row, column).
+// The isotropic tensors (one number times the unit matrix) follow the others
+// in slots of their own, so that a warp takes one branch per slot.
+mj_status make_ell_by_id(mj_plan* p, const std::vector<Entry>& merged, bool& done) {
+    done = false;
+    const int64_t N = p->N;
+    if (N > kEllMaxSites || merged.empty()) return MJ_OK;
+    struct Tensor {
+        double W[9];
+        bool iso;
+    };
+    std::vector<Tensor> tab;
+    std::vector<uint8_t> id(merged.size());
+    int last = 0;  // neighbouring rows repeat ids in turn: look from the last match on
+    for (size_t k = 0; k < merged.size(); ++k) {
+        const double* W = merged[k].W;
+        int t = -1;
+        for (size_t q = 0; q < tab.size() && t < 0; ++q) {
+            const int c = (last + static_cast<int>(q)) % static_cast<int>(tab.size());
+            if (std::memcmp(tab[c].W, W, sizeof(tab[c].W)) == 0) t = c;
+        }
+        if (t < 0) {
+            if (tab.size() == static_cast<size_t>(kEllMaxTensors)) return MJ_OK;
+            Tensor n;
+            std::memcpy(n.W, W, sizeof(n.W));
+            n.iso = W[0] == W[4] && W[0] == W[8];
+            for (int q = 0; q < 9; ++q) n.iso = n.iso && (q % 4 == 0 || W[q] == 0.0);
+            t = static_cast<int>(tab.size());
+            tab.push_back(n);
+        }
+        id[k] = static_cast<uint8_t>(t);
+        last = t + 1 < static_cast<int>(tab.size()) ? t + 1 : 0;
+    }
+    std::vector<int> nfull(N, 0), niso(N, 0);
+    int wfull = 0, wiso = 0;
+    for (size_t k = 0; k < merged.size(); ++k) {
+        if (tab[id[k]].iso) wiso = std::max(wiso, ++niso[merged[k].row]);
+        else wfull = std::max(wfull, ++nfull[merged[k].row]);
+    }
+    const int width = wfull + wiso;
+    std::vector<uint32_t> ent(static_cast<size_t>(width) * N, kEllEmpty);
+    std::fill(nfull.begin(), nfull.end(), 0);
+    std::fill(niso.begin(), niso.end(), wfull);
+    for (size_t k = 0; k < merged.size(); ++k) {
+        const int slot = tab[id[k]].iso ? niso[merged[k].row]++ : nfull[merged[k].row]++;
+        ent[static_cast<size_t>(slot) * N + merged[k].row] =
+            static_cast<uint32_t>(merged[k].col) | (static_cast<uint32_t>(id[k]) << 24);
+    }
+    std::vector<double> flat(9 * tab.size());
+    for (size_t t = 0; t < tab.size(); ++t) std::memcpy(&flat[9 * t], tab[t].W, sizeof(tab[t].W));
+    p->ell_width = width;
+    p->ell_wfull = wfull;
+    mj_status st;
+    if ((st = dalloc(&p->d_ell_ent, ent.size(), "ell entries")) != MJ_OK) return st;
+    if ((st = dalloc(&p->d_ell_tab, flat.size(), "ell tensors")) != MJ_OK) return st;
+    if ((st = cuda_status(cudaMemcpy(p->d_ell_ent, ent.data(), ent.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+                          "ell entries upload")) != MJ_OK)
+        return st;
+    if ((st = cuda_status(cudaMemcpy(p->d_ell_tab, flat.data(), flat.size() * sizeof(double), cudaMemcpyHostToDevice),
+                          "ell tensors upload")) != MJ_OK)
+        return st;
+    p->ell_ntensor = static_cast<int>(tab.size());
+    done = true;
+    return MJ_OK;
+}
+
 // Per-site tensor lists (ELL) from (row site, col site, H block) triplets:
 // B_s = -sum_t (H_st + H_ts^T) m_t.
 mj_status make_ell(mj_plan* p, std::vector<Entry>& ent) {
@@ -188,6 +258,9 @@ mj_status make_ell(mj_plan* p, std::vector<Entry>& ent) {
         }
     }
     const int64_t N = p->N;
+    mj_status st;
+    bool done = false;
+    if ((st = make_ell_by_id(p, merged, done)) != MJ_OK || done) return st;
     std::vector<int> count(N, 0);
     for (const Entry& e : merged) ++count[e.row];
     int width = 0;
@@ -201,7 +274,6 @@ mj_status make_ell(mj_plan* p, std::vector<Entry>& ent) {
         col[static_cast<size_t>(k) * N + e.row] = static_cast<int>(e.col);
         for (int q = 0; q < 9; ++q) val[(static_cast<size_t>(k) * 9 + q) * N + e.row] = e.W[q];
     }
-    mj_status st;
     if ((st = dalloc(&p->d_ell_col, col.size(), "ell col")) != MJ_OK) return st;
     if ((st = dalloc(&p->d_ell_val, val.size(), "ell val")) != MJ_OK) return st;
     if (!col.empty()) {
@@ -304,6 +376,8 @@ void free_plan(mj_plan* p) {
     cudaFree(p->d_stepctr);
     cudaFree(p->d_ell_col);
     cudaFree(p->d_ell_val);
+    cudaFree(p->d_ell_ent);
+    cudaFree(p->d_ell_tab);
     cudaFree(p->d_zee);
     cudaFree(p->d_bmap);
     cudaFree(p->d_mid);

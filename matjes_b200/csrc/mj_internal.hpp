@@ -61,6 +61,12 @@ struct StencilParams {
     int shape;                // mj_shapes.hpp ShapeId; W is then in the shape's offset order
 };
 
+// ELL entries by tensor id (mj_plan): at most this many distinct tensors, on
+// lattices whose site index fits 24 bits.
+constexpr int kEllMaxTensors = 128;
+constexpr int64_t kEllMaxSites = int64_t{1} << 24;
+constexpr uint32_t kEllEmpty = 0xffffffffu;
+
 // Dipolar H on the padded FFT grid (the unpack is fused into the consumers):
 // component c of site (x,y,z) is h[c*cs + x + px*y + zs*z].
 struct DipView {
@@ -129,6 +135,13 @@ struct mj_plan {
     int ell_width = 0;
     int* d_ell_col = nullptr;        // [width][N], -1 = empty
     double* d_ell_val = nullptr;     // [width][9][N]
+    // the same entries by tensor id when the matrix holds few distinct tensors:
+    // col | id << 24 per entry (kEllEmpty = none), slots [0, ell_wfull) full
+    // tensors, the rest isotropic ones; d_ell_col / d_ell_val are then not built
+    int ell_ntensor = 0;             // distinct tensors (0: the form above)
+    int ell_wfull = 0;
+    uint32_t* d_ell_ent = nullptr;   // [width][N]
+    double* d_ell_tab = nullptr;     // [ntensor][9]
     double* d_zee = nullptr;         // per-site Zeeman coefficient zc (ELL)
     // applied field map (SoA per cell) or null for uniform
     double* d_bmap = nullptr;
