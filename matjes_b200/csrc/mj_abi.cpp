@@ -398,6 +398,7 @@ void free_plan(mj_plan* p) {
     cudaFree(p->d_unit);
     cudaFree(p->d_vjp_part);
     cudaFree(p->d_vjp_counter);
+    p->gneb.release();
     delete p;
 }
 

@@ -56,6 +56,7 @@ struct BatchArgs {
     double* tile_g;     // GNEB pass: per-tile path sums (6 x ntile)
     int64_t gneb_n;     // GNEB pass: sites of an image (every replica one image)
     int gneb_nimg;      // GNEB pass: images
+    const int* stop;    // GNEB pass: the launch does nothing when this flag is set (may be null)
 };
 
 // BPASS_GNEB: the projected field pass with, per tile, the sums a GNEB iteration
@@ -231,6 +232,8 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_batch(const __grid_constant_
     // per tile: the energy, and for the GNEB pass its six path sums
     constexpr int NV = PASS == BPASS_GNEB ? 7 : 1;
     __shared__ double wsum[NV][8];
+    if constexpr (PASS == BPASS_GNEB)
+        if (A.stop && *A.stop) return;
     BatchArgs Ar = A;
     if (C.step_base) Ar.step = A.step + *C.step_base;
     const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -450,8 +453,7 @@ struct BatchLauncher {
         k_batch<S, BYT, RY, MINB, PASS, SP><<<nblocks, dim3(32, BYT), G::buf_bytes, s>>>(P, C, A);
         return cuda_status(cudaGetLastError(), "k_batch");
     }
-    // the dynamics and energy passes in the axial form where it holds; the
-    // field and GNEB passes in the full form
+    // the axial form where it holds; the plain field pass in the full form
     static mj_status pass(int ps, bool axial, const StencilParams& P, const DynCoef& C, const BatchArgs& A,
                           int nblocks, cudaStream_t s) {
         switch (ps) {
@@ -462,7 +464,9 @@ struct BatchLauncher {
                 return axial ? launch<BPASS_SIB2, SP_AXIAL>(P, C, A, nblocks, s)
                              : launch<BPASS_SIB2, SP_FULL>(P, C, A, nblocks, s);
             case BPASS_FIELD: return launch<BPASS_FIELD, SP_FULL>(P, C, A, nblocks, s);
-            case BPASS_GNEB: return launch<BPASS_GNEB, SP_FULL>(P, C, A, nblocks, s);
+            case BPASS_GNEB:
+                return axial ? launch<BPASS_GNEB, SP_AXIAL>(P, C, A, nblocks, s)
+                             : launch<BPASS_GNEB, SP_FULL>(P, C, A, nblocks, s);
             default:
                 return axial ? launch<BPASS_ENERGY, SP_AXIAL>(P, C, A, nblocks, s)
                              : launch<BPASS_ENERGY, SP_FULL>(P, C, A, nblocks, s);
@@ -530,6 +534,8 @@ struct mj_batch {
     int* d_accept = nullptr;
     uint32_t* d_stepctr = nullptr;
     double* d_stage = nullptr;
+    mj::GnebWork gneb;                // mj_batch_gneb_path
+    double* d_tile_g = nullptr;       // its path sums (6 per tile)
     double* d_gneb_part = nullptr;    // tangent norms: one partial per (image, block)
     // Monte Carlo: the colouring, its MC tile list, per-replica chain state
     int mc_col[4] = {0, 0, 0, 0};
@@ -565,6 +571,8 @@ void batch_free(mj_batch* b) {
     cudaFree(b->d_stepctr);
     cudaFree(b->d_stage);
     cudaFree(b->d_gneb_part);
+    cudaFree(b->d_tile_g);
+    b->gneb.release();
     cudaFree(b->d_mc_tiles);
     cudaFree(b->d_mc_acc);
     cudaFree(b->d_mc_prop);
@@ -587,8 +595,10 @@ mj_status batch_tiles(mj_batch* b, bool upload_reps) {
     b->ntile = static_cast<int>(tiles.size());
     cudaFree(b->d_tiles);
     cudaFree(b->d_tile_e);
+    cudaFree(b->d_tile_g);
     b->d_tiles = nullptr;
     b->d_tile_e = nullptr;
+    b->d_tile_g = nullptr;
     mj_status st;
     if ((st = cuda_status(cudaMalloc(&b->d_tiles, sizeof(int4) * tiles.size()), "batch tiles")) != MJ_OK) return st;
     if ((st = cuda_status(cudaMalloc(&b->d_tile_e, sizeof(double) * tiles.size()), "batch tile energies")) != MJ_OK)
@@ -660,6 +670,7 @@ BatchArgs batch_args(mj_batch* b, uint32_t step, double dt) {
     A.tile_g = nullptr;
     A.gneb_n = 0;
     A.gneb_nimg = 0;
+    A.stop = nullptr;
     return A;
 }
 
@@ -728,6 +739,7 @@ struct BatchFields {
         A.tile_g = tile_g;
         A.gneb_n = b->Ntot / b->nrep;
         A.gneb_nimg = b->nrep;
+        A.stop = &ctl->done;
         mj_status e = batch_pass(b->shape, b->variant, BPASS_GNEB, b->zaxial, b->sp, c, A, batch_blocks(b), s);
         if (e != MJ_OK) return e;
         k_gneb_img<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, tile_g, b->ntile, E, img, ctl);
@@ -1240,13 +1252,15 @@ mj_status mj_batch_gneb_path(mj_batch* b, const mj_gneb_params* p, double* rx, d
         return st;
     BatchFields fl{b, b->cap_stream, nullptr, DynCoef{}};
     std::memset(&fl.c, 0, sizeof(fl.c));
-    if ((st = cuda_status(cudaMalloc(&fl.tile_g, sizeof(double) * 6 * b->ntile), "GNEB buffers")) != MJ_OK) return st;
+    if (!b->d_tile_g &&
+        (st = cuda_status(cudaMalloc(&b->d_tile_g, sizeof(double) * 6 * b->ntile), "GNEB buffers")) != MJ_OK)
+        return st;
+    fl.tile_g = b->d_tile_g;
     // the path as the work queued on the legacy default stream (an upload) leaves it
     st = cuda_status(cudaStreamSynchronize(0), "GNEB start");
     if (st == MJ_OK)
-        st = gneb_relax(fl, b->d_m, nrep, GnebIdx{n, n, Ntot}, b->num_sms, b->cap_stream, p, 32, rx, ene, dene,
+        st = gneb_relax(fl, b->gneb, b->d_m, nrep, GnebIdx{n, n, Ntot}, b->num_sms, b->cap_stream, p, 32, rx, ene, dene,
                         iterations, max_force, climbing);
-    cudaFree(fl.tile_g);
     return st;
 }
 

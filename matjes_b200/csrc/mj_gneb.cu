@@ -129,7 +129,7 @@ struct PlanFields {
     // the projection and the tiles' path sums, then the sums of every image
     mj_status gneb_tiled(double* F, const double* m, double* E, double* img, const GnebCtl* ctl) {
         const int rec = prof_begin(p, "k_gneb_images", s);
-        mj_status e = launch_gneb_images(p, m, F, part, nrep, &tiles, s);
+        mj_status e = launch_gneb_images(p, m, F, part, nrep, &tiles, ctl ? &ctl->done : nullptr, s);
         prof_end(p, rec, s);
         if (e != MJ_OK) return e;
         k_gneb_tile_sums<<<nrep, 7 * 32, 0, s>>>(part, static_cast<int>(tiles), tiles * nrep, nrep, img, E, ctl);
@@ -189,7 +189,7 @@ mj_status mj_gneb_path(mj_plan* plan, double* m, int32_t nimg, const mj_gneb_par
     const bool prof = plan->prof_on;
     plan->prof_on = false;
     if (st == MJ_OK)
-        st = gneb_relax(fl, m, nimg, fl.X, plan->num_sms, s, p, 32, rx, ene, dene, iterations, max_force, climbing);
+        st = gneb_relax(fl, plan->gneb, m, nimg, fl.X, plan->num_sms, s, p, 32, rx, ene, dene, iterations, max_force, climbing);
     plan->prof_on = prof;
     const mj_status fin = cuda_status(cudaStreamSynchronize(s), "GNEB end");
     if (st == MJ_OK) st = fin;

@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(256) k_gneb_project(double* F, const double* _
 }
 
 // Iteration state on the device: done set by the iteration that stopped (max |F|
-// < ftol or itrmax reached; the iterations after it in a graph do no work but
-// the field pass); the iterations taken.
+// < ftol or itrmax reached; the iterations queued after it do no work); the
+// iterations taken.
 struct GnebCtl {
     int done;
     int pad;
@@ -466,11 +466,38 @@ __global__ void __launch_bounds__(256) k_gneb_move(const double* __restrict__ m,
     st3(mn, i, X.cs, v);
 }
 
+// Working memory above this size is given back at the end of a call.
+constexpr size_t kGnebKeepBytes = size_t{256} << 20;
+
+// W with at least these many device and pinned bytes and its events (the calls
+// that use it are synchronous: nothing of an earlier one is in flight).
+inline mj_status gneb_reserve(GnebWork& W, size_t dev_bytes, size_t host_bytes) {
+    mj_status st = MJ_OK;
+    if (W.dev_bytes < dev_bytes) {
+        cudaFree(W.dev);
+        W.dev = nullptr;
+        W.dev_bytes = 0;
+        if ((st = cuda_status(cudaMalloc(&W.dev, dev_bytes), "GNEB buffers")) != MJ_OK) return st;
+        W.dev_bytes = dev_bytes;
+    }
+    if (W.host_bytes < host_bytes) {
+        cudaFreeHost(W.host);
+        W.host = nullptr;
+        W.host_bytes = 0;
+        if ((st = cuda_status(cudaMallocHost(&W.host, host_bytes), "GNEB buffers")) != MJ_OK) return st;
+        W.host_bytes = host_bytes;
+    }
+    for (cudaEvent_t& e : W.ev)
+        if (!e && (st = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "GNEB events")) != MJ_OK)
+            return st;
+    return MJ_OK;
+}
+
 // The relaxation of the path in m (nrep images, X) by find_path; the field of
-// the images comes from fl (see the header).  The path is left in m.  chunk:
-// iterations per graph replay (even).
+// the images comes from fl (see the header), the working memory from W.  The
+// path is left in m.  chunk: iterations between looks at the stop flag (even).
 template <class Fields>
-mj_status gneb_relax(Fields& fl, double* m, int nrep, GnebIdx X, int num_sms, cudaStream_t s, const mj_gneb_params* p,
+mj_status gneb_relax(Fields& fl, GnebWork& W, double* m, int nrep, GnebIdx X, int num_sms, cudaStream_t s, const mj_gneb_params* p,
                      int chunk, double* rx, double* ene, double* dene, int64_t* iterations, double* max_force,
                      int32_t* climbing) {
     const double spring = p->spring, dt = p->dt, mass = p->mass, ftol = p->ftol;
@@ -486,47 +513,43 @@ mj_status gneb_relax(Fields& fl, double* m, int nrep, GnebIdx X, int num_sms, cu
     // each, the layout of m); E, pl, fp per image, img the iteration's six path
     // sums per image, scal (v.F, F.F, max |F|, lam); part / part2 block
     // partials; cnt the last-block counters; ctl the stop flag
-    double *F1 = nullptr, *F2 = nullptr, *mB = nullptr, *tau = nullptr, *E = nullptr, *part = nullptr,
-           *part2 = nullptr;
-    unsigned int* cnt = nullptr;
-    GnebCtl* ctl = nullptr;
-    GnebCtl* hctl = nullptr;
-    cudaEvent_t ev[2] = {nullptr, nullptr};
+    const size_t nE = 9 * static_cast<size_t>(nrep) + 4;
+    size_t dev_bytes = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = dev_bytes;
+        dev_bytes += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t f3 = sizeof(double) * 3 * static_cast<size_t>(Ntot);
+    const size_t oF1 = take(f3), oF2 = take(f3), omB = take(f3), otau = take(f3), oE = take(sizeof(double) * nE),
+                 opart = take(sizeof(double) * 6 * nbv), opart2 = take(sizeof(double) * std::max(3 * nbv, n3b)),
+                 ocnt = take(sizeof(unsigned int) * (nrep + 1)), octl = take(sizeof(GnebCtl));
+    mj_status st = gneb_reserve(W, dev_bytes, 2 * sizeof(GnebCtl) + sizeof(double) * nE);
+    if (st != MJ_OK) return st;
+    char* base = static_cast<char*>(W.dev);
+    auto at = [&](size_t o) { return reinterpret_cast<double*>(base + o); };
+    double *F1 = at(oF1), *F2 = at(oF2), *mB = at(omB), *tau = at(otau), *E = at(oE), *part = at(opart),
+           *part2 = at(opart2);
+    unsigned int* cnt = reinterpret_cast<unsigned int*>(base + ocnt);
+    GnebCtl* ctl = reinterpret_cast<GnebCtl*>(base + octl);
+    GnebCtl* hctl = static_cast<GnebCtl*>(W.host);
+    double* hE = reinterpret_cast<double*>(hctl + 2);  // the host copy of E .. scal
     cudaGraphExec_t exec = nullptr;
-    mj_status st = MJ_OK;
-    double** bufs[] = {&F1, &F2, &mB, &tau};
-    for (double** q : bufs)
-        if (st == MJ_OK) st = cuda_status(cudaMalloc(q, sizeof(double) * 3 * Ntot), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMalloc(&E, sizeof(double) * (9 * nrep + 4)), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMalloc(&part, sizeof(double) * 6 * nbv), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMalloc(&part2, sizeof(double) * std::max(3 * nbv, n3b)), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMalloc(&cnt, sizeof(unsigned int) * (nrep + 1)), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMalloc(&ctl, sizeof(GnebCtl)), "GNEB buffers");
-    if (st == MJ_OK) st = cuda_status(cudaMallocHost(&hctl, 2 * sizeof(GnebCtl)), "GNEB buffers");
-    for (int q = 0; q < 2 && st == MJ_OK; ++q)
-        st = cuda_status(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming), "GNEB events");
     auto release = [&]() {
         if (exec) cudaGraphExecDestroy(exec);
-        for (cudaEvent_t e : ev)
-            if (e) cudaEventDestroy(e);
-        cudaFreeHost(hctl);
-        for (double* b : {F1, F2, mB, tau, E, part, part2}) cudaFree(b);
-        cudaFree(cnt);
-        cudaFree(ctl);
+        if (W.dev_bytes > kGnebKeepBytes) {
+            cudaFree(W.dev);
+            W.dev = nullptr;
+            W.dev_bytes = 0;
+        }
     };
-    if (st != MJ_OK) {
-        release();
-        return st;
-    }
     double* pl = E + nrep;
     double* fp = E + 2 * nrep;
     double* img = E + 3 * nrep;
     double* scal = E + 9 * nrep;
-    GnebCtl c0;
-    std::memset(&c0, 0, sizeof(c0));
     cudaMemsetAsync(scal, 0, sizeof(double) * 4, s);
     cudaMemsetAsync(cnt, 0, sizeof(unsigned int) * (nrep + 1), s);
-    cudaMemcpyAsync(ctl, &c0, sizeof(c0), cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(ctl, 0, sizeof(GnebCtl), s);
     const dim3 gi(nblk, nrep), gs(nblk, nrep - 1);
     // field, path length pl, tangents of the given mode, fp = F.tau per image
     auto forces = [&](double* F, int mode) -> mj_status {
@@ -550,40 +573,38 @@ mj_status gneb_relax(Fields& fl, double* m, int nrep, GnebIdx X, int num_sms, cu
     k_gneb_force<<<gi, 256, 0, s>>>(F1, tau, fp, pl, E, X, nrep, spring, 1, climb);
     k_gneb_absmax<<<n3b, 256, 0, s>>>(F1, 3 * Ntot, part2);
     k_gneb_maxof<<<1, 256, 0, s>>>(part2, n3b, scal + 2);
-    double h0[4];
-    cudaMemcpyAsync(h0, E, sizeof(double), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h0 + 1, E + nrep - 1, sizeof(double), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h0 + 2, scal + 2, sizeof(double), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hE, E, sizeof(double) * nE, cudaMemcpyDeviceToHost, s);
     if ((st = cuda_status(cudaStreamSynchronize(s), "GNEB initial forces")) != MJ_OK) {
         release();
         return st;
     }
-    const double E_first = h0[0], E_last = h0[1];
-    double fchk = h0[2];
+    const double E_first = hE[0], E_last = hE[nrep - 1];
+    double fchk = hE[9 * nrep + 2];
     int64_t done = 0;
     if (itrmax > 0) {
-        // the first move (lam = 0: the velocity starts at zero) into mB, then
-        // chunks of iterations replayed as one graph: the field with the path
-        // sums, k_gneb_step, k_gneb_move.  Forces and spins alternate between
-        // their two buffers (an even chunk starts each replay on F1 and mB).  Two
-        // chunks are in flight: the stop flag of one is read while the next
-        // runs; the iterations after the stop do no work but the field.
+        // the first move (lam = 0: the velocity starts at zero) into mB, then the
+        // iterations: the field with the path sums, k_gneb_step, k_gneb_move.
+        // Forces and spins alternate between their two buffers (an even chunk
+        // starts on F1 and mB).  Two chunks are in flight: the stop flag of one
+        // is read while the next runs; after the stop every kernel returns at
+        // once, and no iteration past itrmax is queued.  A run of more than four
+        // chunks replays a chunk as one graph; a shorter one launches its
+        // kernels directly (capturing and instantiating the graph queues as many
+        // launches as the chunk has).  40 iterations of 256^2 x 16 images: 3.7 ms
+        // a call, 8.8 to 12.3 ms with the graph, every buffer allocated per call
+        // and two chunks always queued.
         // Four sites per thread once that still gives two blocks per SM: the
         // loads of four sites in flight before each block's reduction.
         const bool spt4 = Ntot >= 2LL * 1024 * num_sms;
         const dim3 gt(nrep, static_cast<unsigned>(spt4 ? (n + 1023) / 1024 : nblk));
-        k_gneb_move<<<gi, 256, 0, s>>>(m, mB, F1, scal, ctl, X, nrep, dt, mass);
-        st = cuda_status(cudaGetLastError(), "k_gneb_move");
-        if (st == MJ_OK) st = cuda_status(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
-        if (st == MJ_OK) {
-            mj_status inner = MJ_OK;
-            for (int k = 0; k < chunk && inner == MJ_OK; ++k) {
+        auto iterations_from = [&](int count) -> mj_status {  // starting on F1 and mB
+            for (int k = 0; k < count; ++k) {
                 double* Fo = (k & 1) ? F2 : F1;
                 double* Fn = (k & 1) ? F1 : F2;
                 double* mc = (k & 1) ? m : mB;
                 double* mo = (k & 1) ? mB : m;
-                inner = fl.iterate(Fn, mc, E, img, ctl);
-                if (inner != MJ_OK) break;
+                const mj_status e = fl.iterate(Fn, mc, E, img, ctl);
+                if (e != MJ_OK) return e;
                 const long long im = static_cast<long long>(itrmax);
                 if (spt4)
                     k_gneb_step<4><<<gt, 256, 0, s>>>(mc, mo, Fo, Fn, E, img, X, nrep, spring, dt, mass, ftol, im, climb,
@@ -592,34 +613,47 @@ mj_status gneb_relax(Fields& fl, double* m, int nrep, GnebIdx X, int num_sms, cu
                     k_gneb_step<1><<<gt, 256, 0, s>>>(mc, mo, Fo, Fn, E, img, X, nrep, spring, dt, mass, ftol, im, climb,
                                                       part2, part2 + 2 * nbv, cnt + nrep, ctl, scal);
                 k_gneb_move<<<gi, 256, 0, s>>>(mc, mo, Fn, scal, ctl, X, nrep, dt, mass);
-                inner = cuda_status(cudaGetLastError(), "GNEB iteration");
+                const mj_status l = cuda_status(cudaGetLastError(), "GNEB iteration");
+                if (l != MJ_OK) return l;
             }
-            cudaGraph_t graph = nullptr;
-            const cudaError_t e = cudaStreamEndCapture(s, &graph);
-            if (inner != MJ_OK) st = inner;
-            else if ((st = cuda_status(e, "end capture")) == MJ_OK)
-                st = cuda_status(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
-            if (graph) cudaGraphDestroy(graph);
+            return MJ_OK;
+        };
+        k_gneb_move<<<gi, 256, 0, s>>>(m, mB, F1, scal, ctl, X, nrep, dt, mass);
+        st = cuda_status(cudaGetLastError(), "k_gneb_move");
+        if (st == MJ_OK && itrmax > 4 * static_cast<int64_t>(chunk)) {
+            st = cuda_status(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
+            if (st == MJ_OK) {
+                const mj_status inner = iterations_from(chunk);
+                cudaGraph_t graph = nullptr;
+                const cudaError_t e = cudaStreamEndCapture(s, &graph);
+                if (inner != MJ_OK) st = inner;
+                else if ((st = cuda_status(e, "end capture")) == MJ_OK)
+                    st = cuda_status(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
+                if (graph) cudaGraphDestroy(graph);
+            }
         }
-        // chunk q: replay, its flag into hctl[q & 1], event ev[q & 1]
+        const int64_t nchunk = (itrmax - 1) / chunk + 1;
+        // chunk q: queued, its flag into hctl[q & 1], event ev[q & 1]
         auto launch = [&](int64_t q) -> mj_status {
-            mj_status e = cuda_status(cudaGraphLaunch(exec, s), "GNEB graph launch");
+            const int64_t left = itrmax - q * chunk;
+            const mj_status e = exec && left >= chunk ? cuda_status(cudaGraphLaunch(exec, s), "GNEB graph launch")
+                                                      : iterations_from(static_cast<int>(std::min<int64_t>(left, chunk)));
             if (e != MJ_OK) return e;
             cudaMemcpyAsync(hctl + (q & 1), ctl, sizeof(GnebCtl), cudaMemcpyDeviceToHost, s);
-            return cuda_status(cudaEventRecord(ev[q & 1], s), "GNEB event");
+            return cuda_status(cudaEventRecord(W.ev[q & 1], s), "GNEB event");
         };
         if (st == MJ_OK) st = launch(0);
-        if (st == MJ_OK) st = launch(1);
+        if (st == MJ_OK && nchunk > 1) st = launch(1);
         for (int64_t q = 0; st == MJ_OK; ++q) {
-            if ((st = cuda_status(cudaEventSynchronize(ev[q & 1]), "GNEB iterations")) != MJ_OK) break;
+            if ((st = cuda_status(cudaEventSynchronize(W.ev[q & 1]), "GNEB iterations")) != MJ_OK) break;
             const GnebCtl hc = hctl[q & 1];
             done = hc.iters;
             if (hc.done) break;
-            if (hc.iters != (q + 1) * chunk) {
+            if (hc.iters != (q + 1) * chunk || q + 1 >= nchunk) {
                 st = set_error(MJ_ERR_CUDA, "GNEB iterations did not advance");
                 break;
             }
-            st = launch(q + 2);
+            if (q + 2 < nchunk) st = launch(q + 2);
         }
         // the chunk still in flight (or, after an error, all queued work) ends first
         const mj_status fin = cuda_status(cudaStreamSynchronize(s), "GNEB iterations");
@@ -627,22 +661,19 @@ mj_status gneb_relax(Fields& fl, double* m, int nrep, GnebIdx X, int num_sms, cu
         // the relaxed path is in mB after an odd number of iterations
         if (st == MJ_OK && (done & 1))
             cudaMemcpyAsync(m, mB, sizeof(double) * 3 * Ntot, cudaMemcpyDeviceToDevice, s);
-        if (st == MJ_OK) {
-            cudaMemcpyAsync(&fchk, scal + 2, sizeof(double), cudaMemcpyDeviceToHost, s);
-            st = cuda_status(cudaStreamSynchronize(s), "GNEB force");
-        }
     }
     // outputs (en_path.out): path length, energy above the reference image, and the
     // derivative along the path -F.tau of the final images' projected fields along
     // the simple tangent (lattice_single); the end images' forces are zero after a
     // move, their projected fields before any
-    std::vector<double> h(3 * nrep);
     if (st == MJ_OK) st = forces(F2, 1);
     if (st == MJ_OK) {
-        cudaMemcpyAsync(h.data(), E, sizeof(double) * 3 * nrep, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(hE, E, sizeof(double) * nE, cudaMemcpyDeviceToHost, s);
         st = cuda_status(cudaStreamSynchronize(s), "GNEB outputs");
     }
     if (st == MJ_OK) {
+        const double* h = hE;
+        if (done > 0) fchk = hE[9 * nrep + 2];
         const double eref = en_zero == 'I' ? E_first : (en_zero == 'F' ? E_last : 0.0);
         auto en = [&](int r) { return r == 0 ? E_first : (r == nrep - 1 ? E_last : h[r]); };
         for (int r = 0; r < nrep; ++r) {

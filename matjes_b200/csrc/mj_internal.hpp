@@ -113,6 +113,28 @@ void build_noise_tables(double* tab);
 
 }  // namespace mj
 
+namespace mj {
+// The working memory of a GNEB relaxation (mj_gneb.cuh), kept by the plan or
+// batch between calls: one device block, one pinned block, two events.
+struct GnebWork {
+    void* dev = nullptr;
+    size_t dev_bytes = 0;
+    void* host = nullptr;
+    size_t host_bytes = 0;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    void release() {
+        cudaFree(dev);
+        cudaFreeHost(host);
+        for (cudaEvent_t& e : ev) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        dev = host = nullptr;
+        dev_bytes = host_bytes = 0;
+    }
+};
+}  // namespace mj
+
 struct mj_plan {
     int device = 0;
     int64_t N = 0;        // spin sites
@@ -184,6 +206,7 @@ struct mj_plan {
     // into the padded grid, which then holds dip_pad_holds (null: unknown)
     bool dip_fuse_pad = false;
     const double* dip_pad_holds = nullptr;
+    mj::GnebWork gneb;        // mj_gneb_path
     int smem_cap_bytes = 0;   // the dynamic shared memory per block that makes the cap
     // per-kernel event timing (mj_profile_enable / mj_profile_read)
     bool prof_on = false;
@@ -280,11 +303,12 @@ MJ_FUSED_SHAPE_DECL(launch_sib_fused_tri3)
 // The GNEB images of a path on a tiled plan without the dipolar term: the
 // projected field into F and per tile the six path sums and the energy
 // (partials[q nblocks + tile], tiles image-major, *tiles_per_image of them).
+// stop (a device flag, may be null): the launch does nothing when it is set.
 mj_status launch_gneb_images(mj_plan* p, const double* m, double* F, double* partials, int nimg,
-                             int64_t* tiles_per_image, cudaStream_t s);
+                             int64_t* tiles_per_image, const int* stop, cudaStream_t s);
 #define MJ_GNEB_SHAPE_DECL(name)                                                                       \
     mj_status name(mj_plan* p, const double* m, double* F, double* partials, int nimg, int64_t* tiles, \
-                   cudaStream_t s);
+                   const int* stop, cudaStream_t s);
 MJ_GNEB_SHAPE_DECL(launch_gneb_images_square_nn)
 MJ_GNEB_SHAPE_DECL(launch_gneb_images_square2)
 MJ_GNEB_SHAPE_DECL(launch_gneb_images_tri_nn)

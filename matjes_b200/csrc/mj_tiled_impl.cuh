@@ -78,6 +78,7 @@ struct TiledArgs {
                         // back to back (3N doubles apart in ms / out, N in aux)
     int smem_bytes;     // host side: dynamic shared memory of the launch when above the
                         // tile's (caps the resident blocks per SM; the excess is unused)
+    const int* stop;    // PASS_GNEB: device flag, the launch does nothing when set (may be null)
     int img_up, img_dn; // PASS_GNEB, set per block: the image has a next / a previous one
 };
 
@@ -621,6 +622,8 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_tiled(const __grid_constant_
         pdl_allow_next();
         if constexpr (!kPurePre) pdl_wait_prev();
     }
+    if constexpr (PASS == PASS_GNEB)
+        if (A.stop && *A.stop) return;
     if (A.R.mode == 2 && bid == 0) ordered_sum<1>(A.R.partials, A.R.nblocks, A.R.out);
     Pre pre[RY];
     bool ok = true;
@@ -1161,7 +1164,7 @@ mj_status launch_sib_fused_shape(mj_plan* p, const DynCoef& C, double* m, double
 // *tiles_per_image receives the count).  No dipolar term.
 template <class S>
 mj_status launch_gneb_images_shape(mj_plan* p, const double* m, double* F, double* partials, int nimg,
-                                   int64_t* tiles_per_image, cudaStream_t s) {
+                                   int64_t* tiles_per_image, const int* stop, cudaStream_t s) {
     TiledArgs A;
     std::memset(&A, 0, sizeof(A));
     A.ms = m;
@@ -1169,6 +1172,7 @@ mj_status launch_gneb_images_shape(mj_plan* p, const double* m, double* F, doubl
     A.bmap = p->d_bmap;
     A.status = p->d_status;
     A.nimg = nimg;
+    A.stop = stop;
     A.pdl = p->use_pdl ? 1 : 0;
     DynCoef C{};
     const bool axial = stencil_axial<S>(p->sp, p->d_bmap != nullptr);

@@ -12,7 +12,7 @@ mj_status launch_sib_fused_square2(mj_plan* p, const DynCoef& C, double* m, doub
     return launch_sib_fused_shape<ShapeSquare2>(p, C, m, draw, E_out, step, s);
 }
 mj_status launch_gneb_images_square2(mj_plan* p, const double* m, double* F, double* partials, int nimg,
-                         int64_t* tiles, cudaStream_t s) {
-    return launch_gneb_images_shape<ShapeSquare2>(p, m, F, partials, nimg, tiles, s);
+                         int64_t* tiles, const int* stop, cudaStream_t s) {
+    return launch_gneb_images_shape<ShapeSquare2>(p, m, F, partials, nimg, tiles, stop, s);
 }
 }  // namespace mj

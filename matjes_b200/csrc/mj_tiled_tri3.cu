@@ -12,7 +12,7 @@ mj_status launch_sib_fused_tri3(mj_plan* p, const DynCoef& C, double* m, double*
     return launch_sib_fused_shape<ShapeTri3>(p, C, m, draw, E_out, step, s);
 }
 mj_status launch_gneb_images_tri3(mj_plan* p, const double* m, double* F, double* partials, int nimg,
-                         int64_t* tiles, cudaStream_t s) {
-    return launch_gneb_images_shape<ShapeTri3>(p, m, F, partials, nimg, tiles, s);
+                         int64_t* tiles, const int* stop, cudaStream_t s) {
+    return launch_gneb_images_shape<ShapeTri3>(p, m, F, partials, nimg, tiles, stop, s);
 }
 }  // namespace mj
