@@ -861,6 +861,13 @@ mj_status mj_plan_create(const mj_lattice_desc* lat, const mj_hamiltonian_desc* 
     if (p->is_stencil) {
         match_shape(sp);
         p->tiled_shape = sp.shape;
+        // The register-capped tiles: 32 x 8 of four warps (8 resident blocks) where
+        // TMA stages them, 32 x 16 of eight warps where an odd Lx means plain loads,
+        // whose halo share is smaller.  SIB step at 10 K, us, variants 0 / 4 / 5:
+        // triangular 1024^2 62.3 / 48.7 / 48.3, 2048^2 202 / 171 / 175; square
+        // 1024^2 49.1 / 40.8 / 40.3; plain loads, triangular 3001 x 2047 430 / 276 /
+        // 320, square 365 / 235 / 241.  mj_plan_autotune picks for one lattice.
+        p->tile_variant = (sp.L[0] & 1) ? 4 : 5;
     }
     if (p->is_stencil) {
         sp.zc = -((1.0 * kMuB * ham->c_zeeman) * lat->moment[g.magatom[0]]);

@@ -513,7 +513,10 @@ struct mj_batch {
     int64_t Ntot = 0;
     mj::StencilParams sp{};
     int shape = 0;
-    int variant = 0;
+    // the register-capped 32 x 8 tiles, as many persistent blocks as are resident
+    // (4, 16, 64, 256 replicas of 32^2 to 256^2, us per step at variants 0 / 3 / 4,
+    // 8 blocks per SM: 18.6 / 14.5 / 14.5, 32.7 / 26.7 / 26.8, 100 / 76 / 80, 356 / 252 / 266)
+    int variant = 3;
     int blocks_per_sm = 8;
     bool zaxial = false;              // every replica's Zeeman field along z
     int num_sms = 148;
