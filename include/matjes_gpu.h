@@ -136,7 +136,11 @@ mj_status mj_plan_noffsets(const mj_plan* plan, int32_t* n);
  * tiles of 4x4, 8x4, 8x2, then 4x4, 8x2, 4x2 compiled for 6, 4, 8 resident
  * blocks per SM (fewer registers).  Tiled variants exist for the square (NN,
  * NN+NNN) and triangular (NN, three shells) offset sets; MJ_ERR_UNSUPPORTED
- * otherwise.  No counterpart in the reference (its SpMV has no tiling). */
+ * otherwise.  A plan left at its default runs calls of two or more steps on a
+ * lattice whose tiles are all resident at once (about 300,000 sites, no dipolar
+ * term) as one launch of many steps; setting a variant makes it run that
+ * variant's launches, one per pass.  The spins are the same bit for bit.  No
+ * counterpart in the reference (its SpMV has no tiling). */
 mj_status mj_plan_set_variant(mj_plan* plan, int32_t variant);
 /* Current variant (-1 generic) and the matched compile-time shape id (0 none). */
 mj_status mj_plan_get_variant(const mj_plan* plan, int32_t* variant, int32_t* shape);

@@ -338,8 +338,9 @@ mj_status alloc_scratch(mj_plan* p) {
     const int64_t N = p->N;
     mj_status st;
     if ((st = dalloc(&p->d_mid, 3 * N, "mid")) != MJ_OK) return st;
-    if ((st = dalloc(&p->d_aux, 3 * N, "aux")) != MJ_OK) return st;
-    if ((st = dalloc(&p->d_aux2, 3 * N, "aux2")) != MJ_OK) return st;
+    const int64_t aux = std::max<int64_t>(3 * N, kStepsAuxDoubles);
+    if ((st = dalloc(&p->d_aux, aux, "aux")) != MJ_OK) return st;
+    if ((st = dalloc(&p->d_aux2, aux, "aux2")) != MJ_OK) return st;
     // generic grid, or the smallest tile of the tiled kernels (32 x 8), whichever has more blocks
     const int64_t tiled_max = p->is_stencil ? static_cast<int64_t>((p->sp.L[0] + 31) / 32) * ((p->sp.L[1] + 7) / 8) * p->sp.L[2] : 0;
     p->partial_cap = 2 * std::max(energy_blocks(p), tiled_max) + 64;
@@ -347,15 +348,22 @@ mj_status alloc_scratch(mj_plan* p) {
     if ((st = dalloc(&p->d_counter, 4, "counter")) != MJ_OK) return st;
     if ((st = cuda_status(cudaMemset(p->d_counter, 0, 4 * sizeof(unsigned int)), "counter init")) != MJ_OK) return st;
     if (p->is_stencil) {
-        const int64_t words = sched_words(p);
-        if ((st = dalloc(&p->d_sched, words, "fused-step scheduler")) != MJ_OK) return st;
-        if ((st = cuda_status(cudaMemset(p->d_sched, 0, sizeof(unsigned int) * words), "scheduler init")) != MJ_OK)
+        const int64_t sched = sched_words(p);
+        if ((st = dalloc(&p->d_sched, sched, "fused-step scheduler")) != MJ_OK) return st;
+        if ((st = cuda_status(cudaMemset(p->d_sched, 0, sizeof(unsigned int) * sched), "scheduler init")) != MJ_OK)
             return st;
     }
+    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
+    // launches of many steps use neither buffer for spins: the tile counters are in
+    // aux2, the energy partials in aux
+    p->aux_doubles = aux;
+    const int64_t words = p->is_stencil && p->sp.shape != 0 ? steps_flag_words(p) : 0;
+    if (words > 0 && words * static_cast<int64_t>(sizeof(unsigned int)) <= aux * static_cast<int64_t>(sizeof(double)) &&
+        aux >= 2 * 8 * (words / kStepsFlagStride))  // room for two slots of energies
+        p->d_steps_flags = reinterpret_cast<unsigned int*>(p->d_aux2);
     if ((st = dalloc(&p->d_scalar, 8, "scalar")) != MJ_OK) return st;
     if ((st = dalloc(&p->d_status, 4, "status")) != MJ_OK) return st;
     if ((st = cuda_status(cudaMemset(p->d_status, 0, 4 * sizeof(int)), "status init")) != MJ_OK) return st;
-    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
     std::vector<double> tab(kNoiseTabDoubles);
     build_noise_tables(tab.data());
     if ((st = dalloc(&p->d_noise_tab, kNoiseTabDoubles, "noise tables")) != MJ_OK) return st;
@@ -454,6 +462,52 @@ mj_status dyn_coef(const mj_dyn_params* d, const mj_plan* plan, DynCoef& c) {
     return MJ_OK;
 }
 
+// The steps of step_sequence in launches of many steps each, for tiled plans
+// whose tiles are all resident at once; `used` is false when they are not.
+// A launch records at most kStepsSlots energies, so with energies the steps
+// are cut there: with the energies after each step, a later launch's first
+// pass gives the last one's, and the last launch adds its final state's.
+mj_status steps_together(mj_plan* p, double* m, const DynCoef& c, int energy_mode, uint32_t step0, int32_t nsteps,
+                         double* E_dev, cudaStream_t s, bool& used) {
+    used = false;
+    if (!p->steps_together || !p->d_steps_flags || !p->is_stencil || p->sp.shape == 0 || p->dip_on || p->fused_sib) return MJ_OK;
+    int warps = 0;
+    mj_status st = launch_steps(p, nullptr, c, &warps, used, s);
+    if (st != MJ_OK || !used) return st;
+    const bool before = energy_mode == MJ_ENERGY_BEFORE;
+    // energies of as many steps per launch as there is room for partials (a tile has at most eight warps)
+    const int64_t tiles = steps_flag_words(p) / kStepsFlagStride;
+    const int32_t slots_max = static_cast<int32_t>(std::min<int64_t>(kStepsSlots, p->aux_doubles / (8 * tiles)));
+    const int32_t chunk = E_dev ? slots_max - 1 : 4096;
+    for (int32_t k0 = 0; k0 < nsteps; k0 += chunk) {
+        const int32_t n = std::min(chunk, nsteps - k0);
+        const bool last = k0 + n == nsteps;
+        StepsJob j;
+        std::memset(&j, 0, sizeof(j));
+        j.m_in = j.m = j.m_out = m;
+        j.mid = p->d_mid;
+        j.nsteps = n;
+        j.step0 = step0 + static_cast<uint32_t>(k0);
+        j.flags = p->d_steps_flags;
+        int slots = 0;
+        double* E = nullptr;
+        if (E_dev) {
+            const bool first = before || k0 > 0;  // the energy of the spins entering this launch is wanted
+            j.partials = p->d_aux;
+            j.e_slot0 = first ? 0 : -1;
+            j.e_final = !before && last;
+            slots = n + (first ? 0 : -1) + (j.e_final ? 1 : 0);
+            E = E_dev + (before ? k0 : std::max(0, k0 - 1));
+        }
+        const int rec = prof_begin(p, "k_steps", s);
+        st = launch_steps(p, &j, c, &warps, used, s);
+        prof_end(p, rec, s);
+        if (st != MJ_OK) return st;
+        if (slots > 0 && (st = launch_steps_energy(p->d_aux, warps, slots, E, s)) != MJ_OK) return st;
+    }
+    return MJ_OK;
+}
+
 // The step sequence shared by mj_step and the graph capture of mj_graph_run.
 // Energies: MJ_ENERGY_AFTER gives E after step k in E_dev[k] (the energy of
 // step k+1's incoming state, fused into its first pass, plus one extra field
@@ -462,6 +516,10 @@ mj_status dyn_coef(const mj_dyn_params* d, const mj_plan* plan, DynCoef& c) {
 mj_status step_sequence(mj_plan* p, double* m, const DynCoef& c, int energy_mode, uint32_t step0, int32_t nsteps,
                         double* E_dev, cudaStream_t s) {
     mj_status st = MJ_OK;
+    if (nsteps > 1) {
+        bool used = false;
+        if ((st = steps_together(p, m, c, energy_mode, step0, nsteps, E_dev, s, used)) != MJ_OK || used) return st;
+    }
     double* cur = m;
     double* other = p->d_mid;
     // the step kernels keep the dipolar pad grid current for the next
@@ -1029,8 +1087,7 @@ mj_status mj_plan_noffsets(const mj_plan* plan, int32_t* n) {
     return MJ_OK;
 }
 
-mj_status mj_plan_set_variant(mj_plan* plan, int32_t variant) {
-    if (!plan) return set_error(MJ_ERR_ARG, "null plan");
+static mj_status set_variant(mj_plan* plan, int32_t variant) {
     if (variant < -1 || variant >= kTiledVariants) return set_error(MJ_ERR_ARG, "variant must be -1..5");
     if (variant >= 0 && !(plan->is_stencil && plan->tiled_shape != 0))
         return set_error(MJ_ERR_UNSUPPORTED, "no tiled kernel for this plan's offsets");
@@ -1046,6 +1103,13 @@ mj_status mj_plan_set_variant(mj_plan* plan, int32_t variant) {
         plan->graph_key.clear();
     }
     return MJ_OK;
+}
+
+mj_status mj_plan_set_variant(mj_plan* plan, int32_t variant) {
+    if (!plan) return set_error(MJ_ERR_ARG, "null plan");
+    const mj_status st = set_variant(plan, variant);
+    if (st == MJ_OK) plan->steps_together = false;  // the program asked for that variant's passes
+    return st;
 }
 
 mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* prm, int32_t steps, int32_t* best,
@@ -1064,6 +1128,15 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* 
         cudaEventDestroy(a);
         return st;
     }
+    // the variants are timed by their own launches; a plan that runs its steps
+    // together (faster than any of them) keeps doing so, with the fastest tile
+    // for its single steps and fields
+    bool together = false;
+    int warps = 0;
+    if (plan->steps_together && plan->d_steps_flags && plan->is_stencil && plan->sp.shape != 0 && !plan->dip_on)
+        launch_steps(plan, nullptr, c, &warps, together, 0);
+    const bool steps_together = plan->steps_together;
+    plan->steps_together = false;
     double best_ms = 1e300;
     int32_t best_v = v0;
     bool best_t = plan->use_tma;
@@ -1077,7 +1150,7 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* 
             continue;
         }
         plan->use_tma = tma;
-        if (plan->is_stencil && (st = mj_plan_set_variant(plan, v)) != MJ_OK) break;
+        if (plan->is_stencil && (st = set_variant(plan, v)) != MJ_OK) break;
         if ((st = cuda_status(cudaMemcpy(plan->d_tmp_m, m, sizeof(double) * 3 * plan->N, cudaMemcpyDeviceToDevice),
                               "autotune copy")) != MJ_OK)
             break;
@@ -1090,7 +1163,7 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* 
         cudaEventElapsedTime(&f, a, b);
         ms = f / steps;
         if (ms_per_step) ms_per_step[cfg] = ms;
-        if (ms < best_ms) {
+        if (ms < best_ms && !(together && v < 0)) {
             best_ms = ms;
             best_v = v;
             best_t = tma;
@@ -1098,9 +1171,10 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* 
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
+    plan->steps_together = steps_together;
     if (st != MJ_OK) return st;
     plan->use_tma = best_t;
-    if (plan->is_stencil && (st = mj_plan_set_variant(plan, best_v)) != MJ_OK) return st;
+    if (plan->is_stencil && (st = set_variant(plan, best_v)) != MJ_OK) return st;
     if ((st = mj_plan_check_status(plan)) != MJ_OK) return st;
     *best = best_v;
     if (best_tma) *best_tma = best_t ? 1 : 0;

@@ -206,6 +206,16 @@ __device__ __forceinline__ double3 cross(double3 a, double3 b) {
     return make_double3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 __device__ __forceinline__ double dot(double3 a, double3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// The same with every fma explicit: the spins' updates below are made of these,
+// so that they round the same way in every kernel that makes them.
+__device__ __forceinline__ double3 cross_f(double3 a, double3 b) {
+    return make_double3(fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x)));
+}
+__device__ __forceinline__ double dot_f(double3 a, double3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+// m + c D
+__device__ __forceinline__ double3 advance(double3 m, double3 D, double c) {
+    return make_double3(fma(D.x, c, m.x), fma(D.y, c, m.y), fma(D.z, c, m.z));
+}
 
 __device__ __forceinline__ double3 ld3(const double* __restrict__ m, int64_t i, int64_t N) {
     return make_double3(__ldg(m + i), __ldg(m + N + i), __ldg(m + 2 * N + i));
@@ -253,19 +263,19 @@ __device__ __forceinline__ double cayley_scale(double q) {
 // Matjes LLG right-hand side (solvers/propagator.f90:13-58):
 // D = -[m^ x B + alpha m^ x (m^ x B)] / (1 + alpha^2), m^ = m/|m| when |m| > 1e-8.
 __device__ __forceinline__ double3 llg_rhs(double3 B, double3 m, double alpha, double inv_den) {
-    const double inv = inv_norm(dot(m, m));
+    const double inv = inv_norm(dot_f(m, m));
     const double3 mn = make_double3(m.x * inv, m.y * inv, m.z * inv);
-    const double3 t = cross(mn, B);
-    const double3 l = make_double3(B.x + alpha * t.x, B.y + alpha * t.y, B.z + alpha * t.z);
-    const double3 o = cross(mn, l);
+    const double3 t = cross_f(mn, B);
+    const double3 l = advance(B, t, alpha);
+    const double3 o = cross_f(mn, l);
     return make_double3(-o.x * inv_den, -o.y * inv_den, -o.z * inv_den);
 }
 
 // Projection onto the old norm (solvers/solver.f90:113-116), |t| > 1e-8 guard.
 __device__ __forceinline__ double3 project(double3 t, double3 m) {
-    const double nt2 = dot(t, t);
+    const double nt2 = dot_f(t, t);
     if (!(nt2 > 1e-16)) return m;
-    const double s = norm_of(dot(m, m)) * inv_norm(nt2);
+    const double s = norm_of(dot_f(m, m)) * inv_norm(nt2);
     return make_double3(t.x * s, t.y * s, t.z * s);
 }
 
@@ -277,12 +287,12 @@ __device__ __forceinline__ double3 project(double3 t, double3 m) {
 template <bool MID = false>
 __device__ __forceinline__ double3 sib_solve(double3 m, double3 p, double3 H, double alpha, double hc) {
     // h = hc H + (hc alpha / |p|) p x H: the normalisation folded into one scalar
-    const double sa = hc * alpha * inv_norm(dot(p, p));
-    const double3 pxh = cross(p, H);
+    const double sa = hc * alpha * inv_norm(dot_f(p, p));
+    const double3 pxh = cross_f(p, H);
     const double3 h = make_double3(fma(sa, pxh.x, hc * H.x), fma(sa, pxh.y, hc * H.y), fma(sa, pxh.z, hc * H.z));
-    const double3 u = cross(m, h);
-    const double3 w = cross(u, h);
-    double c = cayley_scale(dot(h, h));
+    const double3 u = cross_f(m, h);
+    const double3 w = cross_f(u, h);
+    double c = cayley_scale(dot_f(h, h));
     if constexpr (MID) c = 0.5 * c;
     return make_double3(fma(c, u.x + w.x, m.x), fma(c, u.y + w.y, m.y), fma(c, u.z + w.z, m.z));
 }

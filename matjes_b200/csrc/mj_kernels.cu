@@ -258,10 +258,10 @@ __global__ void __launch_bounds__(256) k_euler(const __grid_constant__ F fp, con
         e = total_energy_part(f, m0, hd);
         const double3 D = llg_rhs(minus2(f.B, hd), m0, C.alpha, C.inv_den);
         const double c = C.h_over_hbar;
-        double3 t = make_double3(m0.x + D.x * c, m0.y + D.y * c, m0.z + D.z * c);
+        double3 t = advance(m0, D, c);
         if (C.thermal) {
             const double3 DT = llg_rhs(thermal_field(C, step, i, N), m0, C.alpha, C.inv_den);
-            t = make_double3(t.x + DT.x * c, t.y + DT.y * c, t.z + DT.z * c);
+            t = advance(t, DT, c);
         }
         const double3 mo = project(t, m0);
         flag_nonfinite(status, mo);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, con
         e = total_energy_part(f, m0, hd);
         const double3 D = llg_rhs(minus2(f.B, hd), m0, C.alpha, C.inv_den);
         const double c = C.h_over_hbar;
-        const double3 t = make_double3(m0.x + D.x * c, m0.y + D.y * c, m0.z + D.z * c);
+        const double3 t = advance(m0, D, c);
         const double3 mt = project(t, m0);
         st3(mid, i, N, mt);
         if (pad.p) st_pad(pad, x, y, z, mt);
@@ -324,10 +324,10 @@ __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, con
     const double3 d1 = ld3(D1, i, N);
     const double3 Di = make_double3(0.5 * d1.x + 0.5 * D2.x, 0.5 * d1.y + 0.5 * D2.y, 0.5 * d1.z + 0.5 * D2.z);
     const double c = C.h_over_hbar;
-    double3 t = make_double3(mt.x + Di.x * c, mt.y + Di.y * c, mt.z + Di.z * c);
+    double3 t = advance(mt, Di, c);
     if (C.thermal) {
         const double3 DT = ld3(DTi, i, N);
-        t = make_double3(t.x + DT.x * c, t.y + DT.y * c, t.z + DT.z * c);
+        t = advance(t, DT, c);
     }
     const double3 mo = project(t, mt);
     flag_nonfinite(status, mo);
@@ -483,6 +483,11 @@ __global__ void __launch_bounds__(256) k_soa_to_aos_stream(const double* __restr
 }
 // energy partials summed in the fixed order of ordered_sum (one block)
 __global__ void k_ordered_sum1(const double* partials, int nblocks, double* out) { ordered_sum<1>(partials, nblocks, out); }
+
+// E[slot]: a slot's energy partials in the same fixed order (mj_steps_impl.cuh)
+__global__ void __launch_bounds__(256) k_steps_energy(const double* partials, int n, double* E) {
+    ordered_sum<1>(partials + static_cast<int64_t>(blockIdx.x) * n, n, E + blockIdx.x);
+}
 
 __global__ void k_soa_to_aos(const double* __restrict__ s, double* __restrict__ a, int64_t n) {
     const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -779,6 +784,10 @@ mj_status soa_to_aos_stream(const double* so, double* a, int64_t i0, int64_t cnt
 mj_status launch_ordered_sum(const double* partials, int nblocks, int nthreads, double* out, cudaStream_t s) {
     k_ordered_sum1<<<1, nthreads, 0, s>>>(partials, nblocks, out);
     return cuda_status(cudaGetLastError(), "k_ordered_sum1");
+}
+mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, cudaStream_t s) {
+    k_steps_energy<<<slots, 256, 0, s>>>(partials, n, E);
+    return cuda_status(cudaGetLastError(), "k_steps_energy");
 }
 mj_status soa_to_aos(const double* so, double* a, int64_t n, cudaStream_t s) {
     if (n <= 0) return MJ_OK;

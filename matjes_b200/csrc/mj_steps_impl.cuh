@@ -1,0 +1,442 @@
+// Many time steps in one launch, for lattices whose tiles are all resident at
+// once (mj_shapes.hpp lattices, no dipolar term).
+//
+// A small lattice's step is bound by its two dependent launches, not by its
+// arithmetic: 64^2 sites are 16 tiles on 148 SMs, and a launch with its ramp,
+// halo staging and last block takes 5 us of which the tile's own work is a
+// fraction.  Here every block keeps one 32 x 8 tile for the whole call: the
+// tile's spins stay in registers and shared memory, and a pass reads only the
+// halo cells from global memory.  Blocks synchronise with their eight
+// neighbouring tiles alone, through one counter per tile (the passes whose
+// results the tile has published): before a pass stages its halo it waits for
+// the counters of the neighbours, which also says that they have staged what
+// the tile is about to overwrite (the neighbourhood is symmetric), so spins and
+// midpoints are updated in place.  The thermal draw of a step is made before
+// the wait, and neither it nor m_n goes through memory between the passes.
+// The launch is cooperative, so all blocks run at once and every wait ends; the
+// waits are bounded all the same (kStatusTimeout).
+//
+// The arithmetic is the tiled passes' (mj_tiled_impl.cuh): the spins are the
+// same bit for bit.  us per SIB step at 10 K, this against two launches: square
+// 16^2 4.0 / 10.6, 64^2 4.9 / 10.8, 256^2 6.6 / 12.0, 512^2 11.1 / 15.8;
+// triangular, three shells, 64^2 5.8 / 12.3, 256^2 7.9 / 13.4, 512^2 13.4 / 18.7.
+// What bounds it: up to 256^2 the chain release - acquire - halo load - pass,
+// about 2.2 us a pass; at 512^2 instruction issue (42 ps per site and step).
+#pragma once
+
+#include "mj_tiled_impl.cuh"
+
+namespace mj {
+namespace {
+
+struct StepsArgs {
+    const double* m_in;  // spins entering step 0
+    double* m;           // spins entering step k > 0: m + k m_stride (Euler: alternating with mid)
+    int64_t m_stride;
+    double* mid;         // midpoint of step k: mid + k mid_stride
+    int64_t mid_stride;
+    double* m_out;       // spins after the last step
+    const double* bmap;
+    double* partials;    // energy partials, one per warp: [slot][warps of the launch]
+    int e_slot0;         // slot of the energy of the spins entering step 0 (-1: not recorded), step k's at + k
+    int e_on;
+    int e_final;         // also the energy of the spins after the last step
+    int half;            // the last step makes its predictor only
+    int nsteps;
+    uint32_t step0;
+    unsigned int* flags; // per tile (kStepsFlagStride apart): passes published, zero at the launch
+    int* status;
+};
+
+constexpr uint32_t kStepsWaitPolls = 1u << 20;
+
+// The halo of a block's tile (TileGeom layout; grid x, y over the tiles, z over
+// the layers) and the counters of its neighbours.
+template <class S, int BYT, int RY>
+struct TileRing {
+    using G = TileGeom<S, BYT, RY>;
+    static constexpr int R = G::R, NT = 32 * BYT;
+    static constexpr int KH = ((G::TX + 2 * R) * (G::TY + 2 * R) - G::TX * G::TY + NT - 1) / NT;  // cells per thread
+    int hpos[KH], hsrc[KH];     // a halo cell's place in the tile, its site in the layer (-1: none, or past an open edge)
+    const unsigned int* nflag;  // threads 0 .. 7: the counter of one neighbouring tile each (null: none)
+    unsigned int* flag;         // the tile's own
+
+    __device__ __forceinline__ void init(const StencilParams& P, unsigned int* flags) {
+        const int Lx = P.L[0], Ly = P.L[1];
+        const int tid = threadIdx.x + 32 * threadIdx.y;
+        const int x0 = blockIdx.x * G::TX, y0 = blockIdx.y * G::TY;
+        const int w = min(G::TX, Lx - x0), h = min(G::TY, Ly - y0);
+        // the ring of width R about the tile's w x h sites: rows below and above, then the sides
+        const int full = w + 2 * R;
+#pragma unroll
+        for (int q = 0; q < KH; ++q) {
+            const int c = tid + q * NT;
+            int lx = 0, ly = -1;  // relative to the tile's first site
+            if (c < R * full) {
+                lx = c % full - R;
+                ly = c / full - R;
+            } else if (c < 2 * R * full) {
+                lx = (c - R * full) % full - R;
+                ly = h + (c - R * full) / full;
+            } else if (c < 2 * R * (full + h)) {
+                const int d = c - 2 * R * full;
+                ly = d / (2 * R);
+                lx = d % (2 * R);
+                lx = lx < R ? lx - R : w + lx - R;
+            }
+            hsrc[q] = -1;
+            hpos[q] = (ly + R) * G::PX + lx + G::RX;
+            if (c < 2 * R * (full + h)) {
+                int gx = x0 + lx, gy = y0 + ly;
+                const bool outx = gx < 0 || gx >= Lx, outy = gy < 0 || gy >= Ly;
+                if (!((outx && !P.periodic[0]) || (outy && !P.periodic[1]))) {
+                    if (outx) gx = ((gx % Lx) + Lx) % Lx;
+                    if (outy) gy = ((gy % Ly) + Ly) % Ly;
+                    hsrc[q] = gx + Lx * gy;
+                }
+            }
+        }
+        const int nx = gridDim.x, ny = gridDim.y, z = blockIdx.z;
+        auto of = [&](int tx, int ty) { return flags + static_cast<int64_t>(kStepsFlagStride) * (tx + nx * (ty + ny * z)); };
+        flag = of(blockIdx.x, blockIdx.y);
+        nflag = nullptr;
+        if (tid < 8) {
+            const int k = tid < 4 ? tid : tid + 1;
+            const int tx = static_cast<int>(blockIdx.x) + k % 3 - 1, ty = static_cast<int>(blockIdx.y) + k / 3 - 1;
+            const bool okx = P.periodic[0] || (tx >= 0 && tx < nx), oky = P.periodic[1] || (ty >= 0 && ty < ny);
+            if (okx && oky) nflag = of((tx + nx) % nx, (ty + ny) % ny);
+        }
+    }
+    // until the neighbours have published `target` passes; false on a timeout (all threads of the block)
+    __device__ __forceinline__ bool wait(unsigned int target, int* status) const {
+        bool bad = false;
+        if (nflag) {
+            uint32_t it = 0;
+            while (ld_acquire_u32(nflag) < target) {
+                if (++it > kStepsWaitPolls) {
+                    bad = true;
+                    break;
+                }
+                if (it > 4096) __nanosleep(64);
+            }
+        }
+        if (__syncthreads_or(bad)) {
+            if (threadIdx.x == 0 && threadIdx.y == 0 && status) atomicOr(status, kStatusTimeout);
+            return false;
+        }
+        return true;
+    }
+    // the halo cells of a layer of `src` (component stride N) into the tile
+    __device__ __forceinline__ void load(const double* src, int64_t N, double* sm) const {
+#pragma unroll
+        for (int q = 0; q < KH; ++q)
+            if (hsrc[q] >= 0) {
+                const double vx = __ldcg(src + hsrc[q]), vy = __ldcg(src + N + hsrc[q]), vz = __ldcg(src + 2 * N + hsrc[q]);
+                sm[hpos[q]] = vx;
+                sm[G::NS + hpos[q]] = vy;
+                sm[2 * G::NS + hpos[q]] = vz;
+            }
+    }
+    // after every thread's stores, which the release then covers
+    __device__ __forceinline__ void publish(unsigned int passes) const {
+        __syncthreads();
+        if (threadIdx.x == 0 && threadIdx.y == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(passes) : "memory");
+    }
+};
+
+template <class S, int BYT, int RY, int MINB, int SP, int INTEG>
+__global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant__ StencilParams P,
+                                                          const __grid_constant__ DynCoef C,
+                                                          const __grid_constant__ StepsArgs A) {
+    using G = TileGeom<S, BYT, RY>;
+    constexpr int R = G::R, NT = 32 * BYT;
+    constexpr bool kTwo = INTEG != MJ_EULER;  // passes per step
+    extern __shared__ __align__(128) double sm[];
+    const int Lx = P.L[0], Ly = P.L[1];
+    const int64_t layer = static_cast<int64_t>(Lx) * Ly, N = layer * P.L[2];
+    const int z = blockIdx.z;
+    const int x0 = blockIdx.x * G::TX, y0 = blockIdx.y * G::TY;
+    const int tid = threadIdx.x + 32 * threadIdx.y;
+    const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    // cells across an open edge stay zero
+    for (int q = tid; q < 3 * G::NS; q += NT) sm[q] = 0.0;
+    TileRing<S, BYT, RY> ring;
+    ring.init(P, A.flags);
+    const int x = x0 + static_cast<int>(threadIdx.x), yt = y0 + static_cast<int>(threadIdx.y) * RY;
+    const int64_t i0 = layer * z + x + static_cast<int64_t>(Lx) * yt;
+    const int base = static_cast<int>(threadIdx.y) * RY * G::PX + static_cast<int>(threadIdx.x);
+    const int own = base + G::R * G::PX + G::RX;  // the first own site's cell
+    double3 mn[RY];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RY; ++r) {
+        mn[r] = make_double3(0.0, 0.0, 0.0);
+        if (x < Lx && yt + r < Ly) {
+            const int64_t i = i0 + static_cast<int64_t>(Lx) * r;
+            mn[r] = make_double3(__ldcg(A.m_in + i), __ldcg(A.m_in + N + i), __ldcg(A.m_in + 2 * N + i));
+            const int c = own + r * G::PX;
+            sm[c] = mn[r].x;
+            sm[G::NS + c] = mn[r].y;
+            sm[2 * G::NS + c] = mn[r].z;
+        }
+    }
+    auto wait = [&](unsigned int target) { return ring.wait(target, A.status); };
+    // the halo of `src`, which the neighbours' first `target` passes wrote
+    auto stage = [&](const double* src, unsigned int target) -> bool {
+        if (target > 0 && !wait(target)) return false;
+        ring.load(src + layer * z, N, sm);
+        __syncthreads();
+        return true;
+    };
+    auto publish = [&](unsigned int passes) { ring.publish(passes); };
+    // field of the thread's sites from the staged tile, m0[r] their own spins: real-space
+    // field into B, the sites' energy returned when wanted
+    auto field = [&](const double3 (&m0)[RY], double3 (&B)[RY], bool want_e) -> double {
+        double bx[RY], by[RY], bz[RY];
+#pragma unroll
+        for (int r = 0; r < RY; ++r) bx[r] = by[r] = bz[r] = 0.0;
+        all_columns<S, BYT, RY, SP>(P, sm, base, bx, by, bz, std::make_integer_sequence<int, 2 * S::R + 1>{});
+        double e = 0.0;
+#pragma unroll
+        for (int r = 0; r < RY; ++r) {
+            double b0 = bx[r], b1 = by[r], b2 = bz[r];
+            if (P.has_onsite) {
+                const double* W = P.W0;
+                if constexpr (SP == SP_AXIAL) {
+                    b2 = fma(W[8], m0[r].z, b2);
+                } else {
+                    b0 = fma(W[0], m0[r].x, fma(W[1], m0[r].y, fma(W[2], m0[r].z, b0)));
+                    b1 = fma(W[3], m0[r].x, fma(W[4], m0[r].y, fma(W[5], m0[r].z, b1)));
+                    b2 = fma(W[6], m0[r].x, fma(W[7], m0[r].y, fma(W[8], m0[r].z, b2)));
+                }
+            }
+            const bool in = x < Lx && yt + r < Ly;
+            double3 zee = make_double3(0.0, 0.0, 0.0);
+            if (P.zee_on) {
+                if (A.bmap) {
+                    const int64_t i = in ? i0 + static_cast<int64_t>(Lx) * r : 0;
+                    zee = make_double3(P.zc * __ldg(A.bmap + i), P.zc * __ldg(A.bmap + N + i),
+                                       P.zc * __ldg(A.bmap + 2 * N + i));
+                } else if constexpr (SP == SP_AXIAL) {
+                    zee.z = P.zc * P.bext[2];
+                } else {
+                    zee = make_double3(P.zc * P.bext[0], P.zc * P.bext[1], P.zc * P.bext[2]);
+                }
+            }
+            // the axial form adds no x, y Zeeman field without a map, as the tiled passes
+            const bool zax = SP == SP_AXIAL && !A.bmap;
+            B[r] = zax ? make_double3(b0, b1, b2 + zee.z) : make_double3(b0 + zee.x, b1 + zee.y, b2 + zee.z);
+            if (want_e && in) {
+                const double mz = zax ? m0[r].z * zee.z : dot(m0[r], zee);
+                e += -0.5 * (dot(m0[r], B[r]) + mz);
+            }
+        }
+        return e;
+    };
+    const int nwarps = static_cast<int>(gridDim.x * gridDim.y * gridDim.z) * BYT;
+    auto record = [&](double e, int slot) {
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+        if (threadIdx.x == 0) A.partials[static_cast<int64_t>(slot) * nwarps + bid * BYT + threadIdx.y] = e;
+    };
+    // new spins v of the thread's sites into the tile and dst (after every thread has read the tile)
+    auto store = [&](const double3 (&v)[RY], double* dst) {
+#pragma unroll
+        for (int r = 0; r < RY; ++r)
+            if (x < Lx && yt + r < Ly) {
+                const int c = own + r * G::PX;
+                sm[c] = v[r].x;
+                sm[G::NS + c] = v[r].y;
+                sm[2 * G::NS + c] = v[r].z;
+                st3(dst, i0 + static_cast<int64_t>(Lx) * r, N, v[r]);
+            }
+    };
+    TiledArgs TA = {};
+    for (int k = 0; k < A.nsteps; ++k) {
+        const bool last = k + 1 == A.nsteps;
+        Pre pre[RY];
+        TA.step = A.step0 + static_cast<uint32_t>(k);
+        if (C.thermal) prefetch_sites<S, BYT, RY, PASS_SIB1>(P, C, TA, x0, y0, z, pre);
+        const double* src = k == 0 ? A.m_in : A.m + k * A.m_stride;
+        if constexpr (!kTwo)
+            if (k & 1) src = A.mid;
+        if (!stage(src, static_cast<unsigned int>(kTwo ? 2 * k : k))) return;
+        double3 B[RY], v[RY];
+        const int slot = A.e_slot0 + k;
+        const bool want_e = A.e_on && slot >= 0;
+        const double e = field(mn, B, want_e);
+        if (want_e) record(e, slot);
+        if constexpr (!kTwo) {
+            double* dst = last ? A.m_out : ((k & 1) ? A.m : A.mid);
+#pragma unroll
+            for (int r = 0; r < RY; ++r) {
+                const double3 D = llg_rhs(B[r], mn[r], C.alpha, C.inv_den);
+                const double c = C.h_over_hbar;
+                double3 t = advance(mn[r], D, c);
+                if (C.thermal) {
+                    const double3 DT = llg_rhs(pre[r].b, mn[r], C.alpha, C.inv_den);
+                    t = advance(t, DT, c);
+                }
+                v[r] = project(t, mn[r]);
+                if (x < Lx && yt + r < Ly) flag_nonfinite(A.status, v[r]);
+            }
+            if (last && !(k & 1)) {
+                // the last spins replace those that this step read: the neighbours have staged them first
+                publish(static_cast<unsigned int>(A.nsteps));
+                if (!wait(static_cast<unsigned int>(A.nsteps))) return;
+            }
+            __syncthreads();
+            store(v, dst);
+#pragma unroll
+            for (int r = 0; r < RY; ++r) mn[r] = v[r];
+            publish(static_cast<unsigned int>(last && !(k & 1) ? k + 2 : k + 1));
+            continue;
+        }
+        double3 d1[RY], dt[RY];  // Heun: the predictor's slope and the thermal one
+#pragma unroll
+        for (int r = 0; r < RY; ++r) {
+            if constexpr (INTEG == MJ_SIB) {
+                double3 H = B[r];
+                if (C.thermal) H = make_double3(H.x + pre[r].b.x, H.y + pre[r].b.y, H.z + pre[r].b.z);
+                v[r] = sib_solve<true>(mn[r], mn[r], H, C.alpha, C.sib_hc);
+            } else {
+                d1[r] = llg_rhs(B[r], mn[r], C.alpha, C.inv_den);
+                const double c = C.h_over_hbar;
+                v[r] = project(advance(mn[r], d1[r], c), mn[r]);
+                if (C.thermal) dt[r] = llg_rhs(pre[r].b, mn[r], C.alpha, C.inv_den);
+            }
+        }
+        __syncthreads();  // the tile has been read
+        double* mid = A.mid + k * A.mid_stride;
+        store(v, mid);
+        if (last && A.half) return;
+        publish(static_cast<unsigned int>(2 * k + 1));
+        if (!stage(mid, static_cast<unsigned int>(2 * k + 1))) return;
+        field(v, B, false);
+#pragma unroll
+        for (int r = 0; r < RY; ++r) {
+            if constexpr (INTEG == MJ_SIB) {
+                double3 H = B[r];
+                if (C.thermal) H = make_double3(H.x + pre[r].b.x, H.y + pre[r].b.y, H.z + pre[r].b.z);
+                mn[r] = sib_solve(mn[r], v[r], H, C.alpha, C.sib_hc);
+            } else {
+                const double3 d2 = llg_rhs(B[r], v[r], C.alpha, C.inv_den);
+                const double3 di = make_double3(0.5 * d1[r].x + 0.5 * d2.x, 0.5 * d1[r].y + 0.5 * d2.y,
+                                                0.5 * d1[r].z + 0.5 * d2.z);
+                const double c = C.h_over_hbar;
+                double3 t = advance(v[r], di, c);
+                if (C.thermal) t = advance(t, dt[r], c);
+                mn[r] = project(t, v[r]);
+            }
+            if (x < Lx && yt + r < Ly) flag_nonfinite(A.status, mn[r]);
+        }
+        __syncthreads();
+        store(mn, last ? A.m_out : A.m + (k + 1) * A.m_stride);
+        publish(static_cast<unsigned int>(2 * k + 2));
+    }
+    if (A.e_final) {
+        const unsigned int odd_euler = !kTwo && (A.nsteps & 1) ? 1u : 0u;
+        if (!stage(A.m_out, static_cast<unsigned int>(kTwo ? 2 * A.nsteps : A.nsteps) + odd_euler)) return;
+        double3 B[RY];
+        const double e = field(mn, B, true);
+        record(e, A.e_slot0 + A.nsteps);
+    }
+}
+
+template <class S, int BYT, int RY, int MINB, int SP, int INTEG>
+mj_status launch_steps_cfg(mj_plan* p, const DynCoef& C, const StepsArgs& A, dim3 grid, cudaStream_t s) {
+    auto kern = k_steps<S, BYT, RY, MINB, SP, INTEG>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32, BYT);
+    cfg.dynamicSmemBytes = TileGeom<S, BYT, RY>::buf_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kern, p->sp, C, A), "k_steps");
+}
+
+// A halo reaches the next tile alone, unless a last tile is thinner than the
+// reach: the one before it is then in reach of the periodic images too.
+template <class S>
+bool thin_last_tile(const StencilParams& P) {
+    auto thin = [&](int d, int t) { return P.periodic[d] && P.L[d] > t && P.L[d] % t != 0 && P.L[d] % t < S::R; };
+    return thin(0, 32) || thin(1, kStepsTY);
+}
+
+// Resident tiles of a configuration on the plan's device.
+template <class S, int BYT, int RY, int MINB, int SP, int INTEG>
+int steps_capacity(const mj_plan* p) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<S, BYT, RY, MINB, SP, INTEG>, 32 * BYT,
+                                                      TileGeom<S, BYT, RY>::buf_bytes) != cudaSuccess)
+        return 0;
+    return per_sm * p->num_sms;
+}
+
+template <class S, int SP, int INTEG>
+mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s) {
+    using G = TileGeom<S, 8, 1>;
+    static_assert(G::TY == kStepsTY && TileGeom<S, 4, 2>::TY == kStepsTY, "one tile height");
+    const dim3 grid((p->sp.L[0] + 31) / 32, (p->sp.L[1] + kStepsTY - 1) / kStepsTY, p->sp.L[2]);
+    const int64_t tiles = static_cast<int64_t>(grid.x) * grid.y * grid.z;
+    fits = false;
+    if (thin_last_tile<S>(p->sp)) return MJ_OK;
+    // one site per thread while the blocks of eight warps that are resident hold
+    // the lattice (the shortest chain per pass), two sites per thread above: at
+    // six blocks per SM, then at eight with the registers that leaves (64; 512^2
+    // 11.1 us a step where the two launches take 15.8)
+    const bool one = tiles <= steps_capacity<S, 8, 1, 2, SP, INTEG>(p);
+    const bool six = tiles <= steps_capacity<S, 4, 2, 6, SP, INTEG>(p);
+    if (!one && !six && tiles > steps_capacity<S, 4, 2, 8, SP, INTEG>(p)) return MJ_OK;
+    fits = true;
+    if (!job) return MJ_OK;
+    *warps = static_cast<int>(tiles) * (one ? 8 : 4);
+    StepsArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.m_in = job->m_in;
+    A.m = job->m;
+    A.m_stride = job->m_stride;
+    A.mid = job->mid;
+    A.mid_stride = job->mid_stride;
+    A.m_out = job->m_out;
+    A.bmap = p->d_bmap;
+    A.partials = job->partials;
+    A.e_on = job->partials != nullptr;
+    A.e_slot0 = job->e_slot0;
+    A.e_final = job->e_final;
+    A.half = job->half;
+    A.nsteps = job->nsteps;
+    A.step0 = job->step0;
+    A.flags = job->flags;
+    A.status = p->d_status;
+    mj_status st = cuda_status(cudaMemsetAsync(job->flags, 0, sizeof(unsigned int) * kStepsFlagStride * tiles, s),
+                               "step counters");
+    if (st != MJ_OK) return st;
+    if (one) return launch_steps_cfg<S, 8, 1, 2, SP, INTEG>(p, C, A, grid, s);
+    if (six) return launch_steps_cfg<S, 4, 2, 6, SP, INTEG>(p, C, A, grid, s);
+    return launch_steps_cfg<S, 4, 2, 8, SP, INTEG>(p, C, A, grid, s);
+}
+
+// job = null: only whether the plan's lattice fits (`fits`)
+template <class S>
+mj_status launch_steps_shape(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s) {
+    const bool axial = stencil_axial<S>(p->sp, p->d_bmap != nullptr);
+    switch (C.integrator) {
+        case MJ_EULER:
+            return axial ? steps_run<S, SP_AXIAL, MJ_EULER>(p, job, C, warps, fits, s)
+                         : steps_run<S, SP_FULL, MJ_EULER>(p, job, C, warps, fits, s);
+        case MJ_HEUN_MATJES:
+            return axial ? steps_run<S, SP_AXIAL, MJ_HEUN_MATJES>(p, job, C, warps, fits, s)
+                         : steps_run<S, SP_FULL, MJ_HEUN_MATJES>(p, job, C, warps, fits, s);
+        default:
+            return axial ? steps_run<S, SP_AXIAL, MJ_SIB>(p, job, C, warps, fits, s)
+                         : steps_run<S, SP_FULL, MJ_SIB>(p, job, C, warps, fits, s);
+    }
+}
+
+}  // namespace
+}  // namespace mj

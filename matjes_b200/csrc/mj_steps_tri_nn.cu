@@ -1,0 +1,9 @@
+// Many steps in one launch on one lattice shape (ShapeTriNN); see mj_steps_impl.cuh.
+#include "mj_steps_impl.cuh"
+
+namespace mj {
+mj_status launch_steps_tri_nn(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits,
+                         cudaStream_t s) {
+    return launch_steps_shape<ShapeTriNN>(p, job, C, warps, fits, s);
+}
+}  // namespace mj

@@ -34,6 +34,23 @@ int64_t tiled_energy_blocks(const mj_plan* p) {
     return static_cast<int64_t>((p->sp.L[0] + 31) / 32) * ((p->sp.L[1] + ty - 1) / ty) * p->sp.L[2];
 }
 
+// at most eight resident blocks of 128 threads per SM hold one 32 x 8 tile each
+int64_t steps_flag_words(const mj_plan* p) {
+    const int64_t tiles = static_cast<int64_t>((p->sp.L[0] + 31) / 32) * ((p->sp.L[1] + kStepsTY - 1) / kStepsTY) * p->sp.L[2];
+    return tiles <= 8 * static_cast<int64_t>(p->num_sms) ? tiles * kStepsFlagStride : 0;
+}
+
+mj_status launch_steps(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s) {
+    fits = false;
+    switch (p->sp.shape) {
+        case kShapeSquareNN: return launch_steps_square_nn(p, job, C, warps, fits, s);
+        case kShapeSquare2: return launch_steps_square2(p, job, C, warps, fits, s);
+        case kShapeTriNN: return launch_steps_tri_nn(p, job, C, warps, fits, s);
+        case kShapeTri3: return launch_steps_tri3(p, job, C, warps, fits, s);
+        default: return MJ_OK;
+    }
+}
+
 int64_t sched_words(const mj_plan* p) {
     int min_ty = kTiledVariantTY[0];
     for (int v = 1; v < kTiledVariants; ++v) min_ty = std::min(min_ty, kTiledVariantTY[v]);

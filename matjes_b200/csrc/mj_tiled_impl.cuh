@@ -237,10 +237,10 @@ __device__ __forceinline__ double epilogue(const DynCoef& C, const TiledArgs& A,
     } else if constexpr (PASS == PASS_EULER) {
         const double3 D = llg_rhs(B, m0, C.alpha, C.inv_den);
         const double c = C.h_over_hbar;
-        double3 t = make_double3(m0.x + D.x * c, m0.y + D.y * c, m0.z + D.z * c);
+        double3 t = advance(m0, D, c);
         if (C.thermal) {
             const double3 DT = llg_rhs(pre.b, m0, C.alpha, C.inv_den);
-            t = make_double3(t.x + DT.x * c, t.y + DT.y * c, t.z + DT.z * c);
+            t = advance(t, DT, c);
         }
         const double3 mo = project(t, m0);
         flag_nonfinite(A.status, mo);
@@ -249,7 +249,7 @@ __device__ __forceinline__ double epilogue(const DynCoef& C, const TiledArgs& A,
     } else if constexpr (PASS == PASS_HEUN1) {
         const double3 D = llg_rhs(B, m0, C.alpha, C.inv_den);
         const double c = C.h_over_hbar;
-        const double3 t = make_double3(m0.x + D.x * c, m0.y + D.y * c, m0.z + D.z * c);
+        const double3 t = advance(m0, D, c);
         st3(A.out, i, N, project(t, m0));
         st3(A.aux, i, N, D);
         if (C.thermal) st3(A.aux2, i, N, llg_rhs(pre.b, m0, C.alpha, C.inv_den));
@@ -259,10 +259,10 @@ __device__ __forceinline__ double epilogue(const DynCoef& C, const TiledArgs& A,
         const double3 d1 = pre.a;
         const double3 Di = make_double3(0.5 * d1.x + 0.5 * D2.x, 0.5 * d1.y + 0.5 * D2.y, 0.5 * d1.z + 0.5 * D2.z);
         const double c = C.h_over_hbar;
-        double3 t = make_double3(m0.x + Di.x * c, m0.y + Di.y * c, m0.z + Di.z * c);
+        double3 t = advance(m0, Di, c);
         if (C.thermal) {
             const double3 DT = pre.b;
-            t = make_double3(t.x + DT.x * c, t.y + DT.y * c, t.z + DT.z * c);
+            t = advance(t, DT, c);
         }
         const double3 mo = project(t, m0);
         flag_nonfinite(A.status, mo);
