@@ -22,7 +22,9 @@
 // in shared memory, every offset unrolled) or, for other lattices, a generic
 // one-site-per-thread kernel.  The trajectory is checkpointed every
 // `checkpoint_every` steps; each segment is recomputed (m_n and mb stored)
-// with the plan's own SIB kernels before its backward sweep.
+// with the plan's own SIB kernels before its backward sweep.  On lattices whose
+// tiles are all resident at once the forward steps, the recomputation and the
+// backward steps of a segment are one launch each (k_steps, k_adj_segment).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -32,6 +34,7 @@
 #include "mj_device.cuh"
 #include "mj_internal.hpp"
 #include "mj_stencil.cuh"
+#include "mj_steps_impl.cuh"
 #include "mj_tiled_impl.cuh"
 
 namespace mj {
@@ -566,6 +569,141 @@ __global__ void __launch_bounds__(32 * BYT) k_tadj_b(const __grid_constant__ Ste
 // tile shape of the tiled backward: 32 x 8 sites, one per thread
 constexpr int kTBYT = 8, kTRY = 1;
 
+// The backward steps of a whole segment in one launch, on lattices whose tiles
+// are all resident at once: the scheme of mj_steps_impl.cuh (a block keeps its
+// tile, waits for its eight neighbours alone, cooperative launch, bounded
+// waits).  What a backward step hands to the neighbours is gH2, then gH1; dL/dm,
+// the stage-2 gradients and the field gradient stay in the thread's registers,
+// and so do the thread's shares of the term gradients: kept in memory from one
+// segment to the next and reduced over the grid once, after the last (so the
+// sums do not depend on the checkpoint spacing).  m_n and mb of a step come from the recomputed segment, so
+// their tiles, the two fields and the draw are ready before the wait.
+// Bound by the chain of its two exchanges: 256^2 square, 3 terms, 8.6 us a step,
+// 21.6 us with the two launches (10.9 + 10.7); a forward and backward sweep of
+// 200 steps with checkpoints every 50 10.0 -> 4.6 ms.
+struct SegArgs {
+    const double* g_in;  // dL/dm entering the segment's last step (or its part without W gH1)
+    int with_gH1;        // 1: gH1 of the step after holds the missing part
+    const double* m0;    // m_n of the segment's first step, step k > 0's at segm + k n3
+    const double* segm;
+    const double* segb;  // mb of step k at + k n3
+    int len;
+    uint32_t step0;      // index of the segment's first step
+    double *gH1, *gH2, *mpart, *gb;
+    double* acc;         // the threads' term gradients, [nterm][threads of the launch]
+    int acc_in;          // 1: they hold the segments before
+    int reduce;          // 1: the last segment, reduce them into R
+    const double* bmap;
+    const double* unit;
+    unsigned int* flags;
+    int* status;
+    AdjReduce R;
+};
+
+template <class S>
+__global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_constant__ StencilParams P,
+                                                              const __grid_constant__ DynCoef C, const TermMasks M,
+                                                              const SegArgs A) {
+    using G = TileGeom<S, kTBYT, kTRY>;
+    extern __shared__ __align__(128) double smem_s[];
+    double* tA = smem_s;               // gH2, gH1
+    double* tB = smem_s + 3 * G::NS;   // mb
+    double* tC = smem_s + 6 * G::NS;   // m_n
+    double* Us = smem_s + 9 * G::NS;   // unit tensors
+    const int64_t N = static_cast<int64_t>(P.L[0]) * P.L[1], n3 = 3 * N;
+    const int tid = threadIdx.x + 32 * threadIdx.y;
+    const int x = blockIdx.x * G::TX + threadIdx.x, y = blockIdx.y * G::TY + threadIdx.y;
+    const bool act[1] = {x < P.L[0] && y < P.L[1]};
+    const int64_t i = act[0] ? x + static_cast<int64_t>(P.L[0]) * y : 0;
+    const int base = threadIdx.y * G::PX + threadIdx.x;
+    const int own = base + G::R * G::PX + G::RX;
+    const double3 zero = make_double3(0.0, 0.0, 0.0);
+    for (int q = tid; q < 9 * G::NS; q += 32 * kTBYT) smem_s[q] = 0.0;
+    stage_units<S, kTBYT, kTRY>(A.unit, M, Us);
+    TileRing<S, kTBYT, kTRY> ring;
+    ring.init(P, A.flags);
+    auto put = [&](double* t, double3 v) {
+        if (act[0]) {
+            t[own] = v.x;
+            t[G::NS + own] = v.y;
+            t[2 * G::NS + own] = v.z;
+        }
+    };
+    auto apply = [&](const double* t) {
+        double3 o[1];
+        tiled_apply<S, kTBYT, kTRY>(P, t, base, o);
+        return o[0];
+    };
+    double3 part = act[0] ? ld3(A.g_in, i, N) : zero, gbs = zero;
+    if (act[0] && A.gb) gbs = ld3(A.gb, i, N);
+    const int64_t nthr = static_cast<int64_t>(gridDim.x) * gridDim.y * (32 * kTBYT);
+    const int64_t me = static_cast<int64_t>(blockIdx.x + gridDim.x * blockIdx.y) * (32 * kTBYT) + tid;
+    double acc[kMaxTerms];
+#pragma unroll
+    for (int t = 0; t < kMaxTerms; ++t) acc[t] = t < M.nterm && A.acc_in ? A.acc[t * nthr + me] : 0.0;
+    __syncthreads();
+    if (A.with_gH1) {
+        put(tA, act[0] ? make_double3(__ldcg(A.gH1 + i), __ldcg(A.gH1 + N + i), __ldcg(A.gH1 + 2 * N + i)) : zero);
+        ring.load(A.gH1, N, tA);
+    }
+    unsigned int pass = 0;
+    bool ok = true;               // no wait gave up
+    bool more = A.with_gH1 != 0;  // gH1 of the step after adds to dL/dm
+    for (int k = A.len - 1; k >= 0; --k) {
+        const double* mk = k == 0 ? A.m0 : A.segm + k * n3;
+        const double* bk = A.segb + k * n3;
+        const double3 m0 = act[0] ? ld3(mk, i, N) : zero, b0 = act[0] ? ld3(bk, i, N) : zero;
+        put(tB, b0);
+        put(tC, m0);
+        ring.load(bk, N, tB);
+        ring.load(mk, N, tC);
+        double3 zn = zero;  // Zeeman and thermal field of the site
+        if (act[0]) zn = add3(zeeman(P, A.bmap, i, N), noise(C, A.step0 + static_cast<uint32_t>(k), i, N));
+        __syncthreads();
+        const double3 H2 = add3(apply(tB), zn), H1 = add3(apply(tC), zn);
+        double3 g = part;
+        if (more) {
+            if (pass > 0) {
+                if (!(ok = ring.wait(pass, A.status))) break;
+                ring.load(A.gH1, N, tA);
+                __syncthreads();
+            }
+            g = add3(part, apply(tA));
+        }
+        more = true;
+        const SibGrad s2 = sib_vjp(m0, b0, H2, C.alpha, C.sib_hc, g);
+        __syncthreads();  // the tile of gH1 has been read
+        put(tA, s2.gH);
+        if (act[0]) st3(A.gH2, i, N, s2.gH);
+        ring.publish(++pass);
+        const double3 gh2[1] = {act[0] ? s2.gH : zero};
+        if (M.nterm > 0) tiled_term_grads<S, kTBYT, kTRY>(Us, M, tB, base, gh2, act, acc);
+        if (!(ok = ring.wait(pass, A.status))) break;
+        ring.load(A.gH2, N, tA);
+        __syncthreads();
+        const double3 gy1 = scl3(0.5, add3(s2.gp, apply(tA)));
+        const SibGrad s1 = sib_vjp(m0, m0, H1, C.alpha, C.sib_hc, gy1);
+        part = add3(add3(s2.gm, gy1), add3(s1.gm, s1.gp));
+        if (P.zee_on) gbs = add3(gbs, scl3(P.zc, add3(s1.gH, s2.gH)));
+        __syncthreads();  // the tile of gH2 has been read
+        put(tA, s1.gH);
+        if (act[0]) st3(A.gH1, i, N, s1.gH);
+        ring.publish(++pass);
+        const double3 gh1[1] = {act[0] ? s1.gH : zero};
+        if (M.nterm > 0) tiled_term_grads<S, kTBYT, kTRY>(Us, M, tC, base, gh1, act, acc);
+        __syncthreads();  // the tiles of m_n and mb have been read
+    }
+    // after a timeout the results are invalid, but every block still takes part in the reduction
+    if (act[0] && ok) {
+        st3(A.mpart, i, N, part);
+        if (A.gb) st3(A.gb, i, N, gbs);
+    }
+#pragma unroll
+    for (int t = 0; t < kMaxTerms; ++t)
+        if (t < M.nterm) A.acc[t * nthr + me] = acc[t];
+    if (M.nterm > 0 && A.reduce) term_reduce(acc, M.nterm, A.R.partials, A.R.counter, A.R.slot, A.R.nblocks);
+}
+
 template <class S>
 size_t tadj_smem(int nterm) {
     using G = TileGeom<S, kTBYT, kTRY>;
@@ -576,6 +714,49 @@ template <class S>
 dim3 tadj_grid(const StencilParams& P) {
     using G = TileGeom<S, kTBYT, kTRY>;
     return dim3((P.L[0] + G::TX - 1) / G::TX, (P.L[1] + G::TY - 1) / G::TY, 1);
+}
+
+// the segment launch of the plan's shape; `fits` false when its tiles are not
+// all resident at once (args null: only that question)
+template <class S>
+mj_status segment_shape(const mj_plan* plan, const DynCoef& c, const TermMasks& M, const SegArgs* args, bool& fits,
+                        cudaStream_t s) {
+    using G = TileGeom<S, kTBYT, kTRY>;
+    const size_t sm = sizeof(double) * (9 * G::NS + static_cast<size_t>(M.nterm) * (S::K + 1) * 9);
+    const dim3 grid = tadj_grid<S>(plan->sp);
+    int per_sm = 0;
+    fits = !thin_last_tile<S>(plan->sp) &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_segment<S>, 32 * kTBYT, sm) == cudaSuccess &&
+           static_cast<int64_t>(grid.x) * grid.y <= static_cast<int64_t>(per_sm) * plan->num_sms;
+    if (!fits || !args) return MJ_OK;
+    mj_status st = cuda_status(cudaMemsetAsync(args->flags, 0,
+                                               sizeof(unsigned int) * kStepsFlagStride * grid.x * grid.y, s),
+                               "segment counters");
+    if (st != MJ_OK) return st;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32, kTBYT);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, k_adj_segment<S>, plan->sp, c, M, *args), "k_adj_segment");
+}
+
+mj_status segment_launch(const mj_plan* plan, const DynCoef& c, const TermMasks& M, const SegArgs* args, bool& fits,
+                         cudaStream_t s) {
+    fits = false;
+    if (plan->sp.L[2] != 1) return MJ_OK;
+    switch (plan->sp.shape) {
+        case kShapeSquareNN: return segment_shape<ShapeSquareNN>(plan, c, M, args, fits, s);
+        case kShapeSquare2: return segment_shape<ShapeSquare2>(plan, c, M, args, fits, s);
+        case kShapeTriNN: return segment_shape<ShapeTriNN>(plan, c, M, args, fits, s);
+        case kShapeTri3: return segment_shape<ShapeTri3>(plan, c, M, args, fits, s);
+        default: return MJ_OK;
+    }
 }
 
 struct CaArgs {
@@ -744,6 +925,8 @@ struct mj_adjoint {
     double* d_g0 = nullptr;     // outputs of the backward sweep (copied to the caller's buffers)
     double* d_gterms = nullptr; // kMaxTerms
     double* d_gb = nullptr;     // 3N
+    double* d_acc = nullptr;          // the threads' term gradients between segment launches
+    unsigned int* d_flags = nullptr;  // tile counters of the many-step launches (null: the lattice is too large)
     // the two sweeps as CUDA graphs over the buffers above, cached with their key
     cudaStream_t cap = nullptr;
     cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
@@ -774,6 +957,8 @@ void adjoint_free(mj_adjoint* a) {
     cudaFree(a->d_partials);
     cudaFree(a->d_counter);
     cudaFree(a->d_slots);
+    cudaFree(a->d_flags);
+    cudaFree(a->d_acc);
     delete a;
 }
 
@@ -809,12 +994,37 @@ void stage2(mj_plan* plan, const DynCoef& c, uint32_t step, const double* m, con
     k_adj_f2<<<adj_grid(plan->sp), dim3(kABX, kABY), 0, s>>>(plan->sp, c, step, plan->d_bmap, m, mb, out);
 }
 
+// whether the plan's SIB steps run many in one launch (mj_steps_impl.cuh)
+bool steps_fit(const mj_adjoint* a, const DynCoef& c, cudaStream_t s) {
+    bool fits = false;
+    int warps = 0;
+    if (a->d_flags && a->plan->steps_together && launch_steps(a->plan, nullptr, c, &warps, fits, s) != MJ_OK) fits = false;
+    return fits;
+}
+
 // forward sweep from checkpoint 0 (already holding m_0) to checkpoint nseg
 void forward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, cudaStream_t s) {
     mj_plan* plan = a->plan;
     const int64_t n3 = 3 * a->N;
     double* mid = a->d_work + 2 * n3;
     const int E = a->every;
+    if (steps_fit(a, c, s)) {  // one launch per segment
+        for (int seg = 0; seg < a->nseg; ++seg) {
+            StepsJob j;
+            std::memset(&j, 0, sizeof(j));
+            j.m_in = ckpt(a, seg);
+            j.m = a->d_work;
+            j.mid = mid;
+            j.m_out = ckpt(a, seg + 1);
+            j.nsteps = std::min(E, a->nsteps - seg * E);
+            j.step0 = step0 + static_cast<uint32_t>(seg * E);
+            j.flags = a->d_flags;
+            int warps = 0;
+            bool fits = false;
+            launch_steps(plan, &j, c, &warps, fits, s);
+        }
+        return;
+    }
     for (int32_t k = 0; k < a->nsteps; ++k) {
         const double* src = (k % E == 0) ? ckpt(a, k / E) : a->d_work + (k % 2) * n3;
         const bool bound = ((k + 1) % E == 0) || (k + 1 == a->nsteps);
@@ -837,15 +1047,63 @@ void backward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, bool wan
     const int E = a->every;
     int slot = 0;
     bool first = true;
+    const bool together = steps_fit(a, c, s);
+    bool segments = false;  // the backward steps of a segment in one launch
+    if (a->d_flags && plan->steps_together && segment_launch(plan, c, M, nullptr, segments, s) != MJ_OK) segments = false;
     for (int seg = a->nseg - 1; seg >= 0; --seg) {
         const int s0 = seg * E;
         const int len = std::min(E, a->nsteps - s0);
         // recompute the segment: m_n (slot 0 = the checkpoint) and mb of every step
         auto segm = [&](int k) -> double* { return k == 0 ? ckpt(a, seg) : a->d_segm + k * n3; };
-        for (int k = 0; k < len; ++k) {
+        if (together) {
+            StepsJob j;
+            std::memset(&j, 0, sizeof(j));
+            j.m_in = ckpt(a, seg);
+            j.m = a->d_segm;
+            j.m_stride = n3;
+            j.mid = a->d_segb;
+            j.mid_stride = n3;
+            j.m_out = a->d_work;  // not reached: the last step is its predictor
+            j.nsteps = len;
+            j.step0 = step0 + static_cast<uint32_t>(s0);
+            j.half = 1;
+            j.flags = a->d_flags;
+            int warps = 0;
+            bool fits = false;
+            launch_steps(plan, &j, c, &warps, fits, s);
+        }
+        for (int k = 0; k < len && !together; ++k) {
             const uint32_t step = step0 + static_cast<uint32_t>(s0 + k);
             stage1(plan, c, step, segm(k), a->d_segb + k * n3, s);
             if (k + 1 < len) stage2(plan, c, step, segm(k), a->d_segb + k * n3, segm(k + 1), s);
+        }
+        if (segments) {
+            SegArgs g;
+            std::memset(&g, 0, sizeof(g));
+            g.g_in = first ? a->d_gin : a->d_mpart;
+            g.with_gH1 = first ? 0 : 1;
+            g.m0 = ckpt(a, seg);
+            g.segm = a->d_segm;
+            g.segb = a->d_segb;
+            g.len = len;
+            g.step0 = step0 + static_cast<uint32_t>(s0);
+            g.gH1 = a->d_gH1;
+            g.gH2 = a->d_gH2;
+            g.mpart = a->d_mpart;
+            g.gb = gb;
+            g.bmap = plan->d_bmap;
+            g.unit = plan->d_unit;
+            g.flags = a->d_flags;
+            g.status = plan->d_status;
+            g.acc = a->d_acc;
+            g.acc_in = first ? 0 : 1;
+            g.reduce = seg == 0;
+            if (g.reduce) slot = 1;
+            g.R = AdjReduce{a->d_partials, a->d_counter, a->d_slots, a->nblocks};
+            bool fits = false;
+            segment_launch(plan, c, M, &g, fits, s);
+            first = false;
+            continue;
         }
         for (int k = len - 1; k >= 0; --k) {
             const uint32_t step = step0 + static_cast<uint32_t>(s0 + k);
@@ -879,7 +1137,7 @@ std::string sweep_key(const mj_adjoint* a, const DynCoef& c, uint32_t step0, int
     k.append(reinterpret_cast<const char*>(&a->plan->sp), sizeof(StencilParams));
     const void* ptrs[2] = {a->plan->d_bmap, a->plan->d_unit};
     k.append(reinterpret_cast<const char*>(ptrs), sizeof(ptrs));
-    k += "/" + std::to_string(step0) + "/" + std::to_string(flags);
+    k += "/" + std::to_string(step0) + "/" + std::to_string(flags) + "/" + std::to_string(a->plan->steps_together);
     return k;
 }
 
@@ -1040,6 +1298,13 @@ mj_status mj_adjoint_create(mj_plan* plan, int32_t nsteps, int32_t checkpoint_ev
         return st;
     }
     cudaMemset(a->d_counter, 0, sizeof(unsigned int) * 4);
+    const int64_t flags = steps_flag_words(plan);
+    const size_t nacc = static_cast<size_t>(plan_nterm(plan)) * a->nblocks * (kABX * kABY);
+    if (flags > 0 && ((st = al(&a->d_flags, sizeof(unsigned int) * flags, "adjoint tile counters")) != MJ_OK ||
+                      (nacc > 0 && (st = al(&a->d_acc, sizeof(double) * nacc, "adjoint term sums")) != MJ_OK))) {
+        adjoint_free(a);
+        return st;
+    }
     if ((st = cuda_status(cudaDeviceSynchronize(), "adjoint create")) != MJ_OK) {
         adjoint_free(a);
         return st;
