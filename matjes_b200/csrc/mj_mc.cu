@@ -21,10 +21,19 @@
 namespace mj {
 namespace {
 
+// The chain's state on the device during a call: accepted moves, the running
+// totals (E, summed spins), the cone and its cosine (updated after every sweep).
+struct McChain {
+    unsigned long long acc;
+    unsigned int counter[2];
+    double run[4];
+    double cone, cos_cone;
+};
+
 struct McCoef {
     double kT;          // eV
     double inv_kT;      // 1/kT (0 at T = 0)
-    double cos_cone;
+    McChain* chain;
     const double* tab;  // sin/cos tables (the plan's thermal-draw tables)
     double* track;      // tracked totals: per-block partials [4][track_n] of (dE, dm) of accepted moves, or null
     int track_n;        // partials per component (colours x blocks of a sweep)
@@ -38,8 +47,7 @@ struct McCoef {
 // S: the plan's compile-time stencil shape, void for runtime offsets
 template <class S>
 __global__ void __launch_bounds__(32 * kMcBY, 8) k_mc_color(const __grid_constant__ StencilParams P, const double* __restrict__ bmap,
-                                                  double* m, const McCoef C, const McClass K,
-                                                  unsigned long long* accepted) {
+                                                  double* m, const McCoef C, const McClass K) {
     const int y = K.ry + K.sy * static_cast<int>(blockIdx.y * kMcBY + threadIdx.y);
     const int z = K.rz + K.sz * static_cast<int>(blockIdx.z);
     const int x = mc_class_x(K, y, z, static_cast<int>(blockIdx.x * 32 + threadIdx.x));
@@ -52,7 +60,7 @@ __global__ void __launch_bounds__(32 * kMcBY, 8) k_mc_color(const __grid_constan
         const double3 s = ld3(m, i, N);
         const double3 Pf = pair_field<S>(P, m, N, P.L[0], P.L[1], P.L[2], x, y, z);
         double3 sn;
-        acc = mc_move(P, C.keys, C.tab, C.proposal, C.kT, C.inv_kT, C.cos_cone, static_cast<uint32_t>(i), C.sweep,
+        acc = mc_move(P, C.keys, C.tab, C.proposal, C.kT, C.inv_kT, __ldg(&C.chain->cos_cone), static_cast<uint32_t>(i), C.sweep,
                       C.stream, s, Pf, zeeman(P, bmap, i, N), sn, dE);
         if (acc) {
             st3(m, i, N, sn);
@@ -66,7 +74,7 @@ __global__ void __launch_bounds__(32 * kMcBY, 8) k_mc_color(const __grid_constan
     }
     // accepted moves of the block, added once per block (an integer sum: any order gives the same count)
     const int n = __syncthreads_count(acc);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && n) atomicAdd(accepted, static_cast<unsigned long long>(n));
+    if (threadIdx.x == 0 && threadIdx.y == 0 && n) atomicAdd(&C.chain->acc, static_cast<unsigned long long>(n));
 }
 
 // sum of the spins (per-block partials summed in block order by the last block)
@@ -82,18 +90,44 @@ __global__ void __launch_bounds__(256) k_mc_magnetisation(const double* __restri
     grid_reduce<3>(v, partials, counter, out, nblocks);
 }
 
-// the totals after a sweep: run = (E, Mx, My, Mz) plus the sweep's partials,
-// summed in a fixed order; copied to E_out / M_out when given
-__global__ void __launch_bounds__(256) k_mc_track(const double* partials, int n, double* run, double* E_out,
-                                                  double* M_out) {
-    __shared__ double sum[4];
-    ordered_sum<4>(partials, n, sum);
+// The end of a sweep, one launch instead of a one-block sum and a host round
+// trip: block q < 4 (with partials) adds component q of the sweep's partials, in
+// a fixed order, to the running total and copies it to E_out / M_out when given;
+// the last block applies the cone rule of sample_sphere (track_value.f90
+// cone_update: +-1e-4 per move toward an acceptance rate of 0.5, cone in
+// [0.01, pi]) to the sweep's number of moves and the running rate.  1024^2, cone
+// adapted and totals recorded after every sweep: 2.6 us, where the one-block sum
+// took 15 and the round trip for the host's cone rule about 20; a sweep 82 -> 51 us.
+constexpr int kMcEndThreads = 1024;
+__global__ void __launch_bounds__(kMcEndThreads) k_mc_sweep_end(const double* __restrict__ partials, int n, McChain* chain,
+                                                                double* E_out, double* M_out, int adapt,
+                                                                long long accepted0, long long proposed, double step) {
+    if (blockIdx.x + 1 == gridDim.x) {
+        if (threadIdx.x == 0 && adapt) {
+            const double rate = static_cast<double>(accepted0 + static_cast<long long>(chain->acc)) / static_cast<double>(proposed);
+            double c = chain->cone;
+            if (rate > 0.5 && c < kPi) c = fmin(kPi, __dadd_rn(c, step));
+            else if (rate < 0.5 && c > 0.01) c = fmax(0.01, __dsub_rn(c, step));
+            chain->cone = c;
+            chain->cos_cone = cos(c);
+        }
+        return;
+    }
+    const int q = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __shared__ double wsum[kMcEndThreads / 32];
+    double s = 0.0;
+    for (int b = threadIdx.x; b < n; b += kMcEndThreads) s += __ldcg(partials + static_cast<int64_t>(q) * n + b);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) wsum[wid] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < 4; ++q) run[q] += sum[q];
-        if (E_out) *E_out = run[0];
-        if (M_out)
-            for (int q = 0; q < 3; ++q) M_out[q] = run[1 + q];
+    if (wid != 0) return;
+    s = wsum[lane];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        const double t = chain->run[q] + s;
+        chain->run[q] = t;
+        if (q == 0 && E_out) *E_out = t;
+        if (q > 0 && M_out) M_out[q - 1] = t;
     }
 }
 
@@ -129,17 +163,12 @@ mj_status mj_mc_sweeps(mj_plan* plan, double* m, mj_mc_params* p, int32_t nsweep
     const int nbc = static_cast<int>(grid.x * grid.y * grid.z);  // blocks of one colour pass
     const int ncol = static_cast<int>(classes.size());
     const bool track = p->track_totals && (E_dev || M_dev);
-    // the call's scratch: accepted count, ticket counter, running totals (E, M);
-    // magnetisation partials; the tracked totals' per-block partials
-    struct Scratch {
-        unsigned long long acc;
-        unsigned int counter[2];
-        double run[4];
-    };
-    Scratch* d_scr = nullptr;
+    // the call's scratch: the chain's state; magnetisation partials; the tracked
+    // totals' per-block partials
+    McChain* d_scr = nullptr;
     double* d_part = nullptr;
     double* d_track = nullptr;
-    mj_status st = cuda_status(cudaMalloc(&d_scr, sizeof(Scratch)), "MC scratch");
+    mj_status st = cuda_status(cudaMalloc(&d_scr, sizeof(McChain)), "MC scratch");
     if (st == MJ_OK && (M_dev || track)) st = cuda_status(cudaMalloc(&d_part, sizeof(double) * 3 * nbm), "MC scratch");
     if (st == MJ_OK && track)
         st = cuda_status(cudaMalloc(&d_track, sizeof(double) * 4 * static_cast<size_t>(ncol) * nbc), "MC scratch");
@@ -148,7 +177,11 @@ mj_status mj_mc_sweeps(mj_plan* plan, double* m, mj_mc_params* p, int32_t nsweep
         cudaFree(d_scr);
         return st;
     }
-    cudaMemsetAsync(d_scr, 0, sizeof(Scratch), s);
+    McChain chain;
+    std::memset(&chain, 0, sizeof(chain));
+    chain.cone = p->cone;
+    chain.cos_cone = std::cos(p->cone);
+    cudaMemcpyAsync(d_scr, &chain, sizeof(chain), cudaMemcpyHostToDevice, s);
     if (track) {  // the totals at the start of the call
         if ((st = launch_energy(plan, m, &d_scr->run[0], s)) == MJ_OK) {
             k_mc_magnetisation<<<nbm, 256, 0, s>>>(m, N, d_part, d_scr->counter, &d_scr->run[1], nbm);
@@ -169,70 +202,61 @@ mj_status mj_mc_sweeps(mj_plan* plan, double* m, mj_mc_params* p, int32_t nsweep
     C.proposal = p->proposal;
     C.stream = p->stream_id;
     mc_keys(p->seed, C.keys);
+    C.chain = d_scr;
     C.track = d_track;
     C.track_n = ncol * nbc;
-    // the cone rule of sample_sphere (track_value.f90 cone_update: +-1e-4 per move
-    // toward an acceptance rate of 0.5, cone in [0.01, pi]), applied once per
-    // sweep with the sweep's number of moves and the running rate
+    // the adaptive cone's step per sweep; its rule runs on the device (k_mc_sweep_end)
     const bool adapt = p->adapt_cone && p->proposal == MJ_MC_CONE;
-    int64_t total = 0;
-    unsigned long long h_acc = 0;
-    auto drain = [&]() -> mj_status {  // accepted moves since the last drain
-        mj_status e = cuda_status(cudaMemcpyAsync(&h_acc, &d_scr->acc, sizeof(h_acc), cudaMemcpyDeviceToHost, s),
-                                  "MC counters");
-        if (e == MJ_OK) e = cuda_status(cudaStreamSynchronize(s), "MC sweeps");
-        if (e == MJ_OK) e = cuda_status(cudaMemsetAsync(&d_scr->acc, 0, sizeof(h_acc), s), "MC counters");
-        total += static_cast<int64_t>(h_acc);
-        p->accepted_total += static_cast<int64_t>(h_acc);
-        return e;
-    };
+    const double cone_step = 1e-4 * static_cast<double>(N);
+    const int64_t proposed0 = p->proposed_total;
     for (int32_t k = 0; k < nsweeps && st == MJ_OK; ++k) {
         C.sweep = p->sweep0 + static_cast<uint32_t>(k);
-        C.cos_cone = std::cos(p->cone);
         for (int ci = 0; ci < ncol; ++ci) {
             const McClass& K = classes[ci];
             C.track_off = ci * nbc;
             switch (plan->sp.shape) {
                 case kShapeSquareNN:
-                    k_mc_color<ShapeSquareNN><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K, &d_scr->acc);
+                    k_mc_color<ShapeSquareNN><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K);
                     break;
                 case kShapeSquare2:
-                    k_mc_color<ShapeSquare2><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K, &d_scr->acc);
+                    k_mc_color<ShapeSquare2><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K);
                     break;
                 case kShapeTriNN:
-                    k_mc_color<ShapeTriNN><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K, &d_scr->acc);
+                    k_mc_color<ShapeTriNN><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K);
                     break;
                 case kShapeTri3:
-                    k_mc_color<ShapeTri3><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K, &d_scr->acc);
+                    k_mc_color<ShapeTri3><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K);
                     break;
                 default:
-                    k_mc_color<void><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K, &d_scr->acc);
+                    k_mc_color<void><<<grid, blk, 0, s>>>(plan->sp, plan->d_bmap, m, C, K);
             }
         }
         if ((st = cuda_status(cudaGetLastError(), "k_mc_color")) != MJ_OK) break;
-        if (track) {
-            k_mc_track<<<1, 256, 0, s>>>(d_track, ncol * nbc, d_scr->run, E_dev ? E_dev + k : nullptr,
-                                         M_dev ? M_dev + 3 * k : nullptr);
-            if ((st = cuda_status(cudaGetLastError(), "k_mc_track")) != MJ_OK) break;
-        } else if (E_dev && (st = launch_energy(plan, m, E_dev + k, s)) != MJ_OK) {
-            break;
+        if (track || adapt) {
+            k_mc_sweep_end<<<track ? 5 : 1, kMcEndThreads, 0, s>>>(
+                d_track, ncol * nbc, d_scr, E_dev ? E_dev + k : nullptr, M_dev ? M_dev + 3 * k : nullptr, adapt ? 1 : 0,
+                static_cast<long long>(p->accepted_total), static_cast<long long>(proposed0 + N * (k + 1)), cone_step);
+            if ((st = cuda_status(cudaGetLastError(), "k_mc_sweep_end")) != MJ_OK) break;
         }
+        if (!track && E_dev && (st = launch_energy(plan, m, E_dev + k, s)) != MJ_OK) break;
         if (M_dev && !track) {
             k_mc_magnetisation<<<nbm, 256, 0, s>>>(m, N, d_part, d_scr->counter, M_dev + 3 * k, nbm);
             if ((st = cuda_status(cudaGetLastError(), "k_mc_magnetisation")) != MJ_OK) break;
         }
-        p->proposed_total += N;
-        if (adapt) {
-            if ((st = drain()) != MJ_OK) break;
-            const double rate = static_cast<double>(p->accepted_total) / static_cast<double>(p->proposed_total);
-            const double step = 1e-4 * static_cast<double>(N);
-            if (rate > 0.5 && p->cone < kPi) p->cone = std::min(kPi, p->cone + step);
-            else if (rate < 0.5 && p->cone > 0.01) p->cone = std::max(0.01, p->cone - step);
-        }
     }
-    if (st == MJ_OK && !adapt) st = drain();
-    if (accepted) *accepted = total;
-    if (st == MJ_OK) p->sweep0 += static_cast<uint32_t>(nsweeps);
+    // the counts and the cone back (the call returns after its sweeps)
+    if (st == MJ_OK) {
+        st = cuda_status(cudaMemcpyAsync(&chain, d_scr, sizeof(chain), cudaMemcpyDeviceToHost, s), "MC counters");
+        const mj_status sy = cuda_status(cudaStreamSynchronize(s), "MC sweeps");
+        if (st == MJ_OK) st = sy;
+    }
+    if (st == MJ_OK) {
+        p->accepted_total += static_cast<int64_t>(chain.acc);
+        p->proposed_total += N * nsweeps;
+        if (adapt) p->cone = chain.cone;
+        p->sweep0 += static_cast<uint32_t>(nsweeps);
+        if (accepted) *accepted = static_cast<int64_t>(chain.acc);
+    }
     cudaFree(d_track);
     cudaFree(d_part);
     cudaFree(d_scr);

@@ -37,18 +37,20 @@ __device__ __forceinline__ double3 cone_proposal(double3 s, double cos_cone, dou
     const double st = sqrt(1.0 - ct * ct);
     const double cti = s.z;
     const double rxy2 = s.x * s.x + s.y * s.y;
-    const double sti = sqrt(rxy2);
-    double cpi = 1.0, spi = 0.0;
+    double cpi = 1.0, spi = 0.0, sti;
     if (!(rxy2 < 0.00001)) {
-        const double inv = 1.0 / sti;
+        const double inv = rsqrt(rxy2);  // 1/sin, and sin = sin^2 / sin
+        sti = rxy2 * inv;
         cpi = s.x * inv;
         spi = s.y * inv;
+    } else {
+        sti = sqrt(rxy2);
     }
     double sph, cph;
     sincos2pi_word(w2, tab, &sph, &cph);
     const double t = st * sph * cti + ct * sti;
     const double3 n = make_double3(-st * cph * spi + t * cpi, st * cph * cpi + t * spi, -st * sph * sti + ct * cti);
-    const double inv_n = 1.0 / sqrt(dot(n, n));
+    const double inv_n = inv_norm(dot(n, n));  // a rotated unit vector: |n| = 1 to rounding
     return make_double3(n.x * inv_n, n.y * inv_n, n.z * inv_n);
 }
 
@@ -78,13 +80,14 @@ __device__ __forceinline__ void pair_term(const StencilParams& P, const double* 
                                           int Ly, int x, int y, int64_t layer, double3& b) {
     constexpr int dx = S::DX[k], dy = S::DY[k];
     int nx = x + dx, ny = y + dy;
-    if (nx < 0 || nx >= Lx) {
+    // (an offset of compile-time sign leaves by one edge alone)
+    if (dx < 0 ? nx < 0 : (dx > 0 && nx >= Lx)) {
         if (!P.periodic[0]) return;
-        nx = wrap(nx, Lx);
+        nx = Lx > S::R ? (dx < 0 ? nx + Lx : nx - Lx) : wrap(nx, Lx);
     }
-    if (ny < 0 || ny >= Ly) {
+    if (dy < 0 ? ny < 0 : (dy > 0 && ny >= Ly)) {
         if (!P.periodic[1]) return;
-        ny = wrap(ny, Ly);
+        ny = Ly > S::R ? (dy < 0 ? ny + Ly : ny - Ly) : wrap(ny, Ly);
     }
     const double3 v = ld3(m, layer + nx + static_cast<int64_t>(Lx) * ny, Ntot);
     if constexpr (S::ISO[k] != 0) {
@@ -123,9 +126,10 @@ __device__ __forceinline__ double3 pair_field(const StencilParams& P, const doub
     return b;
 }
 
-__device__ __forceinline__ double onsite_energy(const StencilParams& P, double3 s) {
+// the on-site part of dE: -(s'.W0 s' - s.W0 s)/2 = -(s' - s).W0 (s' + s)/2, W0 symmetric
+__device__ __forceinline__ double onsite_change(const StencilParams& P, double3 s, double3 sn, double3 d) {
     if (!P.has_onsite) return 0.0;
-    return -0.5 * dot(s, mat3(P.W0, s, make_double3(0.0, 0.0, 0.0)));
+    return -0.5 * dot(d, mat3(P.W0, add3(s, sn), make_double3(0.0, 0.0, 0.0)));
 }
 
 // the proposal of a move (track_value.f90 sample_*); B the site's effective field
@@ -152,13 +156,18 @@ __device__ __forceinline__ bool mc_move(const StencilParams& P, const uint32_t* 
                                         double3& sn, double& dE) {
     uint32_t c[4] = {site, sweep, stream, kMcTag};
     philox10k(c, keys);
-    double3 B = add3(Pf, zb);
-    if (P.has_onsite) B = mat3(P.W0, s, B);
+    double3 B = make_double3(0.0, 0.0, 0.0);
+    if (proposal == MJ_MC_UNDERRELAX || proposal == MJ_MC_OVERRELAX) {
+        B = add3(Pf, zb);
+        if (P.has_onsite) B = mat3(P.W0, s, B);
+    }
     sn = propose(proposal, s, B, cos_cone, c, tab);
     const double3 d = make_double3(sn.x - s.x, sn.y - s.y, sn.z - s.z);
-    dE = -dot(d, Pf) + (onsite_energy(P, sn) - onsite_energy(P, s)) - dot(d, zb);
+    dE = -dot(d, add3(Pf, zb)) + onsite_change(P, s, sn, d);
+    // u < exp(max(-dE/kT, -200)) as ln u < -dE/kT (ln u >= -33 ln 2: the bound of
+    // -200 never decides), with the logarithm of the thermal draw's tables
     bool acc = dE < 0.0;
-    if (!acc && kT > 0.0) acc = u32_open(c[2]) < exp(fmax(-dE * inv_kT, -200.0));
+    if (!acc && kT > 0.0) acc = tab_log(u32_half(c[2]), tab) < -dE * inv_kT;
     return acc;
 }
 
