@@ -12,6 +12,7 @@
 //
 // The passes are templates over a field provider: StencilField (single-atom
 // cells; neighbour offsets and 3x3 tensors in the launch parameters),
+// CubicField (its six nearest neighbours in three dimensions, unrolled),
 // EllIdField (multi-atom cells and COO input with few distinct tensors;
 // per-site lists of column and tensor id) or EllField (any COO input; per-site
 // tensor lists).  Every thread of a block calls begin() before the site test.
@@ -99,6 +100,101 @@ struct StencilField {
     }
 };
 
+// Simple-cubic nearest neighbours (+-x, +-y, +-z and no other offset): the bulk
+// crystal and the films of several layers.  The run-time offset loop above
+// resolves three wraps per neighbour and waits for its loads one neighbour at a
+// time; here the six indices are selects and their 18 loads go out together.
+// SP_AXIAL (as in mj_tiled_impl.cuh): the in-plane tensors have W[0][1] = W[1][0]
+// = 0, the z bonds are isotropic, the on-site tensor is its zz entry alone.  The
+// neighbours are added in the order of the plan's offsets, so the field is the
+// offset loop's bit for bit.  Bound by instruction issue and the L2 (the
+// neighbouring rows and layers come from there).  96 x 96 x 97 periodic at 10 K:
+// a SIB step 48.6 us with the energy, 78.3 with the offset loop and a second draw
+// (passes 26.7 + 19.4 us against 41.9 + 31.8).
+enum { CUBIC_FULL = 0, CUBIC_AXIAL = 1 };
+template <int SP>
+struct CubicField {
+    int L[3], periodic[3];
+    double W[6][9];  // -z +z -y +y -x +x
+    double W0[9];
+    double zc, bext[3];
+    int has_onsite, zee_on;
+    const double* bmap;
+
+    static constexpr int BX = StencilField::BX, BY = StencilField::BY;
+    __device__ __forceinline__ void begin() const {}
+    __device__ __forceinline__ int64_t nsites() const { return static_cast<int64_t>(L[0]) * L[1] * L[2]; }
+    __device__ __forceinline__ bool site(int64_t& i, int& x, int& y, int& z) const {
+        x = blockIdx.x * BX + threadIdx.x;
+        y = blockIdx.y * BY + threadIdx.y;
+        z = blockIdx.z;
+        const bool a = x < L[0] && y < L[1];
+        i = a ? x + static_cast<int64_t>(L[0]) * (y + static_cast<int64_t>(L[1]) * z) : 0;
+        return a;
+    }
+    __device__ __forceinline__ FieldOut field(const double* __restrict__ m, int64_t i, int x, int y, int z, double3 m0) const {
+        const int64_t N = nsites();
+        const int64_t sx = 1, sy = L[0], sz = static_cast<int64_t>(L[0]) * L[1];
+        // neighbour indices (the site itself past an open edge, not used there)
+        int64_t j[6];
+        bool in[6];
+        auto pair = [&](int q, int d, int v, int64_t stride) {
+            const int n = L[d];
+            const bool up = v + 1 < n, dn = v > 0;
+            in[q] = dn || periodic[d];
+            in[q + 1] = up || periodic[d];
+            j[q] = dn ? i - stride : (periodic[d] ? i + stride * (n - 1) : i);
+            j[q + 1] = up ? i + stride : (periodic[d] ? i - stride * (n - 1) : i);
+        };
+        pair(0, 2, z, sz);
+        pair(2, 1, y, sy);
+        pair(4, 0, x, sx);
+        double3 a[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a[k] = ld3(m, j[k], N);
+        double bx = 0.0, by = 0.0, bz = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            if (!in[k]) continue;
+            const double* w = W[k];
+            if constexpr (SP == CUBIC_AXIAL) {
+                if (k < 2) {
+                    bx = fma(w[0], a[k].x, bx);
+                    by = fma(w[0], a[k].y, by);
+                    bz = fma(w[0], a[k].z, bz);
+                } else {
+                    bx = fma(w[0], a[k].x, fma(w[2], a[k].z, bx));
+                    by = fma(w[4], a[k].y, fma(w[5], a[k].z, by));
+                    bz = fma(w[6], a[k].x, fma(w[7], a[k].y, fma(w[8], a[k].z, bz)));
+                }
+            } else {
+                bx = fma(w[0], a[k].x, fma(w[1], a[k].y, fma(w[2], a[k].z, bx)));
+                by = fma(w[3], a[k].x, fma(w[4], a[k].y, fma(w[5], a[k].z, by)));
+                bz = fma(w[6], a[k].x, fma(w[7], a[k].y, fma(w[8], a[k].z, bz)));
+            }
+        }
+        if (has_onsite) {
+            if constexpr (SP == CUBIC_AXIAL) {
+                bz = fma(W0[8], m0.z, bz);
+            } else {
+                bx = fma(W0[0], m0.x, fma(W0[1], m0.y, fma(W0[2], m0.z, bx)));
+                by = fma(W0[3], m0.x, fma(W0[4], m0.y, fma(W0[5], m0.z, by)));
+                bz = fma(W0[6], m0.x, fma(W0[7], m0.y, fma(W0[8], m0.z, bz)));
+            }
+        }
+        FieldOut f;
+        f.Bzee = make_double3(0.0, 0.0, 0.0);
+        if (zee_on) {
+            double3 b;
+            if (bmap) b = make_double3(__ldg(bmap + i), __ldg(bmap + N + i), __ldg(bmap + 2 * N + i));
+            else b = make_double3(bext[0], bext[1], bext[2]);
+            f.Bzee = make_double3(zc * b.x, zc * b.y, zc * b.z);
+        }
+        f.B = make_double3(bx + f.Bzee.x, by + f.Bzee.y, bz + f.Bzee.z);
+        return f;
+    }
+};
+
 // What the two ELL forms share: one site per thread, the Zeeman term per site.
 struct EllSites {
     int64_t N;
@@ -159,7 +255,8 @@ struct EllField : EllSites {
 // the general form's 76, the tensors copied to shared memory once per block
 // (the lanes of a warp read at most one tensor per atom of the cell).
 // 384 x 384 cells of two atoms, 9 entries a site: a SIB step 38.9 us, 109.0 us
-// with the general form (passes 18.4 + 15.5 us against 56.7 + 42.3).
+// with the general form (passes 18.4 + 15.5 us against 56.7 + 42.3); 35.6 us since
+// the corrector reads the predictor's draw.
 struct EllIdField : EllSites {
     int wfull;             // slots of full tensors; the slots after them are isotropic
     int ntensor;
@@ -204,12 +301,23 @@ struct EllIdField : EllSites {
     }
 };
 
+// Energy of a pass.  The first pass of a two-pass step leaves its partials
+// (reduce_part) and the first block of the second pass sums them (reduce_rest),
+// in the fixed order of ordered_sum: no ticket, no last-block tail between them.
 struct Reduce {
     double* partials;
     unsigned int* counter;
     double* out;  // null = no energy wanted
     int nblocks;
 };
+__device__ __forceinline__ void reduce_part(const Reduce& R, double e) {
+    if (!R.out) return;
+    double v[1] = {e};
+    block_partials<1>(v, R.partials, R.nblocks, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+}
+__device__ __forceinline__ void reduce_rest(const Reduce& R) {
+    if (R.out && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) ordered_sum<1>(R.partials, R.nblocks, R.out);
+}
 
 __device__ __forceinline__ double3 minus2(double3 B, double3 hd) {
     return make_double3(B.x - 2.0 * hd.x, B.y - 2.0 * hd.y, B.z - 2.0 * hd.z);
@@ -300,10 +408,7 @@ __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, con
         st3(D1, i, N, D);
         if (C.thermal) st3(DTo, i, N, llg_rhs(thermal_field(C, step, i, N), m0, C.alpha, C.inv_den));
     }
-    if (R.out) {
-        double v[1] = {e};
-        grid_reduce<1>(v, R.partials, R.counter, R.out, R.nblocks);
-    }
+    reduce_part(R, e);
 }
 
 // Heun-Matjes pass 2: corrector restarted from the predictor.
@@ -311,10 +416,11 @@ template <class F>
 __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, const DynCoef C,
                                                const double* __restrict__ mid, const double* __restrict__ D1,
                                                const double* __restrict__ DTi, double* __restrict__ mout,
-                                               const DipView Hd, int* status, const DipPad pad) {
+                                               const DipView Hd, Reduce R, int* status, const DipPad pad) {
     int64_t i;
     int x, y, z;
     fp.begin();
+    reduce_rest(R);
     if (!fp.site(i, x, y, z)) return;
     const int64_t N = fp.nsites();
     const double3 mt = ld3(mid, i, N);
@@ -335,11 +441,13 @@ __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, con
     if (pad.p) st_pad(pad, x, y, z, mo);
 }
 
-// SIB pass 1: Cayley predictor from m_n with A(m_n); writes the midpoint (m_n + m~)/2.
+// SIB pass 1: Cayley predictor from m_n with A(m_n); writes the midpoint (m_n + m~)/2
+// and, when given a buffer, its Philox draw for the corrector (48 bytes a site
+// written and read back cost less than drawing it again, about 240 instructions).
 template <class F>
 __global__ void __launch_bounds__(256) k_sib1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                               const double* __restrict__ m, double* __restrict__ mid,
-                                              const DipView Hd, Reduce R, const DipPad pad) {
+                                              double* __restrict__ draw, const DipView Hd, Reduce R, const DipPad pad) {
     int64_t i;
     int x, y, z;
     fp.begin();
@@ -354,26 +462,26 @@ __global__ void __launch_bounds__(256) k_sib1(const __grid_constant__ F fp, cons
         double3 H = minus2(f.B, hd);
         if (C.thermal) {
             const double3 b = thermal_field(C, step, i, N);
+            if (draw) st3(draw, i, N, b);
             H = make_double3(H.x + b.x, H.y + b.y, H.z + b.z);
         }
         const double3 mb = sib_solve<true>(m0, m0, H, C.alpha, C.sib_hc);
         st3(mid, i, N, mb);
         if (pad.p) st_pad(pad, x, y, z, mb);
     }
-    if (R.out) {
-        double v[1] = {e};
-        grid_reduce<1>(v, R.partials, R.counter, R.out, R.nblocks);
-    }
+    reduce_part(R, e);
 }
 
 // SIB pass 2: corrector from m_n with A(midpoint); in place (only the own site of m is read).
 template <class F>
 __global__ void __launch_bounds__(256) k_sib2(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
-                                              const double* __restrict__ mid, double* m, const DipView Hd,
-                                              int* status, const DipPad pad) {
+                                              const double* __restrict__ mid, double* m,
+                                              const double* __restrict__ draw, const DipView Hd, Reduce R, int* status,
+                                              const DipPad pad) {
     int64_t i;
     int x, y, z;
     fp.begin();
+    reduce_rest(R);
     if (!fp.site(i, x, y, z)) return;
     const int64_t N = fp.nsites();
     const double3 mb = ld3(mid, i, N);
@@ -381,7 +489,7 @@ __global__ void __launch_bounds__(256) k_sib2(const __grid_constant__ F fp, cons
     const double3 hd = Hd.h ? ld_dip(Hd, x, y, z) : make_double3(0.0, 0.0, 0.0);
     double3 H = minus2(f.B, hd);
     if (C.thermal) {
-        const double3 b = thermal_field(C, step, i, N);
+        const double3 b = draw ? ld3(draw, i, N) : thermal_field(C, step, i, N);
         H = make_double3(H.x + b.x, H.y + b.y, H.z + b.z);
     }
     const double3 m0 = make_double3(m[i], m[N + i], m[2 * N + i]);
@@ -603,18 +711,20 @@ mj_status step_impl(mj_plan* p, const Launch<F>& L, double* m, double* m_out, co
             if (pd.p) p->dip_pad_holds = p->d_mid;
             Hd = dip_field(p, p->d_mid, s, st);
             if (st != MJ_OK) return st;
-            MJ_LAUNCH("k_heun2", k_heun2<F>, L.fp, c, p->d_mid, p->d_aux, p->d_aux2, m, Hd, p->d_status, pd);
+            MJ_LAUNCH("k_heun2", k_heun2<F>, L.fp, c, p->d_mid, p->d_aux, p->d_aux2, m, Hd, make_reduce(p, E_prev),
+                      p->d_status, pd);
             if (pd.p) p->dip_pad_holds = m;
             return MJ_OK;
         }
         case MJ_SIB: {
             DipView Hd = dip_field(p, m, s, st);
             if (st != MJ_OK) return st;
-            MJ_LAUNCH("k_sib1", k_sib1<F>, L.fp, c, step, m, p->d_mid, Hd, make_reduce(p, E_prev), pd);
+            double* draw = (c.thermal && c.noise == MJ_NOISE_PHILOX && p->store_draw) ? p->d_aux : nullptr;
+            MJ_LAUNCH("k_sib1", k_sib1<F>, L.fp, c, step, m, p->d_mid, draw, Hd, make_reduce(p, E_prev), pd);
             if (pd.p) p->dip_pad_holds = p->d_mid;
             Hd = dip_field(p, p->d_mid, s, st);
             if (st != MJ_OK) return st;
-            MJ_LAUNCH("k_sib2", k_sib2<F>, L.fp, c, step, p->d_mid, m, Hd, p->d_status, pd);
+            MJ_LAUNCH("k_sib2", k_sib2<F>, L.fp, c, step, p->d_mid, m, draw, Hd, make_reduce(p, E_prev), p->d_status, pd);
             if (pd.p) p->dip_pad_holds = m;
             return MJ_OK;
         }
@@ -634,6 +744,52 @@ mj_status temperature_impl(mj_plan* p, const Launch<F>& L, const double* m, doub
 
 Launch<StencilField> stencil_launch(const mj_plan* p) {
     return Launch<StencilField>{stencil_of(p), grid_stencil(p->sp), dim3(StencilField::BX, StencilField::BY)};
+}
+// the six nearest neighbours of a simple-cubic lattice in the order that the
+// shells of such a cell give them
+bool is_cubic(const StencilParams& P) {
+    static const int order[6][3] = {{0, 0, -1}, {0, 0, 1}, {0, -1, 0}, {0, 1, 0}, {-1, 0, 0}, {1, 0, 0}};
+    if (P.n_off != 6) return false;
+    for (int k = 0; k < 6; ++k)
+        for (int d = 0; d < 3; ++d)
+            if (P.off[k][d] != order[k][d]) return false;
+    return true;
+}
+bool cubic_axial(const StencilParams& P) {
+    if (!P.iso[0] || !P.iso[1]) return false;
+    for (int k = 2; k < 6; ++k)
+        if (P.W[k][1] != 0.0 || P.W[k][3] != 0.0) return false;
+    if (P.has_onsite)
+        for (int q = 0; q < 8; ++q)
+            if (P.W0[q] != 0.0) return false;
+    return true;
+}
+template <int SP>
+Launch<CubicField<SP>> cubic_launch(const mj_plan* p) {
+    const StencilParams& P = p->sp;
+    CubicField<SP> f;
+    for (int d = 0; d < 3; ++d) {
+        f.L[d] = P.L[d];
+        f.periodic[d] = P.periodic[d];
+        f.bext[d] = P.bext[d];
+    }
+    for (int q = 0; q < 6; ++q)
+        for (int e = 0; e < 9; ++e) f.W[q][e] = P.W[q][e];
+    for (int e = 0; e < 9; ++e) f.W0[e] = P.W0[e];
+    f.zc = P.zc;
+    f.has_onsite = P.has_onsite;
+    f.zee_on = P.zee_on;
+    f.bmap = p->d_bmap;
+    return Launch<CubicField<SP>>{f, grid_stencil(P), dim3(StencilField::BX, StencilField::BY)};
+}
+// f(launch) with the launch of the plan's stencil
+template <class Fn>
+auto with_stencil(const mj_plan* p, Fn&& f) {
+    if (is_cubic(p->sp)) {
+        if (cubic_axial(p->sp)) return f(cubic_launch<CUBIC_AXIAL>(p));
+        return f(cubic_launch<CUBIC_FULL>(p));
+    }
+    return f(stencil_launch(p));
 }
 // f(launch) with the launch of the ELL form the plan holds
 template <class Fn>
@@ -716,7 +872,7 @@ mj_status tiled_step(mj_plan* p, double* m, double* m_out, const DynCoef& c, uin
 
 mj_status launch_field(mj_plan* p, const double* m, double* B, double* e_site, double* E_out, cudaStream_t s) {
     if (tiled(p)) return tiled_field(p, m, B, e_site, E_out, s);
-    if (p->is_stencil) return field_impl(p, stencil_launch(p), m, B, e_site, E_out, s);
+    if (p->is_stencil) return with_stencil(p, [&](const auto& L) { return field_impl(p, L, m, B, e_site, E_out, s); });
     return with_ell(p, [&](const auto& L) { return field_impl(p, L, m, B, e_site, E_out, s); });
 }
 
@@ -727,12 +883,13 @@ mj_status launch_energy(mj_plan* p, const double* m, double* E_out, cudaStream_t
 mj_status launch_step(mj_plan* p, double* m, double* m_out, const DynCoef& c, uint32_t step, double* E_prev_out,
                       cudaStream_t s) {
     if (tiled(p)) return tiled_step(p, m, m_out, c, step, E_prev_out, s);
-    if (p->is_stencil) return step_impl(p, stencil_launch(p), m, m_out, c, step, E_prev_out, s);
+    if (p->is_stencil)
+        return with_stencil(p, [&](const auto& L) { return step_impl(p, L, m, m_out, c, step, E_prev_out, s); });
     return with_ell(p, [&](const auto& L) { return step_impl(p, L, m, m_out, c, step, E_prev_out, s); });
 }
 
 mj_status launch_temperature(mj_plan* p, const double* m, double* out2, cudaStream_t s) {
-    if (p->is_stencil) return temperature_impl(p, stencil_launch(p), m, out2, s);
+    if (p->is_stencil) return with_stencil(p, [&](const auto& L) { return temperature_impl(p, L, m, out2, s); });
     return with_ell(p, [&](const auto& L) { return temperature_impl(p, L, m, out2, s); });
 }
 
