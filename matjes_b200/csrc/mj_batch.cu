@@ -6,8 +6,10 @@
 // z[Ntot], replica r owning sites [off_r, off_r + Lx_r Ly_r).  A replica
 // table (offset, size, Zeeman field, kT, Philox stream, temperature slot) and a
 // tile list (replica, x0, y0), ordered by replica, drive persistent blocks that
-// walk the tiles with a grid stride; each tile runs the same column-walking
-// stencil as the single-lattice tiled kernels (mj_tiled_impl.cuh).  Per-replica
+// walk the tiles with a grid stride, the next tile's cells copied to a second
+// buffer in shared memory (cp.async) while the current one computes; each tile
+// runs the same column-walking stencil as the single-lattice tiled kernels
+// (mj_tiled_impl.cuh).  Per-replica
 // energies are tile partials reduced in tile order (deterministic).
 //
 // Parallel tempering follows the reference's rule (paratemp-MC/paratemp.f90:
@@ -40,9 +42,22 @@ struct BatchRep {
 
 namespace {
 
+// One tile: what staging it needs, so that no block waits for the replica table
+// before it can address its cells.  256 replicas, 5.07 M sites: 239 us a step with
+// the next tile's copies in flight, 252 with plain loads between two barriers
+// (passes 128 + 109 us: the predictor's instruction issue, the corrector's 487 MB).
+struct __align__(16) BatchTile {
+    int64_t off;  // first packed site of the replica
+    int Lx, Ly;
+    int x0, y0;
+    int rep;
+    int pad;
+};
+
 struct BatchArgs {
     const BatchRep* reps;
-    const int4* tiles;  // (replica, x0, y0, -)
+    const BatchTile* tiles;
+    const double* sigma;  // per replica: sqrt(alpha kT hbar / dt), 0 = no thermal field
     int ntile;
     int64_t Ntot;
     const double* ms;   // stencil input (m or midpoint)
@@ -51,7 +66,6 @@ struct BatchArgs {
     double* aux;        // stored Philox draw (SIB)
     double* tile_e;     // per-tile energy, null = none
     uint32_t step;
-    double dt;          // SIB timestep (fs); sigma = sqrt(alpha kT hbar / dt) per replica
     int project;        // field pass: remove the component along m (B - (B.m) m)
     double* tile_g;     // GNEB pass: per-tile path sums (6 x ntile)
     int64_t gneb_n;     // GNEB pass: sites of an image (every replica one image)
@@ -67,36 +81,36 @@ struct BatchArgs {
 // wp^2 |A|^2 + 2 wp wm A.B + wm^2 |B|^2 and F.tau = wp F.A + wm F.B.
 enum { BPASS_ENERGY = 0, BPASS_FIELD = 1, BPASS_GNEB = 2, BPASS_SIB1 = 4, BPASS_SIB2 = 5 };
 
+// cp.async of 8 bytes, or 8 bytes of zeros (ok = false)
+__device__ __forceinline__ void copy8_async(uint32_t dst, const double* src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+
+// the copies of tile T's cells (with halo; zeros across an open edge) into sm, as one group
 template <class S, int BYT, int RY>
-__device__ __forceinline__ void load_tile_b(const StencilParams& P, const BatchRep& R, const double* ms, int64_t Ntot,
-                                            int x0, int y0, double* sm) {
+__device__ __forceinline__ void load_tile_b(const StencilParams& P, const BatchTile& T, const double* ms, int64_t Ntot,
+                                            double* sm) {
     using G = TileGeom<S, BYT, RY>;
-    const int Lx = R.Lx, Ly = R.Ly;
-    const double* mx = ms + R.off;
+    const double* mx = ms + T.off;
     const int tid = threadIdx.x + 32 * threadIdx.y;
+    const uint32_t s0 = smem_u32(sm);
     for (int idx = tid; idx < G::NS; idx += 32 * BYT) {
         const int ly = idx / G::PX;
         const int lx = idx - ly * G::PX;
-        int gx = x0 + lx - G::RX, gy = y0 + ly - G::R;
+        int gx = T.x0 + lx - G::RX, gy = T.y0 + ly - G::R;
         bool ok = true;
-        if (gx < 0 || gx >= Lx) {
-            if (P.periodic[0]) gx = ((gx % Lx) + Lx) % Lx;
+        if (gx < 0 || gx >= T.Lx) {
+            if (P.periodic[0]) gx = wrap(gx, T.Lx);
             else ok = false;
         }
-        if (gy < 0 || gy >= Ly) {
-            if (P.periodic[1]) gy = ((gy % Ly) + Ly) % Ly;
+        if (gy < 0 || gy >= T.Ly) {
+            if (P.periodic[1]) gy = wrap(gy, T.Ly);
             else ok = false;
         }
-        double vx = 0.0, vy = 0.0, vz = 0.0;
-        if (ok) {
-            const int64_t j = gx + static_cast<int64_t>(Lx) * gy;
-            vx = __ldg(mx + j);
-            vy = __ldg(mx + Ntot + j);
-            vz = __ldg(mx + 2 * Ntot + j);
-        }
-        sm[idx] = vx;
-        sm[G::NS + idx] = vy;
-        sm[2 * G::NS + idx] = vz;
+        const double* src = ok ? mx + (gx + static_cast<int64_t>(T.Lx) * gy) : mx;
+        copy8_async(s0 + 8u * idx, src, ok);
+        copy8_async(s0 + 8u * (G::NS + idx), src + Ntot, ok);
+        copy8_async(s0 + 8u * (2 * G::NS + idx), src + 2 * Ntot, ok);
     }
 }
 
@@ -104,15 +118,13 @@ __device__ __forceinline__ void load_tile_b(const StencilParams& P, const BatchR
 // the single-lattice tiled kernels; every replica's field then points along z).
 template <class S, int BYT, int RY, int PASS, int SP = SP_FULL>
 __device__ __forceinline__ double compute_tile_b(const StencilParams& P, const DynCoef& C, const BatchArgs& A,
-                                                 const BatchRep& R, int rep, const double* sm, int x0, int y0,
-                                                 double (&gs)[6]) {
+                                                 const BatchRep& R, int rep, double sigma, const double* sm, int x0,
+                                                 int y0, double (&gs)[6]) {
     using G = TileGeom<S, BYT, RY>;
     const int64_t Nt = A.Ntot;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int x = x0 + tx;
-    // same expression and thermal condition as the single-lattice coefficients
-    const bool thermal = C.thermal && (R.kT * C.alpha > 1e-10) && (R.kT > 1e-8);
-    const double sigma = thermal ? sqrt(C.alpha * R.kT * kHbar / A.dt) : 0.0;
+    const bool thermal = sigma != 0.0;
     Pre pre[RY];
     if constexpr (PASS == BPASS_SIB2) {
 #pragma unroll
@@ -228,23 +240,37 @@ template <class S, int BYT, int RY, int MINB, int PASS, int SP>
 __global__ void __launch_bounds__(32 * BYT, MINB) k_batch(const __grid_constant__ StencilParams P, const DynCoef C,
                                                            const BatchArgs A) {
     using G = TileGeom<S, BYT, RY>;
-    extern __shared__ __align__(128) double smem_b[];
+    extern __shared__ __align__(128) double smem_b[];  // two tile buffers
     // per tile: the energy, and for the GNEB pass its six path sums
     constexpr int NV = PASS == BPASS_GNEB ? 7 : 1;
+    constexpr bool kDraws = PASS == BPASS_SIB1 || PASS == BPASS_SIB2;
     __shared__ double wsum[NV][8];
     if constexpr (PASS == BPASS_GNEB)
         if (A.stop && *A.stop) return;
     BatchArgs Ar = A;
     if (C.step_base) Ar.step = A.step + *C.step_base;
     const int tid = threadIdx.x + 32 * threadIdx.y;
-    for (int t = blockIdx.x; t < A.ntile; t += gridDim.x) {
-        const int4 tl = A.tiles[t];
-        const BatchRep R = A.reps[tl.x];
-        load_tile_b<S, BYT, RY>(P, R, A.ms, A.Ntot, tl.y, tl.z, smem_b);
+    int t = blockIdx.x;
+    if (t >= A.ntile) return;
+    BatchTile cur = A.tiles[t], next = cur;
+    load_tile_b<S, BYT, RY>(P, cur, A.ms, A.Ntot, smem_b);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (t + static_cast<int>(gridDim.x) < A.ntile) next = A.tiles[t + gridDim.x];
+    for (int b = 0; t < A.ntile; t += gridDim.x, b ^= 1) {
+        const double* sm = smem_b + b * G::buf_stride_d;
+        const BatchRep R = A.reps[cur.rep];
+        const double sigma = kDraws ? A.sigma[cur.rep] : 0.0;
+        if (t + static_cast<int>(gridDim.x) < A.ntile)
+            load_tile_b<S, BYT, RY>(P, next, A.ms, A.Ntot, smem_b + (b ^ 1) * G::buf_stride_d);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const BatchTile tl = cur;
+        cur = next;
+        if (t + 2 * static_cast<int>(gridDim.x) < A.ntile) next = A.tiles[t + 2 * gridDim.x];
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
         double v[NV];
         double gs[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        v[0] = compute_tile_b<S, BYT, RY, PASS, SP>(P, C, Ar, R, tl.x, smem_b, tl.y, tl.z, gs);
+        v[0] = compute_tile_b<S, BYT, RY, PASS, SP>(P, C, Ar, R, tl.rep, sigma, sm, tl.x0, tl.y0, gs);
 #pragma unroll
         for (int q = 1; q < NV; ++q) v[q] = gs[q - 1];
         if (A.tile_e) {
@@ -266,6 +292,15 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_batch(const __grid_constant_
             }
         }
     }
+}
+
+// sigma of every replica at its current temperature: the expression and the thermal
+// condition of the single-lattice coefficients
+__global__ void k_batch_sigma(const BatchRep* reps, int nrep, int thermal, double alpha, double dt, double* sigma) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nrep) return;
+    const double kT = reps[r].kT;
+    sigma[r] = thermal && (kT * alpha > 1e-10) && (kT > 1e-8) ? sqrt(alpha * kT * kHbar / dt) : 0.0;
 }
 
 // per-replica energies: tile partials summed in tile order, one block per replica
@@ -450,7 +485,14 @@ struct BatchLauncher {
     static constexpr int TY = G::TY;
     template <int PASS, int SP>
     static mj_status launch(const StencilParams& P, const DynCoef& C, const BatchArgs& A, int nblocks, cudaStream_t s) {
-        k_batch<S, BYT, RY, MINB, PASS, SP><<<nblocks, dim3(32, BYT), G::buf_bytes, s>>>(P, C, A);
+        auto kern = k_batch<S, BYT, RY, MINB, PASS, SP>;
+        constexpr size_t smem = 2 * G::buf_stride;
+        if (smem > 48 * 1024) {
+            const mj_status st = cuda_status(
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "k_batch");
+            if (st != MJ_OK) return st;
+        }
+        kern<<<nblocks, dim3(32, BYT), smem, s>>>(P, C, A);
         return cuda_status(cudaGetLastError(), "k_batch");
     }
     // the axial form where it holds; the plain field pass in the full form
@@ -515,7 +557,7 @@ struct mj_batch {
     int shape = 0;
     // the register-capped 32 x 8 tiles, as many persistent blocks as are resident
     // (4, 16, 64, 256 replicas of 32^2 to 256^2, us per step at variants 0 / 3 / 4,
-    // 8 blocks per SM: 18.6 / 14.5 / 14.5, 32.7 / 26.7 / 26.8, 100 / 76 / 80, 356 / 252 / 266)
+    // 8 blocks per SM: 14.8 / 14.7 / 14.5, 27.0 / 25.0 / 27.1, 82 / 73 / 78, 282 / 239 / 244)
     int variant = 3;
     int blocks_per_sm = 8;
     bool zaxial = false;              // every replica's Zeeman field along z
@@ -532,7 +574,8 @@ struct mj_batch {
     double* d_slot_kT = nullptr;
     double* d_noise_tab = nullptr;
     mj::BatchRep* d_reps = nullptr;
-    int4* d_tiles = nullptr;
+    mj::BatchTile* d_tiles = nullptr;
+    double* d_sigma = nullptr;        // per replica, of the current call's alpha and timestep
     int* d_image = nullptr;
     int* d_accept = nullptr;
     uint32_t* d_stepctr = nullptr;
@@ -569,6 +612,7 @@ void batch_free(mj_batch* b) {
     cudaFree(b->d_noise_tab);
     cudaFree(b->d_reps);
     cudaFree(b->d_tiles);
+    cudaFree(b->d_sigma);
     cudaFree(b->d_image);
     cudaFree(b->d_accept);
     cudaFree(b->d_stepctr);
@@ -587,12 +631,12 @@ void batch_free(mj_batch* b) {
 // (re)build the tile list for the current variant and upload the replica table
 mj_status batch_tiles(mj_batch* b, bool upload_reps) {
     const int ty = kBatchTY[b->variant];
-    std::vector<int4> tiles;
+    std::vector<BatchTile> tiles;
     for (int r = 0; r < b->nrep; ++r) {
         BatchRep& R = b->reps[r];
         R.tile0 = static_cast<int>(tiles.size());
         for (int y0 = 0; y0 < R.Ly; y0 += ty)
-            for (int x0 = 0; x0 < R.Lx; x0 += 32) tiles.push_back(make_int4(r, x0, y0, 0));
+            for (int x0 = 0; x0 < R.Lx; x0 += 32) tiles.push_back(BatchTile{R.off, R.Lx, R.Ly, x0, y0, r, 0});
         R.ntiles = static_cast<int>(tiles.size()) - R.tile0;
     }
     b->ntile = static_cast<int>(tiles.size());
@@ -603,10 +647,10 @@ mj_status batch_tiles(mj_batch* b, bool upload_reps) {
     b->d_tile_e = nullptr;
     b->d_tile_g = nullptr;
     mj_status st;
-    if ((st = cuda_status(cudaMalloc(&b->d_tiles, sizeof(int4) * tiles.size()), "batch tiles")) != MJ_OK) return st;
+    if ((st = cuda_status(cudaMalloc(&b->d_tiles, sizeof(BatchTile) * tiles.size()), "batch tiles")) != MJ_OK) return st;
     if ((st = cuda_status(cudaMalloc(&b->d_tile_e, sizeof(double) * tiles.size()), "batch tile energies")) != MJ_OK)
         return st;
-    if ((st = cuda_status(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice),
+    if ((st = cuda_status(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(BatchTile) * tiles.size(), cudaMemcpyHostToDevice),
                           "batch tiles")) != MJ_OK)
         return st;
     if (upload_reps)
@@ -656,10 +700,11 @@ int batch_blocks(const mj_batch* b) {
     return std::max(1, std::min(b->ntile, b->num_sms * b->blocks_per_sm));
 }
 
-BatchArgs batch_args(mj_batch* b, uint32_t step, double dt) {
+BatchArgs batch_args(mj_batch* b, uint32_t step) {
     BatchArgs A;
     A.reps = b->d_reps;
     A.tiles = b->d_tiles;
+    A.sigma = b->d_sigma;
     A.ntile = b->ntile;
     A.Ntot = b->Ntot;
     A.ms = b->d_m;
@@ -668,7 +713,6 @@ BatchArgs batch_args(mj_batch* b, uint32_t step, double dt) {
     A.aux = b->d_aux;
     A.tile_e = nullptr;
     A.step = step;
-    A.dt = dt;
     A.project = 0;
     A.tile_g = nullptr;
     A.gneb_n = 0;
@@ -678,7 +722,7 @@ BatchArgs batch_args(mj_batch* b, uint32_t step, double dt) {
 }
 
 mj_status batch_energy(mj_batch* b, const DynCoef& c, double* E, cudaStream_t s) {
-    BatchArgs A = batch_args(b, 0, 0.0);
+    BatchArgs A = batch_args(b, 0);
     A.tile_e = b->d_tile_e;
     mj_status st = batch_pass(b->shape, b->variant, BPASS_ENERGY, b->zaxial, b->sp, c, A, batch_blocks(b), s);
     if (st != MJ_OK) return st;
@@ -693,9 +737,14 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
     if (graph_mode) c.step_base = b->d_stepctr;
     mj_status st;
     const int nb = batch_blocks(b);
+    auto sigmas = [&]() -> mj_status {
+        k_batch_sigma<<<(b->nrep + 127) / 128, 128, 0, s>>>(b->d_reps, b->nrep, c.thermal, c.alpha, dt, b->d_sigma);
+        return cuda_status(cudaGetLastError(), "k_batch_sigma");
+    };
+    if (nsteps > 0 && (st = sigmas()) != MJ_OK) return st;
     for (int32_t k = 0; k < nsteps; ++k) {
         const uint32_t step = step0 + static_cast<uint32_t>(k);
-        BatchArgs A = batch_args(b, step, dt);
+        BatchArgs A = batch_args(b, step);
         if ((st = batch_pass(b->shape, b->variant, BPASS_SIB1, b->zaxial, b->sp, c, A, nb, s)) != MJ_OK) return st;
         A.ms = b->d_mid;
         A.out = b->d_m;
@@ -708,6 +757,7 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
             k_pt_swap<<<1, 256, 0, s>>>(b->d_reps, b->d_image, b->d_slot_kT, b->nrep, b->d_E, c, round,
                                         static_cast<uint32_t>(swap_every), b->d_accept);
             if ((st = cuda_status(cudaGetLastError(), "k_pt_swap")) != MJ_OK) return st;
+            if (k + 1 < nsteps && (st = sigmas()) != MJ_OK) return st;
         }
     }
     if (E_out) return batch_energy(b, c, E_out, s);
@@ -724,7 +774,7 @@ struct BatchFields {
     DynCoef c;       // unused by the field passes (no dynamics)
 
     mj_status field(double* F, double* m, double* E) {
-        BatchArgs A = batch_args(b, 0, 0.0);
+        BatchArgs A = batch_args(b, 0);
         A.ms = A.mn = m;
         A.out = F;
         A.project = 1;
@@ -735,7 +785,7 @@ struct BatchFields {
         return cuda_status(cudaGetLastError(), "k_batch_energy");
     }
     mj_status iterate(double* F, double* m, double* E, double* img, const GnebCtl* ctl) {
-        BatchArgs A = batch_args(b, 0, 0.0);
+        BatchArgs A = batch_args(b, 0);
         A.ms = A.mn = m;
         A.out = F;
         A.tile_e = b->d_tile_e;
@@ -838,6 +888,7 @@ mj_status mj_batch_create(const mj_lattice_desc* cell, const mj_hamiltonian_desc
         (st = dal(&b->d_slot_kT, sizeof(double) * nrep, "batch ladder")) != MJ_OK ||
         (st = dal(&b->d_noise_tab, sizeof(double) * kNoiseTabDoubles, "batch tables")) != MJ_OK ||
         (st = dal(&b->d_reps, sizeof(BatchRep) * nrep, "batch table")) != MJ_OK ||
+        (st = dal(&b->d_sigma, sizeof(double) * nrep, "batch sigma")) != MJ_OK ||
         (st = dal(&b->d_image, sizeof(int) * nrep, "batch image")) != MJ_OK ||
         (st = dal(&b->d_accept, sizeof(int) * nrep, "batch accept")) != MJ_OK ||
         (st = dal(&b->d_stepctr, sizeof(uint32_t) * 4, "batch step counter")) != MJ_OK) {
@@ -1008,7 +1059,7 @@ mj_status mj_batch_field(mj_batch* b, double* B_dev, double* E_dev, int32_t proj
     DynCoef c;
     std::memset(&c, 0, sizeof(c));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    BatchArgs A = batch_args(b, 0, 0.0);
+    BatchArgs A = batch_args(b, 0);
     A.out = B_dev;
     A.project = project ? 1 : 0;
     A.tile_e = b->d_tile_e;
