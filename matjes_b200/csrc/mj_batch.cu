@@ -194,21 +194,7 @@ __device__ __forceinline__ double compute_tile_b(const StencilParams& P, const D
                     const bool up = rep + 1 < A.gneb_nimg, down = rep > 0;
                     const double3 mp = up ? ld3(A.ms, i + A.gneb_n, Nt) : m0;
                     const double3 mm = down ? ld3(A.ms, i - A.gneb_n, Nt) : m0;
-                    double3 u = make_double3(mp.x - m0.x, mp.y - m0.y, mp.z - m0.z);
-                    double3 w = make_double3(m0.x - mm.x, m0.y - mm.y, m0.z - mm.z);
-                    const double du = dot(u, m0), dw = dot(w, m0);
-                    u = make_double3(u.x - du * m0.x, u.y - du * m0.y, u.z - du * m0.z);
-                    w = make_double3(w.x - dw * m0.x, w.y - dw * m0.y, w.z - dw * m0.z);
-                    gs[0] += dot(u, u);
-                    gs[1] += dot(u, w);
-                    gs[2] += dot(w, w);
-                    gs[3] += dot(Bv, u);
-                    gs[4] += dot(Bv, w);
-                    if (up) {
-                        const double3 c = cross(m0, mp);
-                        const double l = atan2(sqrt(dot(c, c)), dot(m0, mp));
-                        gs[5] += l * l;
-                    }
+                    gneb_path_terms(m0, mp, mm, up, Bv, gs);
                 }
             } else if constexpr (PASS == BPASS_SIB1) {
                 e += total_energy_part(f, m0, zero);
@@ -451,31 +437,21 @@ __global__ void __launch_bounds__(256) k_batch_magnet(const BatchRep* reps, cons
 // pass (BPASS_GNEB, the path sums per tile) and k_gneb_img.
 
 // Per image r (one block each): the energy and the six path sums of the GNEB
-// field pass, each summed over the image's tiles in tile order as
-// k_batch_energy sums the energies (thread t the tiles t, t + 256, ...; then
-// those partials in thread order, the all-zero ones beyond the image's tile
-// count left out), into E[r] and img[q nrep + r]; the seven sums side by side.
-__global__ void __launch_bounds__(256) k_gneb_img(const BatchRep* reps, int nrep, const double* __restrict__ tile_e,
-                                                  const double* __restrict__ tile_g, int ntile, double* E,
-                                                  double* img, const GnebCtl* ctl) {
+// field pass over the image's tiles, one warp per quantity in a fixed order
+// (tiles lane, lane + 32, ..., then the lanes), into E[r] and img[q nrep + r].
+__global__ void __launch_bounds__(7 * 32) k_gneb_img(const BatchRep* reps, int nrep, const double* __restrict__ tile_e,
+                                                     const double* __restrict__ tile_g, int ntile, double* E,
+                                                     double* img, const GnebCtl* ctl) {
     if (ctl->done) return;
-    const int r = blockIdx.x;
-    __shared__ double part[7][256];
-    const BatchRep R = reps[r];
-    for (int q = 0; q < 7; ++q) {
-        const double* src = q == 0 ? tile_e : tile_g + static_cast<int64_t>(q - 1) * ntile;
-        double s = 0.0;
-        for (int t = threadIdx.x; t < R.ntiles; t += blockDim.x) s += src[R.tile0 + t];
-        part[q][threadIdx.x] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x < 7) {
-        const int q = threadIdx.x;
-        const int nk = min(R.ntiles, static_cast<int>(blockDim.x));
-        double tot = 0.0;
-        for (int k = 0; k < nk; ++k) tot += part[q][k];
-        if (q == 0) E[r] = tot;
-        else img[(q - 1) * nrep + r] = tot;
+    const int r = blockIdx.x, lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const int t0 = reps[r].tile0, nt = reps[r].ntiles;
+    const double* src = q == 0 ? tile_e : tile_g + static_cast<int64_t>(q - 1) * ntile;
+    double s = 0.0;
+    for (int t = lane; t < nt; t += 32) s += src[t0 + t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        if (q == 0) E[r] = s;
+        else img[(q - 1) * nrep + r] = s;
     }
 }
 
@@ -795,7 +771,7 @@ struct BatchFields {
         A.stop = &ctl->done;
         mj_status e = batch_pass(b->shape, b->variant, BPASS_GNEB, b->zaxial, b->sp, c, A, batch_blocks(b), s);
         if (e != MJ_OK) return e;
-        k_gneb_img<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, tile_g, b->ntile, E, img, ctl);
+        k_gneb_img<<<b->nrep, 7 * 32, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, tile_g, b->ntile, E, img, ctl);
         return cuda_status(cudaGetLastError(), "k_gneb_img");
     }
 };

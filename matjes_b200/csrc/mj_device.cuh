@@ -387,13 +387,39 @@ __device__ void grid_reduce(double (&v)[NV], double* partials, unsigned int* cou
 }
 
 // ---------------------------------------------------------------------------
+// Squared angle between two unit vectors from u2 = |a - b|^2 = 4 sin^2(angle/2):
+// 4 arcsin^2(x) = 4 sum_n a_n x^2n at x^2 = u2 / 4, a_1 = 1, a_{n+1} = a_n 2 n^2 /
+// ((n + 1)(2n + 1)) (the series of arcsin^2; 18 terms to x^2 = 1/8, angles up to
+// 0.72: truncation below 1e-17 relative), atan2(|a x b|, a.b) beyond.  A third of
+// atan2's and the square root's instructions.
+struct Asin2Series {
+    double a[18];
+    constexpr Asin2Series() : a{} {
+        a[0] = 1.0;
+        for (int n = 1; n < 18; ++n) a[n] = a[n - 1] * (2.0 * n * n) / ((n + 1.0) * (2.0 * n + 1.0));
+    }
+};
+__device__ __forceinline__ double unit_angle2(double u2, double3 a, double3 b) {
+    const double x2 = 0.25 * u2;
+    if (x2 < 0.125) {
+        constexpr Asin2Series S;
+        double s = S.a[17];
+#pragma unroll
+        for (int n = 16; n >= 0; --n) s = fma(s, x2, S.a[n]);
+        return u2 * s;
+    }
+    const double3 c = cross(a, b);
+    const double l = atan2(sqrt(dot(c, c)), dot(a, b));
+    return l * l;
+}
+
 // The six GNEB path sums of one site (GNEB/tangent.f90, gneb_utils.f90):
 // A = P(m_{r+1} - m), B = P(m - m_{r-1}) (zero at the ends), |A|^2, A.B, |B|^2,
-// F.A, F.B, squared angle to image r + 1.  The same arithmetic as the batch's
-// GNEB field pass.
+// F.A, F.B, squared angle to image r + 1.
 __device__ __forceinline__ void gneb_path_terms(double3 m0, double3 mp, double3 mm, bool up, double3 F, double (&g)[6]) {
     double3 u = make_double3(mp.x - m0.x, mp.y - m0.y, mp.z - m0.z);
     double3 w = make_double3(m0.x - mm.x, m0.y - mm.y, m0.z - mm.z);
+    const double u2 = dot(u, u);
     const double du = dot(u, m0), dw = dot(w, m0);
     u = make_double3(u.x - du * m0.x, u.y - du * m0.y, u.z - du * m0.z);
     w = make_double3(w.x - dw * m0.x, w.y - dw * m0.y, w.z - dw * m0.z);
@@ -402,11 +428,7 @@ __device__ __forceinline__ void gneb_path_terms(double3 m0, double3 mp, double3 
     g[2] += dot(w, w);
     g[3] += dot(F, u);
     g[4] += dot(F, w);
-    if (up) {
-        const double3 c = cross(m0, mp);
-        const double l = atan2(sqrt(dot(c, c)), dot(m0, mp));
-        g[5] += l * l;
-    }
+    if (up) g[5] += unit_angle2(u2, m0, mp);
 }
 
 }  // namespace mj

@@ -127,13 +127,6 @@ __global__ void __launch_bounds__(256) k_gneb_scale(double* __restrict__ tau, Gn
     tau[2 * X.cs + i] *= inv;
 }
 
-__device__ __forceinline__ double3 gneb_rotate(double3 v, double3 a, double sn, double cs) {
-    // utilities/rotation.f90 rotate_vector_arr: v cos + sin (v x a) + (1 - cos)(a.v) a
-    const double t = dot(a, v);
-    return make_double3(v.x * cs + sn * (a.z * v.y - a.y * v.z) + (1.0 - cs) * t * a.x,
-                        v.y * cs + sn * (a.x * v.z - a.z * v.x) + (1.0 - cs) * t * a.y,
-                        v.z * cs + sn * (a.y * v.x - a.x * v.y) + (1.0 - cs) * t * a.z);
-}
 __device__ __forceinline__ double gneb_ang(double3 a, double3 b) {
     const double3 c = cross(a, b);
     return atan2(sqrt(dot(c, c)), dot(a, b));
@@ -340,7 +333,9 @@ __global__ void __launch_bounds__(256) k_gneb_sums(const double* __restrict__ m,
 // order, takes max |F|, sets lam = v.F / F.F (0 when v.F < 0; the velocity
 // projection, v = lam F), counts the iteration and sets the stop flag.  r =
 // blockIdx.x: the images of one site range run side by side, so the
-// neighbouring images' spins come from L2.
+// neighbouring images' spins come from L2.  Bound by FP64 instructions and the
+// seven arrays it reads: 256^2 x 16 images 26 us, 33 with the axis, the force and
+// the sine each normalised by a square root and divisions.
 template <int SPT>
 __global__ void __launch_bounds__(256, 4) k_gneb_step(const double* __restrict__ m, const double* __restrict__ mo,
                                                    const double* __restrict__ Fo, double* Fn,
@@ -352,23 +347,34 @@ __global__ void __launch_bounds__(256, 4) k_gneb_step(const double* __restrict__
     const int r = blockIdx.x;
     const int nb = gridDim.x * gridDim.y, bid = blockIdx.x + gridDim.x * blockIdx.y;
     const bool inner = r > 0 && r < nrep - 1;
-    double wp = 0.0, wm = 0.0, inv = 0.0, a = 0.0, k = 0.0;
-    if (inner) {
+    // the image's scalars, once per block
+    __shared__ double img_s[5];
+    if (inner && threadIdx.x == 0) {
+        double wp, wm;
         gneb_weights(E, r, nrep, 0, wp, wm);
         const double t2 = wp * wp * img[r] + 2.0 * wp * wm * img[nrep + r] + wm * wm * img[2 * nrep + r];
-        inv = t2 > 0.0 ? 1.0 / sqrt(t2) : 0.0;
-        a = (wp * img[3 * nrep + r] + wm * img[4 * nrep + r]) * inv;
-        k = spring * (sqrt(img[5 * nrep + r]) - sqrt(img[5 * nrep + r - 1]));
-        if (climb) {
-            __shared__ int ci_s;
-            if (threadIdx.x == 0) ci_s = gneb_maxloc(E, nrep);
-            __syncthreads();
-            if (ci_s == r) {
-                // the climbing image: F - 2 tau (F.tau), no spring
-                a *= 2.0;
-                k = 0.0;
-            }
+        const double inv = t2 > 0.0 ? 1.0 / sqrt(t2) : 0.0;
+        double a = (wp * img[3 * nrep + r] + wm * img[4 * nrep + r]) * inv;
+        double k = spring * (sqrt(img[5 * nrep + r]) - sqrt(img[5 * nrep + r - 1]));
+        if (climb && gneb_maxloc(E, nrep) == r) {
+            // the climbing image: F - 2 tau (F.tau), no spring
+            a *= 2.0;
+            k = 0.0;
         }
+        img_s[0] = wp;
+        img_s[1] = wm;
+        img_s[2] = inv;
+        img_s[3] = a;
+        img_s[4] = k;
+    }
+    __syncthreads();
+    double wp = 0.0, wm = 0.0, inv = 0.0, a = 0.0, k = 0.0;
+    if (inner) {
+        wp = img_s[0];
+        wm = img_s[1];
+        inv = img_s[2];
+        a = img_s[3];
+        k = img_s[4];
     }
     const double h = 0.5 / mass * dt, lam = scal[3];
     double v2[2] = {0.0, 0.0}, fm = 0.0;
@@ -384,17 +390,18 @@ __global__ void __launch_bounds__(256, 4) k_gneb_step(const double* __restrict__
             const double3 t = make_double3(t0.x * inv, t0.y * inv, t0.z * inv);
             const double3 g = ld3(Fn, i, X.cs);
             f = make_double3(g.x - t.x * a + k * t.x, g.y - t.y * a + k * t.y, g.z - t.z * a + k * t.z);
-            // the move's rotation: axis mo x Fo/|Fo| (rotation_axis_arr), angle
-            // between mo and m (sin |m x mo|, cos m.mo)
+            // the move's rotation (rotation_axis_arr, rotate_vector_arr): axis e = c/|c|,
+            // c = mo x Fo (unnormalised where it vanishes), angle between mo and m (sine
+            // |m x mo|, cosine m.mo); R Fo = cos Fo + sin Fo x e, e being normal to Fo.
+            // sin/|c| = |d|/|c| = d^2 / sqrt(d^2 c^2): one rsqrt where the axis, the
+            // force and the sine each took a square root and divisions
             const double3 m1 = ld3(mo, i, X.cs), fo = ld3(Fo, i, X.cs);
-            double3 fn = fo;
-            const double nf = sqrt(dot(fo, fo));
-            if (nf > 1e-30) fn = make_double3(fo.x / nf, fo.y / nf, fo.z / nf);
-            double3 e = cross(m1, fn);
-            const double ne = sqrt(dot(e, e));
-            if (ne > 2.220446049250313e-16) e = make_double3(e.x / ne, e.y / ne, e.z / ne);
-            const double3 c = cross(m0, m1);
-            const double3 fr = gneb_rotate(fo, e, sqrt(dot(c, c)), dot(m0, m1));
+            const double3 c = cross(m1, fo), d = cross(m0, m1);
+            const double c2 = dot(c, c), f2 = dot(fo, fo), d2 = dot(d, d), cs = dot(m0, m1);
+            const double n2 = f2 > 1e-60 ? (c2 > 4.930380657631324e-32 * f2 ? c2 : f2) : 1.0;
+            const double sn = d2 > 1e-200 ? d2 * rsqrt(d2 * n2) : 0.0;  // (no underflow: n2 > 1e-92)
+            const double3 x = cross(fo, c);
+            const double3 fr = make_double3(fma(sn, x.x, cs * fo.x), fma(sn, x.y, cs * fo.y), fma(sn, x.z, cs * fo.z));
             v = make_double3(lam * fr.x + (fr.x + f.x) * h, lam * fr.y + (fr.y + f.y) * h,
                              lam * fr.z + (fr.z + f.z) * h);
         }
@@ -461,8 +468,9 @@ __global__ void __launch_bounds__(256) k_gneb_move(const double* __restrict__ m,
     const double3 f = ld3(F, i, X.cs);
     const double c = scal[3] * dt + 0.5 / mass * dt * dt;
     double3 v = make_double3(m0.x + f.x * c, m0.y + f.y * c, m0.z + f.z * c);
-    const double nr = sqrt(dot(v, v));
-    if (nr > 1e-30) v = make_double3(v.x / nr, v.y / nr, v.z / nr);
+    const double n2 = dot(v, v);
+    const double nr = n2 > 1e-60 ? rsqrt(n2) : 1.0;
+    v = make_double3(v.x * nr, v.y * nr, v.z * nr);
     st3(mn, i, X.cs, v);
 }
 
