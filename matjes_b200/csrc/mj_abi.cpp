@@ -638,32 +638,31 @@ mj_status striped_enqueue(mj_plan* p, double* m_host, double* m_mapped, const Dy
     const int TY = kTiledVariantTY[p->tile_variant];
     const int ry = stencil_reach_y(p);
     const bool per_y = p->sp.periodic[1] != 0;
-    // passes of the step: (pass id, stencil input, own-site m_n, output, aux, aux2, energy partials)
+    // passes of the step: (pass id, stencil input, own-site m_n, output, aux, energy partials)
     struct Pass {
         int id;
         const double* ms;
         const double* mn;
         double* out;
         double* aux;
-        double* aux2;
         bool energy;
     };
     double* m = p->d_tmp_m;
     double* result = m;
     std::vector<Pass> passes;
     if (c.integrator == MJ_EULER) {
-        passes.push_back({1, m, nullptr, p->d_mid, nullptr, nullptr, E_wanted && before});
+        passes.push_back({1, m, nullptr, p->d_mid, nullptr, E_wanted && before});
         result = p->d_mid;
     } else if (c.integrator == MJ_HEUN_MATJES) {
-        passes.push_back({2, m, nullptr, p->d_mid, p->d_aux, p->d_aux2, E_wanted && before});
-        passes.push_back({3, p->d_mid, nullptr, m, p->d_aux, p->d_aux2, false});
+        passes.push_back({2, m, nullptr, p->d_mid, p->d_aux, E_wanted && before});
+        passes.push_back({3, p->d_mid, nullptr, m, p->d_aux, false});
     } else {
         double* bstore = (c.thermal && c.noise == MJ_NOISE_PHILOX && p->store_draw) ? p->d_aux : nullptr;
-        passes.push_back({4, m, nullptr, p->d_mid, bstore, nullptr, E_wanted && before});
-        passes.push_back({5, p->d_mid, m, m, bstore, nullptr, false});
+        passes.push_back({4, m, nullptr, p->d_mid, bstore, E_wanted && before});
+        passes.push_back({5, p->d_mid, m, m, bstore, false});
     }
     const int r = static_cast<int>(passes.size()) - 1;  // the pass that writes `result`
-    if (E_wanted && !before) passes.push_back({0, result, nullptr, nullptr, nullptr, nullptr, true});
+    if (E_wanted && !before) passes.push_back({0, result, nullptr, nullptr, nullptr, true});
     const int Q = static_cast<int>(passes.size());
     // stripe k: tile rows [t[k], t[k + 1])
     std::vector<int> t(K + 1);
@@ -726,7 +725,7 @@ mj_status striped_enqueue(mj_plan* p, double* m_host, double* m_mapped, const Dy
             const int n = ranges(q, k, rg);
             for (int i = 0; i < n; ++i) {
                 if (rg[i][1] <= rg[i][0]) continue;
-                st = launch_tiled(p, P.id, c, P.ms, P.mn, P.out, P.aux, P.aux2, DipView{}, nullptr, 0u, sc,
+                st = launch_tiled(p, P.id, c, P.ms, P.mn, P.out, P.aux, DipView{}, nullptr, 0u, sc,
                                   P.energy ? 1 : 0, rg[i][0], rg[i][1] - rg[i][0]);
                 if (st != MJ_OK) return st;
             }

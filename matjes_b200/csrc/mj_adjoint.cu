@@ -980,7 +980,7 @@ double* ckpt(const mj_adjoint* a, int k) { return a->d_ckpt + static_cast<int64_
 // recomputed in the second stage.
 void stage1(mj_plan* plan, const DynCoef& c, uint32_t step, const double* m, double* mb, cudaStream_t s) {
     if (plan->sp.shape != 0) {
-        launch_tiled(plan, 4, c, m, nullptr, mb, nullptr, nullptr, DipView{nullptr, 0, 0, 0}, nullptr, step, s);
+        launch_tiled(plan, 4, c, m, nullptr, mb, nullptr, DipView{nullptr, 0, 0, 0}, nullptr, step, s);
         return;
     }
     k_adj_f1<<<adj_grid(plan->sp), dim3(kABX, kABY), 0, s>>>(plan->sp, c, step, plan->d_bmap, m, mb);
@@ -988,7 +988,7 @@ void stage1(mj_plan* plan, const DynCoef& c, uint32_t step, const double* m, dou
 void stage2(mj_plan* plan, const DynCoef& c, uint32_t step, const double* m, const double* mb, double* out,
             cudaStream_t s) {
     if (plan->sp.shape != 0) {
-        launch_tiled(plan, 5, c, mb, m, out, nullptr, nullptr, DipView{nullptr, 0, 0, 0}, nullptr, step, s);
+        launch_tiled(plan, 5, c, mb, m, out, nullptr, DipView{nullptr, 0, 0, 0}, nullptr, step, s);
         return;
     }
     k_adj_f2<<<adj_grid(plan->sp), dim3(kABX, kABY), 0, s>>>(plan->sp, c, step, plan->d_bmap, m, mb, out);

@@ -271,6 +271,17 @@ __device__ __forceinline__ double3 llg_rhs(double3 B, double3 m, double alpha, d
     return make_double3(-o.x * inv_den, -o.y * inv_den, -o.z * inv_den);
 }
 
+// What the Heun predictor leaves to the corrector of its slope D1 and its thermal
+// slope DT: D1/2 + DT, so that the corrector's m~ + (D1/2 + D2/2 + DT) dt/hbar
+// (dynamics/spindynamics.f90:282-313) reads one vector per site, not two.
+__device__ __forceinline__ double3 heun_kept(double3 D1, bool thermal, double3 DT) {
+    if (!thermal) return make_double3(0.5 * D1.x, 0.5 * D1.y, 0.5 * D1.z);
+    return make_double3(fma(0.5, D1.x, DT.x), fma(0.5, D1.y, DT.y), fma(0.5, D1.z, DT.z));
+}
+__device__ __forceinline__ double3 heun_slope(double3 kept, double3 D2) {
+    return make_double3(fma(0.5, D2.x, kept.x), fma(0.5, D2.y, kept.y), fma(0.5, D2.z, kept.z));
+}
+
 // Projection onto the old norm (solvers/solver.f90:113-116), |t| > 1e-8 guard.
 __device__ __forceinline__ double3 project(double3 t, double3 m) {
     const double nt2 = dot_f(t, t);

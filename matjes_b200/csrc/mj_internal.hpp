@@ -183,8 +183,8 @@ struct mj_plan {
     void* dip = nullptr;             // DipolarPlan (mj_dipolar.cu)
     // scratch
     double* d_mid = nullptr;         // 3N
-    double* d_aux = nullptr;         // 3N (Heun D1)
-    double* d_aux2 = nullptr;        // 3N (Heun DT)
+    double* d_aux = nullptr;         // 3N (Heun: the predictor's D1/2 + DT; SIB: its draw)
+    double* d_aux2 = nullptr;        // 3N (minimisation velocities)
     double* d_field = nullptr;       // 3N (field scratch)
     double* d_partials = nullptr;    // per-block energy partials
     unsigned int* d_counter = nullptr;
@@ -294,7 +294,7 @@ constexpr int kTiledVariantBYT[kTiledVariants] = {4, 8, 8, 4, 8, 4};     // warp
 // [ty0, ty0 + nty) (plain staging; block ids and energy partials those of the
 // whole-lattice launch, so emode 1 over all row ranges writes the same partials).
 mj_status launch_tiled(mj_plan* p, int pass, const DynCoef& C, const double* ms, const double* mn, double* out,
-                       double* aux, double* aux2, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
+                       double* aux, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
                        int emode = 0, int ty0 = 0, int nty = -1);
 // Many steps in one launch (mj_steps_impl.cuh): `job` null only asks whether the
 // plan's lattice fits (`fits`); else runs it, with *warps energy partials per slot.
@@ -329,7 +329,7 @@ MJ_STEPS_SHAPE_DECL(launch_steps_tri_nn)
 MJ_STEPS_SHAPE_DECL(launch_steps_tri3)
 #define MJ_TILED_SHAPE_DECL(fn)                                                                                   \
     mj_status fn(mj_plan* p, int pass, const DynCoef& C, const double* ms, const double* mn, double* out,         \
-                 double* aux, double* aux2, DipView Hd, double* E_out, uint32_t step, cudaStream_t s, int emode,  \
+                 double* aux, DipView Hd, double* E_out, uint32_t step, cudaStream_t s, int emode,  \
                  int ty0, int nty);
 // one SIB step in one launch (k_sib_fused): tiled plans without the dipolar term
 mj_status launch_sib_fused(mj_plan* p, const DynCoef& C, double* m, double* draw, double* E_out, uint32_t step,

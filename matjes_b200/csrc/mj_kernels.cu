@@ -382,12 +382,11 @@ __global__ void __launch_bounds__(256) k_euler(const __grid_constant__ F fp, con
     }
 }
 
-// Heun-Matjes pass 1: predictor m~ = P(m + D1 h/hbar); keeps D1 and DT for pass 2.
+// Heun-Matjes pass 1: predictor m~ = P(m + D1 h/hbar); keeps D1/2 + DT for pass 2.
 template <class F>
 __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                                const double* __restrict__ m, double* __restrict__ mid,
-                                               double* __restrict__ D1, double* __restrict__ DTo,
-                                               const DipView Hd, Reduce R, const DipPad pad) {
+                                               double* __restrict__ kept, const DipView Hd, Reduce R, const DipPad pad) {
     int64_t i;
     int x, y, z;
     fp.begin();
@@ -405,8 +404,8 @@ __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, con
         const double3 mt = project(t, m0);
         st3(mid, i, N, mt);
         if (pad.p) st_pad(pad, x, y, z, mt);
-        st3(D1, i, N, D);
-        if (C.thermal) st3(DTo, i, N, llg_rhs(thermal_field(C, step, i, N), m0, C.alpha, C.inv_den));
+        st3(kept, i, N,
+            heun_kept(D, C.thermal, C.thermal ? llg_rhs(thermal_field(C, step, i, N), m0, C.alpha, C.inv_den) : D));
     }
     reduce_part(R, e);
 }
@@ -414,8 +413,8 @@ __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, con
 // Heun-Matjes pass 2: corrector restarted from the predictor.
 template <class F>
 __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, const DynCoef C,
-                                               const double* __restrict__ mid, const double* __restrict__ D1,
-                                               const double* __restrict__ DTi, double* __restrict__ mout,
+                                               const double* __restrict__ mid, const double* __restrict__ kept,
+                                               double* __restrict__ mout,
                                                const DipView Hd, Reduce R, int* status, const DipPad pad) {
     int64_t i;
     int x, y, z;
@@ -427,14 +426,7 @@ __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, con
     const FieldOut f = fp.field(mid, i, x, y, z, mt);
     const double3 hd = Hd.h ? ld_dip(Hd, x, y, z) : make_double3(0.0, 0.0, 0.0);
     const double3 D2 = llg_rhs(minus2(f.B, hd), mt, C.alpha, C.inv_den);
-    const double3 d1 = ld3(D1, i, N);
-    const double3 Di = make_double3(0.5 * d1.x + 0.5 * D2.x, 0.5 * d1.y + 0.5 * D2.y, 0.5 * d1.z + 0.5 * D2.z);
-    const double c = C.h_over_hbar;
-    double3 t = advance(mt, Di, c);
-    if (C.thermal) {
-        const double3 DT = ld3(DTi, i, N);
-        t = advance(t, DT, c);
-    }
+    const double3 t = advance(mt, heun_slope(ld3(kept, i, N), D2), C.h_over_hbar);
     const double3 mo = project(t, mt);
     flag_nonfinite(status, mo);
     st3(mout, i, N, mo);
@@ -706,12 +698,12 @@ mj_status step_impl(mj_plan* p, const Launch<F>& L, double* m, double* m_out, co
         case MJ_HEUN_MATJES: {
             DipView Hd = dip_field(p, m, s, st);
             if (st != MJ_OK) return st;
-            MJ_LAUNCH("k_heun1", k_heun1<F>, L.fp, c, step, m, p->d_mid, p->d_aux, p->d_aux2, Hd, make_reduce(p, E_prev),
+            MJ_LAUNCH("k_heun1", k_heun1<F>, L.fp, c, step, m, p->d_mid, p->d_aux, Hd, make_reduce(p, E_prev),
                       pd);
             if (pd.p) p->dip_pad_holds = p->d_mid;
             Hd = dip_field(p, p->d_mid, s, st);
             if (st != MJ_OK) return st;
-            MJ_LAUNCH("k_heun2", k_heun2<F>, L.fp, c, p->d_mid, p->d_aux, p->d_aux2, m, Hd, make_reduce(p, E_prev),
+            MJ_LAUNCH("k_heun2", k_heun2<F>, L.fp, c, p->d_mid, p->d_aux, m, Hd, make_reduce(p, E_prev),
                       p->d_status, pd);
             if (pd.p) p->dip_pad_holds = m;
             return MJ_OK;
@@ -813,10 +805,10 @@ namespace {
 bool tiled(const mj_plan* p) { return p->is_stencil && p->sp.shape != 0; }
 
 mj_status tiled_call(mj_plan* p, const char* name, int pass, const DynCoef& c, const double* ms, const double* mn,
-                     double* out, double* aux, double* aux2, DipView Hd, double* E, uint32_t step, cudaStream_t s,
+                     double* out, double* aux, DipView Hd, double* E, uint32_t step, cudaStream_t s,
                      int emode = 0) {
     const int rec = prof_begin(p, name, s);
-    mj_status st = launch_tiled(p, pass, c, ms, mn, out, aux, aux2, Hd, E, step, s, emode);
+    mj_status st = launch_tiled(p, pass, c, ms, mn, out, aux, Hd, E, step, s, emode);
     prof_end(p, rec, s);
     return st;
 }
@@ -826,7 +818,7 @@ mj_status tiled_field(mj_plan* p, const double* m, double* B, double* e_site, do
     DipView Hd = dip_field(p, m, s, st);
     if (st != MJ_OK) return st;
     DynCoef c{};
-    return tiled_call(p, "k_field", 0, c, m, nullptr, B, e_site, nullptr, Hd, E_out, 0u, s);
+    return tiled_call(p, "k_field", 0, c, m, nullptr, B, e_site, Hd, E_out, 0u, s);
 }
 
 mj_status tiled_step(mj_plan* p, double* m, double* m_out, const DynCoef& c, uint32_t step, double* E_prev,
@@ -836,16 +828,16 @@ mj_status tiled_step(mj_plan* p, double* m, double* m_out, const DynCoef& c, uin
     if (st != MJ_OK) return st;
     switch (c.integrator) {
         case MJ_EULER:
-            return tiled_call(p, "k_euler", 1, c, m, nullptr, m_out, nullptr, nullptr, Hd, E_prev, step, s);
+            return tiled_call(p, "k_euler", 1, c, m, nullptr, m_out, nullptr, Hd, E_prev, step, s);
         // two-pass schemes: pass 1 writes per-block energy partials, the first block
         // of pass 2 sums them (no ticket or last-block tail in pass 1)
         case MJ_HEUN_MATJES:
-            if ((st = tiled_call(p, "k_heun1", 2, c, m, nullptr, p->d_mid, p->d_aux, p->d_aux2, Hd, nullptr, step, s,
+            if ((st = tiled_call(p, "k_heun1", 2, c, m, nullptr, p->d_mid, p->d_aux, Hd, nullptr, step, s,
                                  E_prev ? 1 : 0)) != MJ_OK)
                 return st;
             Hd = dip_field(p, p->d_mid, s, st);
             if (st != MJ_OK) return st;
-            return tiled_call(p, "k_heun2", 3, c, p->d_mid, nullptr, m, p->d_aux, p->d_aux2, Hd, E_prev, step, s,
+            return tiled_call(p, "k_heun2", 3, c, p->d_mid, nullptr, m, p->d_aux, Hd, E_prev, step, s,
                               E_prev ? 2 : 0);
         case MJ_SIB: {
             // Philox draws are made once per step in pass 1 and kept for the corrector
@@ -856,12 +848,12 @@ mj_status tiled_step(mj_plan* p, double* m, double* m_out, const DynCoef& c, uin
                 prof_end(p, rec, s);
                 return st;
             }
-            if ((st = tiled_call(p, "k_sib1", 4, c, m, nullptr, p->d_mid, bstore, nullptr, Hd, nullptr, step, s,
+            if ((st = tiled_call(p, "k_sib1", 4, c, m, nullptr, p->d_mid, bstore, Hd, nullptr, step, s,
                                  E_prev ? 1 : 0)) != MJ_OK)
                 return st;
             Hd = dip_field(p, p->d_mid, s, st);
             if (st != MJ_OK) return st;
-            return tiled_call(p, "k_sib2", 5, c, p->d_mid, m, m, bstore, nullptr, Hd, E_prev, step, s, E_prev ? 2 : 0);
+            return tiled_call(p, "k_sib2", 5, c, p->d_mid, m, m, bstore, Hd, E_prev, step, s, E_prev ? 2 : 0);
         }
         default:
             return set_error(MJ_ERR_ARG, "unknown integrator");

@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
             publish(static_cast<unsigned int>(last && !(k & 1) ? k + 2 : k + 1));
             continue;
         }
-        double3 d1[RY], dt[RY];  // Heun: the predictor's slope and the thermal one
+        double3 kept[RY];  // Heun: what the corrector needs of the predictor's slopes
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
             if constexpr (INTEG == MJ_SIB) {
@@ -300,10 +300,9 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
                 if (C.thermal) H = make_double3(H.x + pre[r].b.x, H.y + pre[r].b.y, H.z + pre[r].b.z);
                 v[r] = sib_solve<true>(mn[r], mn[r], H, C.alpha, C.sib_hc);
             } else {
-                d1[r] = llg_rhs(B[r], mn[r], C.alpha, C.inv_den);
-                const double c = C.h_over_hbar;
-                v[r] = project(advance(mn[r], d1[r], c), mn[r]);
-                if (C.thermal) dt[r] = llg_rhs(pre[r].b, mn[r], C.alpha, C.inv_den);
+                const double3 D = llg_rhs(B[r], mn[r], C.alpha, C.inv_den);
+                v[r] = project(advance(mn[r], D, C.h_over_hbar), mn[r]);
+                kept[r] = heun_kept(D, C.thermal, C.thermal ? llg_rhs(pre[r].b, mn[r], C.alpha, C.inv_den) : D);
             }
         }
         __syncthreads();  // the tile has been read
@@ -320,12 +319,8 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
                 if (C.thermal) H = make_double3(H.x + pre[r].b.x, H.y + pre[r].b.y, H.z + pre[r].b.z);
                 mn[r] = sib_solve(mn[r], v[r], H, C.alpha, C.sib_hc);
             } else {
-                const double3 d2 = llg_rhs(B[r], v[r], C.alpha, C.inv_den);
-                const double3 di = make_double3(0.5 * d1[r].x + 0.5 * d2.x, 0.5 * d1[r].y + 0.5 * d2.y,
-                                                0.5 * d1[r].z + 0.5 * d2.z);
-                const double c = C.h_over_hbar;
-                double3 t = advance(v[r], di, c);
-                if (C.thermal) t = advance(t, dt[r], c);
+                const double3 D2 = llg_rhs(B[r], v[r], C.alpha, C.inv_den);
+                const double3 t = advance(v[r], heun_slope(kept[r], D2), C.h_over_hbar);
                 mn[r] = project(t, v[r]);
             }
             if (x < Lx && yt + r < Ly) flag_nonfinite(A.status, mn[r]);

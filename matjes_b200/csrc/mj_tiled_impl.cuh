@@ -62,8 +62,7 @@ struct TiledArgs {
     const double* ms;   // spins the stencil runs on (m, or the midpoint in pass 2)
     const double* mn;   // m_n (own site) for the SIB corrector
     double* out;        // field B / next state / midpoint
-    double* aux;        // Heun D1, SIB Philox draw, or per-site energy (field pass)
-    double* aux2;       // Heun DT
+    double* aux;        // Heun D1/2 + DT, SIB Philox draw, or per-site energy (field pass)
     const double* bmap; // per-cell applied field (SoA) or null
     DipView Hd;
     TReduce R;
@@ -177,8 +176,8 @@ __device__ __forceinline__ double ldg_or_cg(const double* p) {
 // per-site epilogue inputs that live in global memory, loaded before the
 // stencil so that their latency overlaps it
 struct Pre {
-    double3 a;  // SIB2: m_n;  HEUN2: D1
-    double3 b;  // SIB2: stored Philox draw;  HEUN2: DT
+    double3 a;  // SIB2: m_n;  HEUN2: the predictor's D1/2 + DT
+    double3 b;  // SIB2: stored Philox draw
 };
 
 // The thermal draw of the passes that make one (Euler, Heun predictor, SIB
@@ -197,7 +196,6 @@ __device__ __forceinline__ Pre prefetch(const DynCoef& C, const TiledArgs& A, in
                         : thermal_field(C, A.step, i, N);
     } else if constexpr (PASS == PASS_HEUN2) {
         p.a = ld3(A.aux, i, N);
-        if (C.thermal) p.b = ld3(A.aux2, i, N);
     } else if constexpr (PASS == PASS_SIB1 || PASS == PASS_EULER || PASS == PASS_HEUN1) {
         if (C.thermal) p.b = thermal_field(C, A.step, i, N);
     }
@@ -251,19 +249,11 @@ __device__ __forceinline__ double epilogue(const DynCoef& C, const TiledArgs& A,
         const double c = C.h_over_hbar;
         const double3 t = advance(m0, D, c);
         st3(A.out, i, N, project(t, m0));
-        st3(A.aux, i, N, D);
-        if (C.thermal) st3(A.aux2, i, N, llg_rhs(pre.b, m0, C.alpha, C.inv_den));
+        st3(A.aux, i, N, heun_kept(D, C.thermal, C.thermal ? llg_rhs(pre.b, m0, C.alpha, C.inv_den) : D));
         return energy_part<HD, ZAX>(Brs, Bzee, m0, hd);
     } else if constexpr (PASS == PASS_HEUN2) {
         const double3 D2 = llg_rhs(B, m0, C.alpha, C.inv_den);
-        const double3 d1 = pre.a;
-        const double3 Di = make_double3(0.5 * d1.x + 0.5 * D2.x, 0.5 * d1.y + 0.5 * D2.y, 0.5 * d1.z + 0.5 * D2.z);
-        const double c = C.h_over_hbar;
-        double3 t = advance(m0, Di, c);
-        if (C.thermal) {
-            const double3 DT = pre.b;
-            t = advance(t, DT, c);
-        }
+        const double3 t = advance(m0, heun_slope(pre.a, D2), C.h_over_hbar);
         const double3 mo = project(t, m0);
         flag_nonfinite(A.status, mo);
         st3(A.out, i, N, mo);
@@ -1086,7 +1076,7 @@ bool make_map_images(CUtensorMap* map, const double* base, const StencilParams& 
 // the build parallel).  pass: 0 field, 1 euler, 2 heun1, 3 heun2, 4 sib1, 5 sib2
 template <class S>
 mj_status launch_tiled_shape(mj_plan* p, int pass, const DynCoef& C, const double* ms, const double* mn, double* out,
-                             double* aux, double* aux2, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
+                             double* aux, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
                              int emode, int ty0, int nty) {
     TiledArgs A;
     std::memset(&A, 0, sizeof(A));
@@ -1094,7 +1084,6 @@ mj_status launch_tiled_shape(mj_plan* p, int pass, const DynCoef& C, const doubl
     A.mn = mn;
     A.out = out;
     A.aux = aux;
-    A.aux2 = aux2;
     A.bmap = p->d_bmap;
     A.Hd = Hd;
     A.R.partials = p->d_partials;

@@ -3,9 +3,9 @@
 
 namespace mj {
 mj_status launch_tiled_square2(mj_plan* p, int pass, const DynCoef& C, const double* ms, const double* mn, double* out,
-                         double* aux, double* aux2, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
+                         double* aux, DipView Hd, double* E_out, uint32_t step, cudaStream_t s,
                          int emode, int ty0, int nty) {
-    return launch_tiled_shape<ShapeSquare2>(p, pass, C, ms, mn, out, aux, aux2, Hd, E_out, step, s, emode, ty0, nty);
+    return launch_tiled_shape<ShapeSquare2>(p, pass, C, ms, mn, out, aux, Hd, E_out, step, s, emode, ty0, nty);
 }
 mj_status launch_sib_fused_square2(mj_plan* p, const DynCoef& C, double* m, double* draw, double* E_out, uint32_t step,
                          cudaStream_t s) {
