@@ -178,9 +178,10 @@ mj_status mj_plan_set_fused(mj_plan* plan, int32_t enable);
  *                              launch asks for enough shared memory), so that
  *                              the tiles of a lattice fill the last wave of
  *                              the GPU better;
- *   MJ_OPT_DIP_ZCONV (default 1)  FFT dipolar term with a z grid of a power
- *                              of two up to 32: the z transforms and the
- *                              product with K_F as one kernel (0: cuFFT z
+ *   MJ_OPT_DIP_ZCONV (default 1)  FFT dipolar term with up to 16 lattice
+ *                              planes, or a z grid of a power of two up to 32:
+ *                              the z part as one kernel, a direct sum or
+ *                              transforms with the product (0: cuFFT z
  *                              transforms and a separate product);
  *   MJ_OPT_HOST_ZEROCOPY (default 1)  striped mj_step_host with a mapped pinned
  *                              buffer: kernels write the stepped spins into it

@@ -21,8 +21,14 @@
 // product is kept whenever they exceed 1e-13.  The unpack is fused into the consumers: the field and
 // step kernels read H on the padded (y, x) grid of the lattice planes.
 //
-// When N_rep,z is a power of two up to 32 the z transforms and the pointwise
-// product are one kernel (k_zconv): one warp per (ky, kx) column, lane = z,
+// With few lattice planes (kZdirMax) the z part is not transformed at all: k_zdirect
+// sums H_z = sum_z' K(ky, kx, z - z') M_z' over the planes for every (ky, kx)
+// column, with K transformed along y and x only.  It serves every N_rep,z, reads
+// and writes the Lz planes alone, and for an open z axis uses the mirror symmetry
+// of K (K_xz and K_yz odd in z, the others even) to read half of K.
+//
+// With more planes than that, when N_rep,z is a power of two up to 32, the z
+// transforms and the pointwise product are one kernel (k_zconv): one warp per (ky, kx) column, lane = z,
 // a radix-2 FFT across the lanes by shuffles (forward in decimation in
 // frequency, which leaves the spectrum in bit-reversed order, K_F stored per
 // column in that order, inverse in decimation in time back to natural order).
@@ -54,6 +60,9 @@ struct DipolarPlan {
     cufftDoubleComplex* d_kfc = nullptr;   // complex K_F when it is not real
     cufftHandle f2d = 0, fz = 0, b2d = 0;
     bool have_f2d = false, have_fz = false, have_b2d = false;
+    // the direct z sum: K transformed along y and x, [6][nz][y][kx]
+    int zdir = 0;                          // 0: not used, else 1 + its mode (ZdirMode)
+    cufftDoubleComplex* d_kd = nullptr;
     // the fused z convolution: K_F per column [pc][nz][6] (kz in bit-reversed
     // order), real or complex, and the twiddles exp(-2 pi i m / nz), m < nz / 2
     bool zconv = false;
@@ -243,6 +252,102 @@ __global__ void __launch_bounds__(256) k_zconv(const double2* __restrict__ in, d
     }
 }
 
+// H of the lattice planes by the sum over z (see the header).  A block takes 32
+// consecutive columns, one per lane; its NW warps share the planes' spectra in
+// shared memory, and warp w makes the planes z = w, w + NW, ... (ZPT of them): per
+// distance dz one load of K's six components serves the pairs (z, z - dz) and
+// (z, z + dz) of all of them, the next distance's K in flight meanwhile (holding
+// a block's K in shared memory instead measured slower, 16.7 against 14.9 us at
+// 16 planes of 128 x 65 columns).  Bound by FP64 (36 fma a pair, Lz^2 pairs a
+// column) and the shared memory reads behind them.
+enum ZdirMode { kZdirMirror = 0, kZdirOpen = 1, kZdirCircular = 2 };
+// Planes it is taken for: up to 16, but up to 8 where k_zconv serves N_rep,z too.
+// us of a field call with this / with k_zconv: 8 planes of 64^2 33.8 / 35.9 and of
+// 128^2 42.1 / 43.9, but 16 planes of 32^2 37.8 / 35.9; with this / with the cuFFT
+// transforms and the separate product: 13 planes of 128^2 48.1 / 63.2 and of
+// 100 x 90 45.9 / 55.0, 6 planes of 64^2 33.8 / 42.2.
+constexpr int kZdirMax = 16, kZdirPow2Max = 8;
+
+struct KSix {
+    double2 xx, xy, xz, yy, yz, zz;
+};
+__device__ __forceinline__ KSix load_k6(const double2* __restrict__ k, int64_t stride) {
+    return KSix{__ldg(k),              __ldg(k + stride),     __ldg(k + 2 * stride),
+                __ldg(k + 3 * stride), __ldg(k + 4 * stride), __ldg(k + 5 * stride)};
+}
+__device__ __forceinline__ void cmac(double2& acc, double2 a, double2 b) {
+    acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+    acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void k6_mac(double2 (&h)[3], const KSix& K, double2 mx, double2 my, double2 mz) {
+    cmac(h[0], K.xx, mx);
+    cmac(h[1], K.xy, mx);
+    cmac(h[2], K.xz, mx);
+    cmac(h[0], K.xy, my);
+    cmac(h[1], K.yy, my);
+    cmac(h[2], K.yz, my);
+    cmac(h[0], K.xz, mz);
+    cmac(h[1], K.yz, mz);
+    cmac(h[2], K.zz, mz);
+}
+
+template <int NW, int ZPT, int MODE>
+__global__ void __launch_bounds__(32 * NW, 2) k_zdirect(const double2* __restrict__ in, double2* __restrict__ out,
+                                                        const double2* __restrict__ kd, int64_t pc, int lz, int nz) {
+    extern __shared__ double2 zs[];  // [lz][3][32]
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t col = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+    const bool act = col < pc;
+    for (int row = w; row < 3 * lz; row += NW)
+        zs[row * 32 + lane] = act ? in[static_cast<int64_t>(row) * pc + col] : make_double2(0.0, 0.0);
+    __syncthreads();
+    double2 h[ZPT][3];
+#pragma unroll
+    for (int q = 0; q < ZPT; ++q) h[q][0] = h[q][1] = h[q][2] = make_double2(0.0, 0.0);
+    const int64_t ks = static_cast<int64_t>(nz) * pc;  // component stride
+    const double2* k = kd + (act ? col : 0);
+    const int nd = MODE == kZdirCircular ? nz : lz;
+    KSix kp = load_k6(k, ks), km = kp;
+    auto pair = [&](double2 (&acc)[3], const KSix& K, int zp) {
+        const double2* m = zs + zp * 96 + lane;
+        k6_mac(acc, K, m[0], m[32], m[64]);
+    };
+    for (int dz = 0; dz < nd; ++dz) {
+        KSix np = kp, nm = km;
+        if (dz + 1 < nd) {
+            np = load_k6(k + static_cast<int64_t>(dz + 1) * pc, ks);
+            if constexpr (MODE == kZdirOpen) nm = load_k6(k + static_cast<int64_t>(nz - dz - 1) * pc, ks);
+        }
+        if constexpr (MODE == kZdirMirror) {
+            km = kp;
+            km.xz = make_double2(-kp.xz.x, -kp.xz.y);
+            km.yz = make_double2(-kp.yz.x, -kp.yz.y);
+        }
+#pragma unroll
+        for (int q = 0; q < ZPT; ++q) {
+            const int z = w + NW * q;
+            if (z >= lz) continue;
+            if constexpr (MODE == kZdirCircular) {
+                const int zp = z - dz;
+                pair(h[q], kp, zp < 0 ? zp + nz : zp);
+            } else {
+                if (z - dz >= 0) pair(h[q], kp, z - dz);
+                if (dz > 0 && z + dz < lz) pair(h[q], km, z + dz);
+            }
+        }
+        kp = np;
+        if constexpr (MODE == kZdirOpen) km = nm;
+    }
+    if (!act) return;
+#pragma unroll
+    for (int q = 0; q < ZPT; ++q) {
+        const int z = w + NW * q;
+        if (z >= lz) continue;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[(static_cast<int64_t>(z) * 3 + c) * pc + col] = h[q][c];
+    }
+}
+
 mj_status cufft_status(cufftResult r, const char* where) {
     if (r == CUFFT_SUCCESS) return MJ_OK;
     return set_error(MJ_ERR_CUDA, std::string("cuFFT error ") + std::to_string(static_cast<int>(r)) + " in " + where);
@@ -259,6 +364,7 @@ void free_plan(DipolarPlan* d) {
     cudaFree(d->d_cz);
     cudaFree(d->d_kfr);
     cudaFree(d->d_kfc);
+    cudaFree(d->d_kd);
     cudaFree(d->d_kzr);
     cudaFree(d->d_kzc);
     delete d;
@@ -272,6 +378,7 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
     d->lz = p->sp.L[2];
     const int nx = d->nrep[0], ny = d->nrep[1], nz = d->nrep[2];
     const int nkx = nx / 2 + 1;
+    const bool pow2 = nz >= 2 && nz <= 32 && (nz & (nz - 1)) == 0;  // k_zconv serves it
     d->pr = static_cast<int64_t>(ny) * nx;
     d->pc = static_cast<int64_t>(ny) * nkx;
     const int64_t nk = d->pr * nz, nkc = d->pc * nz;
@@ -308,6 +415,39 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
             return fail(st);
         }
         int dims[3] = {nz, ny, nx}, inembed[3] = {nz, ny, nx}, onembed[3] = {nz, ny, nkx};
+        if (d->lz <= kZdirPow2Max || (d->lz <= kZdirMax && !pow2)) {
+            // K along y and x only, for the direct z sum; its mirror symmetry in z
+            // checked value by value
+            bool mirror = nz >= 2 * d->lz;
+            for (int c = 0; c < 6 && mirror; ++c) {
+                const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
+                for (int z = 1; z < d->lz && mirror; ++z) {
+                    const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
+                    const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
+                    for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
+                }
+            }
+            d->zdir = 1 + (nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular);
+            cufftHandle p2;
+            cufftResult r2 = CUFFT_EXEC_FAILED;
+            if ((st = al(&d->d_kd, sizeof(cufftDoubleComplex) * 6 * nkc, "dipolar K planes")) == MJ_OK &&
+                cudaMemcpyAsync(d_k6, k6.data(), sizeof(double) * 6 * nk, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+                (r2 = cufftPlanMany(&p2, 2, dims + 1, inembed + 1, 1, static_cast<int>(d->pr), onembed + 1, 1,
+                                    static_cast<int>(d->pc), CUFFT_D2Z, 6 * nz)) == CUFFT_SUCCESS) {
+                cufftSetStream(p2, s);
+                r2 = cufftExecD2Z(p2, d_k6, d->d_kd);
+                if (r2 == CUFFT_SUCCESS)
+                    k_scale<<<static_cast<unsigned>((6 * nkc + 255) / 256), 256, 0, s>>>(d->d_kd, 6 * nkc,
+                                                                                         1.0 / static_cast<double>(d->pr));
+                cudaStreamSynchronize(s);
+                cufftDestroy(p2);
+            }
+            if (st != MJ_OK || r2 != CUFFT_SUCCESS) {
+                cudaFree(d_k6);
+                cudaFree(kf);
+                return fail(st != MJ_OK ? st : cufft_status(r2, "K plane transforms"));
+            }
+        }
         cufftHandle pk;
         cufftResult r = cudaMemcpyAsync(d_k6, k6.data(), sizeof(double) * 6 * nk, cudaMemcpyHostToDevice, s) == cudaSuccess
                             ? cufftPlanMany(&pk, 3, dims, inembed, 1, static_cast<int>(nk), onembed, 1,
@@ -342,7 +482,7 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
         }
         d->real_kf = im <= 1e-13 * re;
         // the fused z convolution's K_F: per column, kz in the lanes' bit-reversed order
-        if (nz >= 2 && nz <= 32 && (nz & (nz - 1)) == 0) {
+        if (d->zdir == 0 && pow2) {
             int bits = 0;
             while ((1 << bits) < nz) ++bits;
             auto bitrev = [&](int l) {
@@ -450,6 +590,32 @@ mj_status dipolar_apply(mj_plan* p, const double* m, double* /*H unused: consume
     if (d->have_fz) cufftSetStream(d->fz, s);
     // planes z < Lz of d_cx; the rest of it stays zero
     if ((st = cufft_status(cufftExecD2Z(d->f2d, d->d_pad, d->d_cx), "2D D2Z")) != MJ_OK) return st;
+    if (d->zdir && p->dip_zconv) {
+        const double2* in = reinterpret_cast<const double2*>(d->d_cx);
+        double2* out = reinterpret_cast<double2*>(d->d_cz);
+        const double2* kd = reinterpret_cast<const double2*>(d->d_kd);
+        const unsigned nb = static_cast<unsigned>((d->pc + 31) / 32);
+        const size_t smem = sizeof(double2) * 96 * d->lz;
+        const int nz = d->nrep[2];
+        auto go = [&](auto nw, auto zpt) {
+            constexpr int W = decltype(nw)::value, Z = decltype(zpt)::value;
+            auto run = [&](auto mode) {
+                k_zdirect<W, Z, decltype(mode)::value><<<nb, 32 * W, smem, s>>>(in, out, kd, d->pc, d->lz, nz);
+            };
+            switch (d->zdir - 1) {
+                case kZdirMirror: run(std::integral_constant<int, kZdirMirror>{}); break;
+                case kZdirOpen: run(std::integral_constant<int, kZdirOpen>{}); break;
+                default: run(std::integral_constant<int, kZdirCircular>{}); break;
+            }
+        };
+        using std::integral_constant;
+        if (d->lz <= 4) go(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+        else if (d->lz <= 8) go(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+        else go(integral_constant<int, 8>{}, integral_constant<int, 2>{});
+        st = cuda_status(cudaGetLastError(), "k_zdirect");
+        if (st != MJ_OK) return st;
+        return cufft_status(cufftExecZ2D(d->b2d, d->d_cz, d->d_h), "2D Z2D");
+    }
     if (d->zconv && p->dip_zconv) {
         // z transforms and product in one pass, into the planes z < Lz of d_cz
         ZTwiddle W;
