@@ -36,6 +36,7 @@ struct StencilField {
     const double* bmap;  // per-cell applied field, SoA (null = uniform)
 
     static constexpr int BX = 32, BY = 8;
+    static constexpr int kMinBlocks = 1;  // resident blocks asked of the compiler
     __device__ __forceinline__ void begin() const {}
     __device__ __forceinline__ int64_t nsites() const { return static_cast<int64_t>(P.L[0]) * P.L[1] * P.L[2]; }
     __device__ __forceinline__ bool site(int64_t& i, int& x, int& y, int& z) const {
@@ -109,8 +110,9 @@ struct StencilField {
 // neighbours are added in the order of the plan's offsets, so the field is the
 // offset loop's bit for bit.  Bound by instruction issue and the L2 (the
 // neighbouring rows and layers come from there).  96 x 96 x 97 periodic at 10 K:
-// a SIB step 48.6 us with the energy, 78.3 with the offset loop and a second draw
-// (passes 26.7 + 19.4 us against 41.9 + 31.8).
+// a SIB step 47.2 us with the energy, 78.3 with the offset loop and a second draw
+// (passes 25.6 + 17.9 us against 41.9 + 31.8).  Held to 48 registers for five
+// resident blocks: 47.5 us at the four that 58 allow.
 enum { CUBIC_FULL = 0, CUBIC_AXIAL = 1 };
 template <int SP>
 struct CubicField {
@@ -122,6 +124,7 @@ struct CubicField {
     const double* bmap;
 
     static constexpr int BX = StencilField::BX, BY = StencilField::BY;
+    static constexpr int kMinBlocks = 5;
     __device__ __forceinline__ void begin() const {}
     __device__ __forceinline__ int64_t nsites() const { return static_cast<int64_t>(L[0]) * L[1] * L[2]; }
     __device__ __forceinline__ bool site(int64_t& i, int& x, int& y, int& z) const {
@@ -134,24 +137,28 @@ struct CubicField {
     }
     __device__ __forceinline__ FieldOut field(const double* __restrict__ m, int64_t i, int x, int y, int z, double3 m0) const {
         const int64_t N = nsites();
-        const int64_t sx = 1, sy = L[0], sz = static_cast<int64_t>(L[0]) * L[1];
+        // 32-bit site indices (the launcher checks that N fits): one multiply-add per address
+        const int ii = static_cast<int>(i), sy = L[0], sz = L[0] * L[1];
+        const double* __restrict__ mx = m;
+        const double* __restrict__ my = m + N;
+        const double* __restrict__ mz = m + 2 * N;
         // neighbour indices (the site itself past an open edge, not used there)
-        int64_t j[6];
+        int j[6];
         bool in[6];
-        auto pair = [&](int q, int d, int v, int64_t stride) {
+        auto pair = [&](int q, int d, int v, int stride) {
             const int n = L[d];
             const bool up = v + 1 < n, dn = v > 0;
             in[q] = dn || periodic[d];
             in[q + 1] = up || periodic[d];
-            j[q] = dn ? i - stride : (periodic[d] ? i + stride * (n - 1) : i);
-            j[q + 1] = up ? i + stride : (periodic[d] ? i - stride * (n - 1) : i);
+            j[q] = dn ? ii - stride : (periodic[d] ? ii + stride * (n - 1) : ii);
+            j[q + 1] = up ? ii + stride : (periodic[d] ? ii - stride * (n - 1) : ii);
         };
         pair(0, 2, z, sz);
         pair(2, 1, y, sy);
-        pair(4, 0, x, sx);
+        pair(4, 0, x, 1);
         double3 a[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) a[k] = ld3(m, j[k], N);
+        for (int k = 0; k < 6; ++k) a[k] = make_double3(__ldg(mx + j[k]), __ldg(my + j[k]), __ldg(mz + j[k]));
         double bx = 0.0, by = 0.0, bz = 0.0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
@@ -207,6 +214,7 @@ struct EllSites {
     int zee_on;
 
     static constexpr int BX = 256, BY = 1;
+    static constexpr int kMinBlocks = 5;
     __device__ __forceinline__ int64_t nsites() const { return N; }
     __device__ __forceinline__ bool site(int64_t& i, int& x, int& y, int& z) const {
         i = blockIdx.x * static_cast<int64_t>(BX) + threadIdx.x;
@@ -256,7 +264,7 @@ struct EllField : EllSites {
 // (the lanes of a warp read at most one tensor per atom of the cell).
 // 384 x 384 cells of two atoms, 9 entries a site: a SIB step 38.9 us, 109.0 us
 // with the general form (passes 18.4 + 15.5 us against 56.7 + 42.3); 35.6 us since
-// the corrector reads the predictor's draw.
+// the corrector reads the predictor's draw, 33.6 at five resident blocks.
 struct EllIdField : EllSites {
     int wfull;             // slots of full tensors; the slots after them are isotropic
     int ntensor;
@@ -325,7 +333,7 @@ __device__ __forceinline__ double3 minus2(double3 B, double3 hd) {
 
 // ---------------------------------------------------------------------------
 template <class F>
-__global__ void __launch_bounds__(256) k_field(const __grid_constant__ F fp, const double* __restrict__ m,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_field(const __grid_constant__ F fp, const double* __restrict__ m,
                                                const DipView Hd, double* __restrict__ B,
                                                double* __restrict__ e_site, Reduce R) {
     int64_t i;
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(256) k_field(const __grid_constant__ F fp, con
 
 // Euler: one fused pass m -> mout.
 template <class F>
-__global__ void __launch_bounds__(256) k_euler(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_euler(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                                const double* __restrict__ m, double* __restrict__ mout,
                                                const DipView Hd, Reduce R, int* status, const DipPad pad) {
     int64_t i;
@@ -384,7 +392,7 @@ __global__ void __launch_bounds__(256) k_euler(const __grid_constant__ F fp, con
 
 // Heun-Matjes pass 1: predictor m~ = P(m + D1 h/hbar); keeps D1/2 + DT for pass 2.
 template <class F>
-__global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_heun1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                                const double* __restrict__ m, double* __restrict__ mid,
                                                double* __restrict__ kept, const DipView Hd, Reduce R, const DipPad pad) {
     int64_t i;
@@ -412,7 +420,7 @@ __global__ void __launch_bounds__(256) k_heun1(const __grid_constant__ F fp, con
 
 // Heun-Matjes pass 2: corrector restarted from the predictor.
 template <class F>
-__global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, const DynCoef C,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_heun2(const __grid_constant__ F fp, const DynCoef C,
                                                const double* __restrict__ mid, const double* __restrict__ kept,
                                                double* __restrict__ mout,
                                                const DipView Hd, Reduce R, int* status, const DipPad pad) {
@@ -437,7 +445,7 @@ __global__ void __launch_bounds__(256) k_heun2(const __grid_constant__ F fp, con
 // and, when given a buffer, its Philox draw for the corrector (48 bytes a site
 // written and read back cost less than drawing it again, about 240 instructions).
 template <class F>
-__global__ void __launch_bounds__(256) k_sib1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_sib1(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                               const double* __restrict__ m, double* __restrict__ mid,
                                               double* __restrict__ draw, const DipView Hd, Reduce R, const DipPad pad) {
     int64_t i;
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(256) k_sib1(const __grid_constant__ F fp, cons
 
 // SIB pass 2: corrector from m_n with A(midpoint); in place (only the own site of m is read).
 template <class F>
-__global__ void __launch_bounds__(256) k_sib2(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_sib2(const __grid_constant__ F fp, const DynCoef C, uint32_t step,
                                               const double* __restrict__ mid, double* m,
                                               const double* __restrict__ draw, const DipView Hd, Reduce R, int* status,
                                               const DipPad pad) {
@@ -493,7 +501,7 @@ __global__ void __launch_bounds__(256) k_sib2(const __grid_constant__ F fp, cons
 
 // Reference temperature estimator (dynamics/measure_temp.f90:21-43): sum |m x B|^2, sum m.B.
 template <class F>
-__global__ void __launch_bounds__(256) k_temperature(const __grid_constant__ F fp, const double* __restrict__ m,
+__global__ void __launch_bounds__(256, F::kMinBlocks) k_temperature(const __grid_constant__ F fp, const double* __restrict__ m,
                                                      const DipView Hd, Reduce R) {
     int64_t i;
     int x, y, z;
@@ -739,9 +747,9 @@ Launch<StencilField> stencil_launch(const mj_plan* p) {
 }
 // the six nearest neighbours of a simple-cubic lattice in the order that the
 // shells of such a cell give them
-bool is_cubic(const StencilParams& P) {
+bool is_cubic(const StencilParams& P, int64_t N) {
     static const int order[6][3] = {{0, 0, -1}, {0, 0, 1}, {0, -1, 0}, {0, 1, 0}, {-1, 0, 0}, {1, 0, 0}};
-    if (P.n_off != 6) return false;
+    if (P.n_off != 6 || N > 0x7fffffff) return false;
     for (int k = 0; k < 6; ++k)
         for (int d = 0; d < 3; ++d)
             if (P.off[k][d] != order[k][d]) return false;
@@ -777,7 +785,7 @@ Launch<CubicField<SP>> cubic_launch(const mj_plan* p) {
 // f(launch) with the launch of the plan's stencil
 template <class Fn>
 auto with_stencil(const mj_plan* p, Fn&& f) {
-    if (is_cubic(p->sp)) {
+    if (is_cubic(p->sp, p->N)) {
         if (cubic_axial(p->sp)) return f(cubic_launch<CUBIC_AXIAL>(p));
         return f(cubic_launch<CUBIC_FULL>(p));
     }
