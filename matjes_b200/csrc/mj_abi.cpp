@@ -337,10 +337,17 @@ mj_status ell_from_blocks(mj_plan* p, const Geometry& g, const std::vector<Block
 mj_status alloc_scratch(mj_plan* p) {
     const int64_t N = p->N;
     mj_status st;
-    if ((st = dalloc(&p->d_mid, 3 * N, "mid")) != MJ_OK) return st;
-    const int64_t aux = std::max<int64_t>(3 * N, kStepsAuxDoubles);
-    if ((st = dalloc(&p->d_aux, aux, "aux")) != MJ_OK) return st;
-    if ((st = dalloc(&p->d_aux2, aux, "aux2")) != MJ_OK) return st;
+    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
+    // launches of many steps use neither mid nor aux for spins: the tiles' boxes are
+    // in mid, the energy partials in aux
+    const int64_t tiles = steps_tiles(p), words = steps_box_words(p);
+    static_assert(sizeof(unsigned long long) == sizeof(double), "boxes in the midpoint buffer");
+    if ((st = dalloc(&p->d_mid, std::max(3 * N, words), "mid")) != MJ_OK) return st;
+    p->aux_doubles = std::max<int64_t>(3 * N, tiles > 0 ? kStepsAuxDoubles : 0);
+    if ((st = dalloc(&p->d_aux, p->aux_doubles, "aux")) != MJ_OK) return st;
+    if ((st = dalloc(&p->d_aux2, 3 * N, "aux2")) != MJ_OK) return st;
+    if (tiles > 0 && p->aux_doubles >= 2 * 8 * tiles)  // room for two slots of energies
+        p->d_steps_box = reinterpret_cast<unsigned long long*>(p->d_mid);
     // generic grid, or the smallest tile of the tiled kernels (32 x 8), whichever has more blocks
     const int64_t tiled_max = p->is_stencil ? static_cast<int64_t>((p->sp.L[0] + 31) / 32) * ((p->sp.L[1] + 7) / 8) * p->sp.L[2] : 0;
     p->partial_cap = 2 * std::max(energy_blocks(p), tiled_max) + 64;
@@ -353,14 +360,6 @@ mj_status alloc_scratch(mj_plan* p) {
         if ((st = cuda_status(cudaMemset(p->d_sched, 0, sizeof(unsigned int) * sched), "scheduler init")) != MJ_OK)
             return st;
     }
-    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
-    // launches of many steps use neither buffer for spins: the tile counters are in
-    // aux2, the energy partials in aux
-    p->aux_doubles = aux;
-    const int64_t words = p->is_stencil && p->sp.shape != 0 ? steps_flag_words(p) : 0;
-    if (words > 0 && words * static_cast<int64_t>(sizeof(unsigned int)) <= aux * static_cast<int64_t>(sizeof(double)) &&
-        aux >= 2 * 8 * (words / kStepsFlagStride))  // room for two slots of energies
-        p->d_steps_flags = reinterpret_cast<unsigned int*>(p->d_aux2);
     if ((st = dalloc(&p->d_scalar, 8, "scalar")) != MJ_OK) return st;
     if ((st = dalloc(&p->d_status, 4, "status")) != MJ_OK) return st;
     if ((st = cuda_status(cudaMemset(p->d_status, 0, 4 * sizeof(int)), "status init")) != MJ_OK) return st;
@@ -470,13 +469,13 @@ mj_status dyn_coef(const mj_dyn_params* d, const mj_plan* plan, DynCoef& c) {
 mj_status steps_together(mj_plan* p, double* m, const DynCoef& c, int energy_mode, uint32_t step0, int32_t nsteps,
                          double* E_dev, cudaStream_t s, bool& used) {
     used = false;
-    if (!p->steps_together || !p->d_steps_flags || !p->is_stencil || p->sp.shape == 0 || p->dip_on || p->fused_sib) return MJ_OK;
+    if (!p->steps_together || !p->d_steps_box || !p->is_stencil || p->sp.shape == 0 || p->dip_on || p->fused_sib) return MJ_OK;
     int warps = 0;
     mj_status st = launch_steps(p, nullptr, c, &warps, used, s);
     if (st != MJ_OK || !used) return st;
     const bool before = energy_mode == MJ_ENERGY_BEFORE;
     // energies of as many steps per launch as there is room for partials (a tile has at most eight warps)
-    const int64_t tiles = steps_flag_words(p) / kStepsFlagStride;
+    const int64_t tiles = std::max<int64_t>(1, steps_tiles(p));
     const int32_t slots_max = static_cast<int32_t>(std::min<int64_t>(kStepsSlots, p->aux_doubles / (8 * tiles)));
     const int32_t chunk = E_dev ? slots_max - 1 : 4096;
     for (int32_t k0 = 0; k0 < nsteps; k0 += chunk) {
@@ -484,11 +483,10 @@ mj_status steps_together(mj_plan* p, double* m, const DynCoef& c, int energy_mod
         const bool last = k0 + n == nsteps;
         StepsJob j;
         std::memset(&j, 0, sizeof(j));
-        j.m_in = j.m = j.m_out = m;
-        j.mid = p->d_mid;
+        j.m_in = j.m_out = m;
         j.nsteps = n;
         j.step0 = step0 + static_cast<uint32_t>(k0);
-        j.flags = p->d_steps_flags;
+        j.box = p->d_steps_box;
         int slots = 0;
         double* E = nullptr;
         if (E_dev) {
@@ -1132,7 +1130,7 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m, const mj_dyn_params* 
     // for its single steps and fields
     bool together = false;
     int warps = 0;
-    if (plan->steps_together && plan->d_steps_flags && plan->is_stencil && plan->sp.shape != 0 && !plan->dip_on)
+    if (plan->steps_together && plan->d_steps_box && plan->is_stencil && plan->sp.shape != 0 && !plan->dip_on)
         launch_steps(plan, nullptr, c, &warps, together, 0);
     const bool steps_together = plan->steps_together;
     plan->steps_together = false;

@@ -571,16 +571,16 @@ constexpr int kTBYT = 8, kTRY = 1;
 
 // The backward steps of a whole segment in one launch, on lattices whose tiles
 // are all resident at once: the scheme of mj_steps_impl.cuh (a block keeps its
-// tile, waits for its eight neighbours alone, cooperative launch, bounded
-// waits).  What a backward step hands to the neighbours is gH2, then gH1; dL/dm,
+// tile and exchanges edge values with its neighbours through the tiles' boxes,
+// cooperative launch, bounded waits).  What a backward step hands to the neighbours is gH2, then gH1; dL/dm,
 // the stage-2 gradients and the field gradient stay in the thread's registers,
 // and so do the thread's shares of the term gradients: kept in memory from one
 // segment to the next and reduced over the grid once, after the last (so the
 // sums do not depend on the checkpoint spacing).  m_n and mb of a step come from the recomputed segment, so
 // their tiles, the two fields and the draw are ready before the wait.
-// Bound by the chain of its two exchanges: 256^2 square, 3 terms, 8.6 us a step,
+// Bound by the chain of its two exchanges: 256^2 square, 3 terms, 7.5 us a step,
 // 21.6 us with the two launches (10.9 + 10.7); a forward and backward sweep of
-// 200 steps with checkpoints every 50 10.0 -> 4.6 ms.
+// 200 steps with checkpoints every 50 10.0 -> 3.4 ms.
 struct SegArgs {
     const double* g_in;  // dL/dm entering the segment's last step (or its part without W gH1)
     int with_gH1;        // 1: gH1 of the step after holds the missing part
@@ -589,13 +589,13 @@ struct SegArgs {
     const double* segb;  // mb of step k at + k n3
     int len;
     uint32_t step0;      // index of the segment's first step
-    double *gH1, *gH2, *mpart, *gb;
+    double *gH1, *mpart, *gb;
     double* acc;         // the threads' term gradients, [nterm][threads of the launch]
     int acc_in;          // 1: they hold the segments before
     int reduce;          // 1: the last segment, reduce them into R
     const double* bmap;
     const double* unit;
-    unsigned int* flags;
+    unsigned long long* box;
     int* status;
     AdjReduce R;
 };
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
     for (int q = tid; q < 9 * G::NS; q += 32 * kTBYT) smem_s[q] = 0.0;
     stage_units<S, kTBYT, kTRY>(A.unit, M, Us);
     TileRing<S, kTBYT, kTRY> ring;
-    ring.init(P, A.flags);
+    ring.init(P, A.box);
     auto put = [&](double* t, double3 v) {
         if (act[0]) {
             t[own] = v.x;
@@ -663,32 +663,25 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
         const double3 H2 = add3(apply(tB), zn), H1 = add3(apply(tC), zn);
         double3 g = part;
         if (more) {
-            if (pass > 0) {
-                if (!(ok = ring.wait(pass, A.status))) break;
-                ring.load(A.gH1, N, tA);
-                __syncthreads();
-            }
+            if (pass > 0 && !(ok = ring.fetch(pass, tA, A.status))) break;
             g = add3(part, apply(tA));
         }
         more = true;
         const SibGrad s2 = sib_vjp(m0, b0, H2, C.alpha, C.sib_hc, g);
+        ring.post(0, s2.gH, ++pass);
         __syncthreads();  // the tile of gH1 has been read
         put(tA, s2.gH);
-        if (act[0]) st3(A.gH2, i, N, s2.gH);
-        ring.publish(++pass);
         const double3 gh2[1] = {act[0] ? s2.gH : zero};
         if (M.nterm > 0) tiled_term_grads<S, kTBYT, kTRY>(Us, M, tB, base, gh2, act, acc);
-        if (!(ok = ring.wait(pass, A.status))) break;
-        ring.load(A.gH2, N, tA);
-        __syncthreads();
+        if (!(ok = ring.fetch(pass, tA, A.status))) break;
         const double3 gy1 = scl3(0.5, add3(s2.gp, apply(tA)));
         const SibGrad s1 = sib_vjp(m0, m0, H1, C.alpha, C.sib_hc, gy1);
         part = add3(add3(s2.gm, gy1), add3(s1.gm, s1.gp));
         if (P.zee_on) gbs = add3(gbs, scl3(P.zc, add3(s1.gH, s2.gH)));
+        ring.post(0, s1.gH, ++pass);
         __syncthreads();  // the tile of gH2 has been read
         put(tA, s1.gH);
-        if (act[0]) st3(A.gH1, i, N, s1.gH);
-        ring.publish(++pass);
+        if (act[0] && k == 0) st3(A.gH1, i, N, s1.gH);
         const double3 gh1[1] = {act[0] ? s1.gH : zero};
         if (M.nterm > 0) tiled_term_grads<S, kTBYT, kTRY>(Us, M, tC, base, gh1, act, acc);
         __syncthreads();  // the tiles of m_n and mb have been read
@@ -729,9 +722,9 @@ mj_status segment_shape(const mj_plan* plan, const DynCoef& c, const TermMasks& 
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_segment<S>, 32 * kTBYT, sm) == cudaSuccess &&
            static_cast<int64_t>(grid.x) * grid.y <= static_cast<int64_t>(per_sm) * plan->num_sms;
     if (!fits || !args) return MJ_OK;
-    mj_status st = cuda_status(cudaMemsetAsync(args->flags, 0,
-                                               sizeof(unsigned int) * kStepsFlagStride * grid.x * grid.y, s),
-                               "segment counters");
+    mj_status st = cuda_status(cudaMemsetAsync(args->box, 0,
+                                               sizeof(unsigned long long) * 12 * steps_box_sites(S::R) * grid.x * grid.y, s),
+                               "segment boxes");
     if (st != MJ_OK) return st;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -926,7 +919,7 @@ struct mj_adjoint {
     double* d_gterms = nullptr; // kMaxTerms
     double* d_gb = nullptr;     // 3N
     double* d_acc = nullptr;          // the threads' term gradients between segment launches
-    unsigned int* d_flags = nullptr;  // tile counters of the many-step launches (null: the lattice is too large)
+    unsigned long long* d_box = nullptr;  // the tiles' boxes of the many-step launches (null: the lattice is too large)
     // the two sweeps as CUDA graphs over the buffers above, cached with their key
     cudaStream_t cap = nullptr;
     cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
@@ -957,7 +950,7 @@ void adjoint_free(mj_adjoint* a) {
     cudaFree(a->d_partials);
     cudaFree(a->d_counter);
     cudaFree(a->d_slots);
-    cudaFree(a->d_flags);
+    cudaFree(a->d_box);
     cudaFree(a->d_acc);
     delete a;
 }
@@ -998,7 +991,7 @@ void stage2(mj_plan* plan, const DynCoef& c, uint32_t step, const double* m, con
 bool steps_fit(const mj_adjoint* a, const DynCoef& c, cudaStream_t s) {
     bool fits = false;
     int warps = 0;
-    if (a->d_flags && a->plan->steps_together && launch_steps(a->plan, nullptr, c, &warps, fits, s) != MJ_OK) fits = false;
+    if (a->d_box && a->plan->steps_together && launch_steps(a->plan, nullptr, c, &warps, fits, s) != MJ_OK) fits = false;
     return fits;
 }
 
@@ -1013,12 +1006,10 @@ void forward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, cudaStrea
             StepsJob j;
             std::memset(&j, 0, sizeof(j));
             j.m_in = ckpt(a, seg);
-            j.m = a->d_work;
-            j.mid = mid;
             j.m_out = ckpt(a, seg + 1);
             j.nsteps = std::min(E, a->nsteps - seg * E);
             j.step0 = step0 + static_cast<uint32_t>(seg * E);
-            j.flags = a->d_flags;
+            j.box = a->d_box;
             int warps = 0;
             bool fits = false;
             launch_steps(plan, &j, c, &warps, fits, s);
@@ -1049,7 +1040,7 @@ void backward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, bool wan
     bool first = true;
     const bool together = steps_fit(a, c, s);
     bool segments = false;  // the backward steps of a segment in one launch
-    if (a->d_flags && plan->steps_together && segment_launch(plan, c, M, nullptr, segments, s) != MJ_OK) segments = false;
+    if (a->d_box && plan->steps_together && segment_launch(plan, c, M, nullptr, segments, s) != MJ_OK) segments = false;
     for (int seg = a->nseg - 1; seg >= 0; --seg) {
         const int s0 = seg * E;
         const int len = std::min(E, a->nsteps - s0);
@@ -1067,7 +1058,7 @@ void backward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, bool wan
             j.nsteps = len;
             j.step0 = step0 + static_cast<uint32_t>(s0);
             j.half = 1;
-            j.flags = a->d_flags;
+            j.box = a->d_box;
             int warps = 0;
             bool fits = false;
             launch_steps(plan, &j, c, &warps, fits, s);
@@ -1088,12 +1079,11 @@ void backward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, bool wan
             g.len = len;
             g.step0 = step0 + static_cast<uint32_t>(s0);
             g.gH1 = a->d_gH1;
-            g.gH2 = a->d_gH2;
             g.mpart = a->d_mpart;
             g.gb = gb;
             g.bmap = plan->d_bmap;
             g.unit = plan->d_unit;
-            g.flags = a->d_flags;
+            g.box = a->d_box;
             g.status = plan->d_status;
             g.acc = a->d_acc;
             g.acc_in = first ? 0 : 1;
@@ -1298,9 +1288,9 @@ mj_status mj_adjoint_create(mj_plan* plan, int32_t nsteps, int32_t checkpoint_ev
         return st;
     }
     cudaMemset(a->d_counter, 0, sizeof(unsigned int) * 4);
-    const int64_t flags = steps_flag_words(plan);
+    const int64_t words = steps_box_words(plan);
     const size_t nacc = static_cast<size_t>(plan_nterm(plan)) * a->nblocks * (kABX * kABY);
-    if (flags > 0 && ((st = al(&a->d_flags, sizeof(unsigned int) * flags, "adjoint tile counters")) != MJ_OK ||
+    if (words > 0 && ((st = al(&a->d_box, sizeof(unsigned long long) * words, "adjoint tile boxes")) != MJ_OK ||
                       (nacc > 0 && (st = al(&a->d_acc, sizeof(double) * nacc, "adjoint term sums")) != MJ_OK))) {
         adjoint_free(a);
         return st;

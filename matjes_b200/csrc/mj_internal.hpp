@@ -114,9 +114,8 @@ void build_noise_tables(double* tab);
 }  // namespace mj
 
 namespace mj {
-// d_aux and d_aux2 hold at least this many doubles: the energy partials of eight
-// slots (8 warps per tile, as many tiles as are resident at one site per thread)
-// and the tile counters of a launch of many steps.
+// d_aux holds at least this many doubles: the energy partials of a launch of many
+// steps, up to 8 per tile and step.
 constexpr int64_t kStepsAuxDoubles = 32768;
 
 // The working memory of a GNEB relaxation (mj_gneb.cuh), kept by the plan or
@@ -155,8 +154,8 @@ struct mj_plan {
     bool store_draw = true;          // SIB: the predictor stores its Philox draw for the corrector (else recomputed)
     bool steps_together = true;             // many steps in one launch where the lattice fits (off once a
                                             // program picks a kernel variant)
-    unsigned int* d_steps_flags = nullptr;  // their tile counters, in d_aux2 (null: the lattice does not fit)
-    int64_t aux_doubles = 0;                // size of d_aux and of d_aux2
+    unsigned long long* d_steps_box = nullptr;  // their tiles' boxes, in d_mid (null: the lattice does not fit)
+    int64_t aux_doubles = 0;                    // size of d_aux
     unsigned int* d_sched = nullptr; // fused step scheduler: work counter, exit ticket, done tiles per row
     int num_sms = 148;
     int* d_status = nullptr;         // device status word: kStatusTimeout | kStatusNonFinite
@@ -299,13 +298,14 @@ mj_status launch_tiled(mj_plan* p, int pass, const DynCoef& C, const double* ms,
 // Many steps in one launch (mj_steps_impl.cuh): `job` null only asks whether the
 // plan's lattice fits (`fits`); else runs it, with *warps energy partials per slot.
 constexpr int kStepsTY = 8;          // tile height
-constexpr int kStepsFlagStride = 8;  // words between two tiles' counters
+// sites of a 32 x 8 tile within R of its edge: the places of its box (TileRing), 12 words each
+constexpr int steps_box_sites(int R) { return 64 * R + (kStepsTY - 2 * R) * 2 * R; }
 constexpr int kStepsSlots = 64;      // energies recorded per launch, at most
 struct StepsJob {
     const double* m_in;   // spins entering the first step
-    double* m;            // spins entering step k > 0 at m + k m_stride
+    double* m;            // spins entering step k > 0 stored at m + k m_stride (null: not stored)
     int64_t m_stride;
-    double* mid;          // midpoints at mid + k mid_stride (Euler: the other spin buffer, strides 0)
+    double* mid;          // midpoints at mid + k mid_stride (null: not stored)
     int64_t mid_stride;
     double* m_out;        // spins after the last step
     int nsteps;
@@ -314,13 +314,15 @@ struct StepsJob {
     double* partials;     // energy partials [slot][*warps], null = no energies
     int e_slot0;          // slot of the energy of the spins entering the first step, -1 = not recorded
     int e_final;          // record the energy after the last step too
-    unsigned int* flags;  // steps_flag_words(p) words of scratch
+    unsigned long long* box;  // steps_box_words(p) words of scratch
 };
 mj_status launch_steps(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s);
 // E[k] = the sum of slot k's n partials, k < slots
 mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, cudaStream_t s);
-// counter words of the plan's tiles, 0 when the lattice is too large for any configuration
-int64_t steps_flag_words(const mj_plan* p);
+// tiles of the plan's lattice, 0 when it has more than any configuration keeps resident
+// (or no tiled kernels); words of their boxes
+int64_t steps_tiles(const mj_plan* p);
+int64_t steps_box_words(const mj_plan* p);
 #define MJ_STEPS_SHAPE_DECL(fn) \
     mj_status fn(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s);
 MJ_STEPS_SHAPE_DECL(launch_steps_square_nn)

@@ -4,24 +4,29 @@
 // A small lattice's step is bound by its two dependent launches, not by its
 // arithmetic: 64^2 sites are 16 tiles on 148 SMs, and a launch with its ramp,
 // halo staging and last block takes 5 us of which the tile's own work is a
-// fraction.  Here every block keeps one 32 x 8 tile for the whole call: the
-// tile's spins stay in registers and shared memory, and a pass reads only the
-// halo cells from global memory.  Blocks synchronise with their eight
-// neighbouring tiles alone, through one counter per tile (the passes whose
-// results the tile has published): before a pass stages its halo it waits for
-// the counters of the neighbours, which also says that they have staged what
-// the tile is about to overwrite (the neighbourhood is symmetric), so spins and
-// midpoints are updated in place.  The thermal draw of a step is made before
-// the wait, and neither it nor m_n goes through memory between the passes.
-// The launch is cooperative, so all blocks run at once and every wait ends; the
-// waits are bounded all the same (kStatusTimeout).
+// fraction.  Here every block keeps one 32 x 8 tile for the whole call, its spins
+// in registers and shared memory, and a pass needs only the halo from outside.
+//
+// Exchange (TileRing): a tile posts its edge spins in a box of its own in global
+// memory, every 64-bit word half of a double and the pass number that wrote it; a
+// reader polls the words it needs until all carry the pass it waits for.  A word
+// is written and read whole, so data and flag arrive together: no fence, no
+// counter, one trip through the L2 (posting with a release, polling a counter
+// and then loading took three).  Boxes alternate between two halves by the
+// pass's parity: a tile posts pass p + 2 after it has read its neighbours' p + 1,
+// which they posted after reading p, so nothing is overwritten unread (whom a
+// tile reads also reads it).  The thermal draw of a step is made before the wait,
+// and neither it nor m_n goes through memory between the passes.  The launch is
+// cooperative, so all blocks run at once and every wait ends; the waits are
+// bounded all the same (kStatusTimeout).
 //
 // The arithmetic is the tiled passes' (mj_tiled_impl.cuh): the spins are the
 // same bit for bit.  us per SIB step at 10 K, this against two launches: square
-// 16^2 4.0 / 10.6, 64^2 4.9 / 10.8, 256^2 6.6 / 12.0, 512^2 11.1 / 15.8;
-// triangular, three shells, 64^2 5.8 / 12.3, 256^2 7.9 / 13.4, 512^2 13.4 / 18.7.
-// What bounds it: up to 256^2 the chain release - acquire - halo load - pass,
-// about 2.2 us a pass; at 512^2 instruction issue (42 ps per site and step).
+// 16^2 3.1 / 10.6, 64^2 3.2 / 10.3, 256^2 4.0 / 11.6, 512^2 10.3 / 15.5;
+// triangular, three shells, 64^2 3.7 / 12.6, 256^2 4.9 / 13.4, 512^2 12.2 / 18.3
+// (with a release, a counter and a load per exchange 4.9 at 64^2, 6.6 at 256^2).
+// What bounds it: up to 256^2 the chain post - poll - pass, 1.6 to 2 us a pass;
+// at 512^2 instruction issue (39 ps per site and step).
 #pragma once
 
 #include "mj_tiled_impl.cuh"
@@ -31,9 +36,9 @@ namespace {
 
 struct StepsArgs {
     const double* m_in;  // spins entering step 0
-    double* m;           // spins entering step k > 0: m + k m_stride (Euler: alternating with mid)
+    double* m;           // spins entering step k > 0 stored at m + k m_stride, unless null
     int64_t m_stride;
-    double* mid;         // midpoint of step k: mid + k mid_stride
+    double* mid;         // midpoint of step k stored at mid + k mid_stride, unless null
     int64_t mid_stride;
     double* m_out;       // spins after the last step
     const double* bmap;
@@ -44,28 +49,44 @@ struct StepsArgs {
     int half;            // the last step makes its predictor only
     int nsteps;
     uint32_t step0;
-    unsigned int* flags; // per tile (kStepsFlagStride apart): passes published, zero at the launch
+    unsigned long long* box;  // the tiles' boxes, zero at the launch
     int* status;
 };
 
 constexpr uint32_t kStepsWaitPolls = 1u << 20;
 
 // The halo of a block's tile (TileGeom layout; grid x, y over the tiles, z over
-// the layers) and the counters of its neighbours.
+// the layers) and the boxes its cells come from.  A tile's box: [parity][word][kN]
+// over the sites within R of the tile's edge (box_index), word 2 c and 2 c + 1
+// the low and high half of component c.
 template <class S, int BYT, int RY>
 struct TileRing {
     using G = TileGeom<S, BYT, RY>;
     static constexpr int R = G::R, NT = 32 * BYT;
     static constexpr int KH = ((G::TX + 2 * R) * (G::TY + 2 * R) - G::TX * G::TY + NT - 1) / NT;  // cells per thread
-    int hpos[KH], hsrc[KH];     // a halo cell's place in the tile, its site in the layer (-1: none, or past an open edge)
-    const unsigned int* nflag;  // threads 0 .. 7: the counter of one neighbouring tile each (null: none)
-    unsigned int* flag;         // the tile's own
+    static constexpr int kN = steps_box_sites(R);
+    static_assert(G::TX == 32 && G::TY == kStepsTY, "box_index");
+    int hpos[KH], hsrc[KH];  // a halo cell's place in the tile, its site in the layer (-1: none, or past an open edge)
+    int hbox[KH];            // its place in the boxes
+    int obox[RY];            // the thread's sites' places in the tile's box (-1: not near the edge)
+    unsigned long long* box;
 
-    __device__ __forceinline__ void init(const StencilParams& P, unsigned int* flags) {
+    // place of site (lx, ly) of a w x h tile in its box: the first R rows, the last R, then the sides; -1 inside
+    static __device__ __forceinline__ int box_index(int lx, int ly, int w, int h) {
+        if (ly < R) return ly * 32 + lx;
+        if (ly >= h - R) return (R + ly - (h - R)) * 32 + lx;
+        if (lx < R) return 64 * R + (ly - R) * 2 * R + lx;
+        if (lx >= w - R) return 64 * R + (ly - R) * 2 * R + R + lx - (w - R);
+        return -1;
+    }
+    __device__ __forceinline__ void init(const StencilParams& P, unsigned long long* boxes) {
         const int Lx = P.L[0], Ly = P.L[1];
         const int tid = threadIdx.x + 32 * threadIdx.y;
         const int x0 = blockIdx.x * G::TX, y0 = blockIdx.y * G::TY;
         const int w = min(G::TX, Lx - x0), h = min(G::TY, Ly - y0);
+        const int nx = gridDim.x, ny = gridDim.y, z = blockIdx.z;
+        auto base_of = [&](int tx, int ty) { return 12 * kN * (tx + nx * (ty + ny * z)); };
+        box = boxes;
         // the ring of width R about the tile's w x h sites: rows below and above, then the sides
         const int full = w + 2 * R;
 #pragma unroll
@@ -85,6 +106,7 @@ struct TileRing {
                 lx = lx < R ? lx - R : w + lx - R;
             }
             hsrc[q] = -1;
+            hbox[q] = 0;
             hpos[q] = (ly + R) * G::PX + lx + G::RX;
             if (c < 2 * R * (full + h)) {
                 int gx = x0 + lx, gy = y0 + ly;
@@ -93,32 +115,63 @@ struct TileRing {
                     if (outx) gx = ((gx % Lx) + Lx) % Lx;
                     if (outy) gy = ((gy % Ly) + Ly) % Ly;
                     hsrc[q] = gx + Lx * gy;
+                    const int tx = gx / G::TX, ty = gy / G::TY;
+                    hbox[q] = base_of(tx, ty) + box_index(gx - tx * G::TX, gy - ty * G::TY, min(G::TX, Lx - tx * G::TX),
+                                                          min(G::TY, Ly - ty * G::TY));
                 }
             }
         }
-        const int nx = gridDim.x, ny = gridDim.y, z = blockIdx.z;
-        auto of = [&](int tx, int ty) { return flags + static_cast<int64_t>(kStepsFlagStride) * (tx + nx * (ty + ny * z)); };
-        flag = of(blockIdx.x, blockIdx.y);
-        nflag = nullptr;
-        if (tid < 8) {
-            const int k = tid < 4 ? tid : tid + 1;
-            const int tx = static_cast<int>(blockIdx.x) + k % 3 - 1, ty = static_cast<int>(blockIdx.y) + k / 3 - 1;
-            const bool okx = P.periodic[0] || (tx >= 0 && tx < nx), oky = P.periodic[1] || (ty >= 0 && ty < ny);
-            if (okx && oky) nflag = of((tx + nx) % nx, (ty + ny) % ny);
+#pragma unroll
+        for (int r = 0; r < RY; ++r) {
+            const int lx = threadIdx.x, ly = threadIdx.y * RY + r;
+            const int b = lx < w && ly < h ? box_index(lx, ly, w, h) : -1;
+            obox[r] = b < 0 ? -1 : base_of(blockIdx.x, blockIdx.y) + b;
         }
     }
-    // until the neighbours have published `target` passes; false on a timeout (all threads of the block)
-    __device__ __forceinline__ bool wait(unsigned int target, int* status) const {
+    // the halo cells of a layer of `src` (component stride N) into the tile
+    __device__ __forceinline__ void load(const double* src, int64_t N, double* sm) const {
+#pragma unroll
+        for (int q = 0; q < KH; ++q)
+            if (hsrc[q] >= 0)
+                set(sm, hpos[q], make_double3(__ldcg(src + hsrc[q]), __ldcg(src + N + hsrc[q]), __ldcg(src + 2 * N + hsrc[q])));
+    }
+    // the vector v of the thread's site r as pass `pass` into the box
+    __device__ __forceinline__ void post(int r, double3 v, unsigned int pass) const {
+        if (obox[r] < 0) return;
+        unsigned long long* b = box + obox[r] + (pass & 1u) * (6 * kN);
+        const unsigned long long tag = static_cast<unsigned long long>(pass) << 32;
+        const double c[3] = {v.x, v.y, v.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            put_word(b + (2 * k) * kN, tag | static_cast<unsigned int>(__double2loint(c[k])));
+            put_word(b + (2 * k + 1) * kN, tag | static_cast<unsigned int>(__double2hiint(c[k])));
+        }
+    }
+    // the halo cells as the neighbours posted them in pass `pass` into the tile;
+    // false (all threads of the block, after a barrier) when a wait gave up
+    __device__ __forceinline__ bool fetch(unsigned int pass, double* sm, int* status) const {
         bool bad = false;
-        if (nflag) {
-            uint32_t it = 0;
-            while (ld_acquire_u32(nflag) < target) {
-                if (++it > kStepsWaitPolls) {
+#pragma unroll
+        for (int q = 0; q < KH; ++q) {
+            if (hsrc[q] < 0) continue;
+            const unsigned long long* b = box + hbox[q] + (pass & 1u) * (6 * kN);
+            unsigned long long u[6];
+            for (uint32_t it = 0;; ++it) {
+                bool ok = true;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) u[k] = get_word(b + k * kN);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) ok = ok && static_cast<unsigned int>(u[k] >> 32) == pass;
+                if (ok) break;
+                if (it > kStepsWaitPolls) {
                     bad = true;
                     break;
                 }
                 if (it > 4096) __nanosleep(64);
             }
+            auto half = [&](int k) { return static_cast<int>(static_cast<unsigned int>(u[k])); };
+            set(sm, hpos[q], make_double3(__hiloint2double(half(1), half(0)), __hiloint2double(half(3), half(2)),
+                                          __hiloint2double(half(5), half(4))));
         }
         if (__syncthreads_or(bad)) {
             if (threadIdx.x == 0 && threadIdx.y == 0 && status) atomicOr(status, kStatusTimeout);
@@ -126,22 +179,18 @@ struct TileRing {
         }
         return true;
     }
-    // the halo cells of a layer of `src` (component stride N) into the tile
-    __device__ __forceinline__ void load(const double* src, int64_t N, double* sm) const {
-#pragma unroll
-        for (int q = 0; q < KH; ++q)
-            if (hsrc[q] >= 0) {
-                const double vx = __ldcg(src + hsrc[q]), vy = __ldcg(src + N + hsrc[q]), vz = __ldcg(src + 2 * N + hsrc[q]);
-                sm[hpos[q]] = vx;
-                sm[G::NS + hpos[q]] = vy;
-                sm[2 * G::NS + hpos[q]] = vz;
-            }
+    static __device__ __forceinline__ void set(double* sm, int c, double3 v) {
+        sm[c] = v.x;
+        sm[G::NS + c] = v.y;
+        sm[2 * G::NS + c] = v.z;
     }
-    // after every thread's stores, which the release then covers
-    __device__ __forceinline__ void publish(unsigned int passes) const {
-        __syncthreads();
-        if (threadIdx.x == 0 && threadIdx.y == 0)
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(passes) : "memory");
+    static __device__ __forceinline__ void put_word(unsigned long long* p, unsigned long long v) {
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    }
+    static __device__ __forceinline__ unsigned long long get_word(const unsigned long long* p) {
+        unsigned long long v;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        return v;
     }
 };
 
@@ -162,7 +211,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
     // cells across an open edge stay zero
     for (int q = tid; q < 3 * G::NS; q += NT) sm[q] = 0.0;
     TileRing<S, BYT, RY> ring;
-    ring.init(P, A.flags);
+    ring.init(P, A.box);
     const int x = x0 + static_cast<int>(threadIdx.x), yt = y0 + static_cast<int>(threadIdx.y) * RY;
     const int64_t i0 = layer * z + x + static_cast<int64_t>(Lx) * yt;
     const int base = static_cast<int>(threadIdx.y) * RY * G::PX + static_cast<int>(threadIdx.x);
@@ -181,15 +230,6 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
             sm[2 * G::NS + c] = mn[r].z;
         }
     }
-    auto wait = [&](unsigned int target) { return ring.wait(target, A.status); };
-    // the halo of `src`, which the neighbours' first `target` passes wrote
-    auto stage = [&](const double* src, unsigned int target) -> bool {
-        if (target > 0 && !wait(target)) return false;
-        ring.load(src + layer * z, N, sm);
-        __syncthreads();
-        return true;
-    };
-    auto publish = [&](unsigned int passes) { ring.publish(passes); };
     // field of the thread's sites from the staged tile, m0[r] their own spins: real-space
     // field into B, the sites' energy returned when wanted
     auto field = [&](const double3 (&m0)[RY], double3 (&B)[RY], bool want_e) -> double {
@@ -239,16 +279,18 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
         for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
         if (threadIdx.x == 0) A.partials[static_cast<int64_t>(slot) * nwarps + bid * BYT + threadIdx.y] = e;
     };
-    // new spins v of the thread's sites into the tile and dst (after every thread has read the tile)
-    auto store = [&](const double3 (&v)[RY], double* dst) {
+    // new spins v of the thread's sites: posted as pass `pass` (0: not) as soon as
+    // they are known, into the tile once every thread has read it, and into dst
+    auto store = [&](const double3 (&v)[RY], unsigned int pass, double* dst) {
+        if (pass)
+#pragma unroll
+            for (int r = 0; r < RY; ++r) ring.post(r, v[r], pass);
+        __syncthreads();
 #pragma unroll
         for (int r = 0; r < RY; ++r)
             if (x < Lx && yt + r < Ly) {
-                const int c = own + r * G::PX;
-                sm[c] = v[r].x;
-                sm[G::NS + c] = v[r].y;
-                sm[2 * G::NS + c] = v[r].z;
-                st3(dst, i0 + static_cast<int64_t>(Lx) * r, N, v[r]);
+                ring.set(sm, own + r * G::PX, v[r]);
+                if (dst) st3(dst, i0 + static_cast<int64_t>(Lx) * r, N, v[r]);
             }
     };
     TiledArgs TA = {};
@@ -257,17 +299,18 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
         Pre pre[RY];
         TA.step = A.step0 + static_cast<uint32_t>(k);
         if (C.thermal) prefetch_sites<S, BYT, RY, PASS_SIB1>(P, C, TA, x0, y0, z, pre);
-        const double* src = k == 0 ? A.m_in : A.m + k * A.m_stride;
-        if constexpr (!kTwo)
-            if (k & 1) src = A.mid;
-        if (!stage(src, static_cast<unsigned int>(kTwo ? 2 * k : k))) return;
+        if (k == 0) {
+            ring.load(A.m_in + layer * z, N, sm);
+            __syncthreads();
+        } else if (!ring.fetch(static_cast<unsigned int>(kTwo ? 2 * k : k), sm, A.status)) {
+            return;
+        }
         double3 B[RY], v[RY];
         const int slot = A.e_slot0 + k;
         const bool want_e = A.e_on && slot >= 0;
         const double e = field(mn, B, want_e);
         if (want_e) record(e, slot);
         if constexpr (!kTwo) {
-            double* dst = last ? A.m_out : ((k & 1) ? A.m : A.mid);
 #pragma unroll
             for (int r = 0; r < RY; ++r) {
                 const double3 D = llg_rhs(B[r], mn[r], C.alpha, C.inv_den);
@@ -280,16 +323,18 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
                 v[r] = project(t, mn[r]);
                 if (x < Lx && yt + r < Ly) flag_nonfinite(A.status, v[r]);
             }
-            if (last && !(k & 1)) {
-                // the last spins replace those that this step read: the neighbours have staged them first
-                publish(static_cast<unsigned int>(A.nsteps));
-                if (!wait(static_cast<unsigned int>(A.nsteps))) return;
-            }
-            __syncthreads();
-            store(v, dst);
 #pragma unroll
             for (int r = 0; r < RY; ++r) mn[r] = v[r];
-            publish(static_cast<unsigned int>(last && !(k & 1) ? k + 2 : k + 1));
+            const unsigned int pass = static_cast<unsigned int>(k + 1);
+            if (last && A.nsteps == 1) {
+                // the neighbours may still read the spins that m_out replaces: their
+                // first pass says that they have
+                store(v, pass, nullptr);
+                if (!ring.fetch(pass, sm, A.status)) return;
+                store(v, 0u, A.m_out);
+            } else {
+                store(v, last && !A.e_final ? 0u : pass, last ? A.m_out : nullptr);
+            }
             continue;
         }
         double3 kept[RY];  // Heun: what the corrector needs of the predictor's slopes
@@ -305,12 +350,10 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
                 kept[r] = heun_kept(D, C.thermal, C.thermal ? llg_rhs(pre[r].b, mn[r], C.alpha, C.inv_den) : D);
             }
         }
-        __syncthreads();  // the tile has been read
-        double* mid = A.mid + k * A.mid_stride;
-        store(v, mid);
-        if (last && A.half) return;
-        publish(static_cast<unsigned int>(2 * k + 1));
-        if (!stage(mid, static_cast<unsigned int>(2 * k + 1))) return;
+        const bool end = last && A.half;
+        store(v, end ? 0u : static_cast<unsigned int>(2 * k + 1), A.mid ? A.mid + k * A.mid_stride : nullptr);
+        if (end) return;
+        if (!ring.fetch(static_cast<unsigned int>(2 * k + 1), sm, A.status)) return;
         field(v, B, false);
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
@@ -325,13 +368,11 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
             }
             if (x < Lx && yt + r < Ly) flag_nonfinite(A.status, mn[r]);
         }
-        __syncthreads();
-        store(mn, last ? A.m_out : A.m + (k + 1) * A.m_stride);
-        publish(static_cast<unsigned int>(2 * k + 2));
+        store(mn, last && !A.e_final ? 0u : static_cast<unsigned int>(2 * k + 2),
+              last ? A.m_out : (A.m ? A.m + (k + 1) * A.m_stride : nullptr));
     }
     if (A.e_final) {
-        const unsigned int odd_euler = !kTwo && (A.nsteps & 1) ? 1u : 0u;
-        if (!stage(A.m_out, static_cast<unsigned int>(kTwo ? 2 * A.nsteps : A.nsteps) + odd_euler)) return;
+        if (!ring.fetch(static_cast<unsigned int>(kTwo ? 2 * A.nsteps : A.nsteps), sm, A.status)) return;
         double3 B[RY];
         const double e = field(mn, B, true);
         record(e, A.e_slot0 + A.nsteps);
@@ -383,7 +424,7 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     // one site per thread while the blocks of eight warps that are resident hold
     // the lattice (the shortest chain per pass), two sites per thread above: at
     // six blocks per SM, then at eight with the registers that leaves (64; 512^2
-    // 11.1 us a step where the two launches take 15.8)
+    // 10.3 us a step where the two launches take 15.5)
     const bool one = tiles <= steps_capacity<S, 8, 1, 2, SP, INTEG>(p);
     const bool six = tiles <= steps_capacity<S, 4, 2, 6, SP, INTEG>(p);
     if (!one && !six && tiles > steps_capacity<S, 4, 2, 8, SP, INTEG>(p)) return MJ_OK;
@@ -406,10 +447,10 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     A.half = job->half;
     A.nsteps = job->nsteps;
     A.step0 = job->step0;
-    A.flags = job->flags;
+    A.box = job->box;
     A.status = p->d_status;
-    mj_status st = cuda_status(cudaMemsetAsync(job->flags, 0, sizeof(unsigned int) * kStepsFlagStride * tiles, s),
-                               "step counters");
+    mj_status st = cuda_status(cudaMemsetAsync(job->box, 0, sizeof(unsigned long long) * 12 * steps_box_sites(S::R) * tiles, s),
+                               "step boxes");
     if (st != MJ_OK) return st;
     if (one) return launch_steps_cfg<S, 8, 1, 2, SP, INTEG>(p, C, A, grid, s);
     if (six) return launch_steps_cfg<S, 4, 2, 6, SP, INTEG>(p, C, A, grid, s);

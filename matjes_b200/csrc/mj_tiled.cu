@@ -35,9 +35,14 @@ int64_t tiled_energy_blocks(const mj_plan* p) {
 }
 
 // at most eight resident blocks of 128 threads per SM hold one 32 x 8 tile each
-int64_t steps_flag_words(const mj_plan* p) {
+int64_t steps_tiles(const mj_plan* p) {
+    if (!p->is_stencil || p->sp.shape == 0) return 0;
     const int64_t tiles = static_cast<int64_t>((p->sp.L[0] + 31) / 32) * ((p->sp.L[1] + kStepsTY - 1) / kStepsTY) * p->sp.L[2];
-    return tiles <= 8 * static_cast<int64_t>(p->num_sms) ? tiles * kStepsFlagStride : 0;
+    return tiles <= 8 * static_cast<int64_t>(p->num_sms) ? tiles : 0;
+}
+int64_t steps_box_words(const mj_plan* p) {
+    const int R = p->sp.shape == kShapeTri3 ? ShapeTri3::R : 1;
+    return steps_tiles(p) * 12 * steps_box_sites(R);
 }
 
 mj_status launch_steps(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s) {
