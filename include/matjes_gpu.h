@@ -526,7 +526,11 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
 /* Tile variant (0: 32x16 tiles, 4 sites per thread; 1: 32x16, 2 per thread;
  * 2: 32x32, 4 per thread; 3: 32x8, 2 per thread, registers capped for 8
  * resident blocks of 4 warps; 4: 32x16, 2 per thread, capped for 4 blocks of 8
- * warps) and persistent blocks per SM (1..64). */
+ * warps) and persistent blocks per SM (1..64).  A batch left at its default runs
+ * its steps as launches of many steps over groups of replicas whose tiles are all
+ * resident at once (when each replica alone fits: about 300,000 sites); setting a
+ * configuration makes it run these passes, two launches a step.  The spins are
+ * the same bit for bit. */
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
 /* Times `steps` steps of every (variant, blocks per SM in {2,4,8,16,32}) on the
  * current state (restored afterwards), keeps the fastest; ms_table (25 doubles,

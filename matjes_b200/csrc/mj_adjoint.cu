@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
     for (int q = tid; q < 9 * G::NS; q += 32 * kTBYT) smem_s[q] = 0.0;
     stage_units<S, kTBYT, kTRY>(A.unit, M, Us);
     TileRing<S, kTBYT, kTRY> ring;
-    ring.init(P, A.box);
+    ring.init(P.periodic, P.L[0], P.L[1], blockIdx.x, blockIdx.y, gridDim.x, 0, A.box);
     auto put = [&](double* t, double3 v) {
         if (act[0]) {
             t[own] = v.x;
@@ -718,7 +718,7 @@ mj_status segment_shape(const mj_plan* plan, const DynCoef& c, const TermMasks& 
     const size_t sm = sizeof(double) * (9 * G::NS + static_cast<size_t>(M.nterm) * (S::K + 1) * 9);
     const dim3 grid = tadj_grid<S>(plan->sp);
     int per_sm = 0;
-    fits = !thin_last_tile<S>(plan->sp) &&
+    fits = !thin_last_tile<S>(plan->sp.periodic, plan->sp.L[0], plan->sp.L[1]) &&
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_segment<S>, 32 * kTBYT, sm) == cudaSuccess &&
            static_cast<int64_t>(grid.x) * grid.y <= static_cast<int64_t>(per_sm) * plan->num_sms;
     if (!fits || !args) return MJ_OK;

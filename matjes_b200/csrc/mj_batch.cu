@@ -26,6 +26,7 @@
 
 #include "mj_gneb.cuh"
 #include "mj_mc.cuh"
+#include "mj_steps_impl.cuh"
 #include "mj_tiled_impl.cuh"
 
 namespace mj {
@@ -280,6 +281,140 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_batch(const __grid_constant_
     }
 }
 
+// Many SIB steps of a group of replicas whose tiles are all resident at once, in
+// one launch: the scheme of mj_steps_impl.cuh (a block keeps its 32 x 8 tile, edge
+// spins go through the tiles' boxes, cooperative launch, bounded waits), the
+// arithmetic of the passes above.  A large batch runs group after group between
+// two swap rounds.  us per step, this against the passes: 4 replicas (44 k sites) 4.1 /
+// 13.5, 16 (324 k) 15.0 / 24.8, 64 (1.4 M) 53 / 72, 256 (5.07 M) 188 / 238: small
+// batches were bound by two launches a step, large ones by the corrector's HBM
+// traffic; now instruction issue (37 ps per site and step).
+struct BatchStepTile {
+    int64_t off;      // first packed site of the replica
+    int Lx, Ly;
+    int tx, ty, nx;   // the tile within its replica, tiles a row
+    int tile0;        // the replica's first box in the launch
+    int rep;
+    int pad;
+};
+
+struct BatchStepArgs {
+    const BatchStepTile* tiles;
+    const BatchRep* reps;
+    const double* sigma;
+    double* m;
+    int64_t Ntot;
+    uint32_t step0;
+    int nsteps;
+    unsigned long long* box;
+    int* status;
+};
+
+template <class S, int BYT, int RY, int MINB, int SP>
+__global__ void __launch_bounds__(32 * BYT, MINB) k_batch_steps(const __grid_constant__ StencilParams P,
+                                                                const __grid_constant__ DynCoef C,
+                                                                const BatchStepArgs A) {
+    using G = TileGeom<S, BYT, RY>;
+    extern __shared__ __align__(128) double sm_s[];
+    const BatchStepTile T = A.tiles[blockIdx.x];
+    const int64_t N = A.Ntot;
+    const int tid = threadIdx.x + 32 * threadIdx.y;
+    for (int q = tid; q < 3 * G::NS; q += 32 * BYT) sm_s[q] = 0.0;  // cells across an open edge stay zero
+    TileRing<S, BYT, RY> ring;
+    ring.init(P.periodic, T.Lx, T.Ly, T.tx, T.ty, T.nx, T.tile0, A.box);
+    const int x = T.tx * G::TX + static_cast<int>(threadIdx.x), yt = T.ty * G::TY + static_cast<int>(threadIdx.y) * RY;
+    const int li0 = x + T.Lx * yt;  // the first site within its replica
+    double* m = A.m + T.off;
+    const int base = static_cast<int>(threadIdx.y) * RY * G::PX + static_cast<int>(threadIdx.x);
+    const int own = base + G::R * G::PX + G::RX;
+    const double sigma = A.sigma[T.rep];
+    const bool thermal = sigma != 0.0;
+    const uint32_t stream = C.stream_id + A.reps[T.rep].stream;
+    const double3 zb = make_double3(A.reps[T.rep].zb[0], A.reps[T.rep].zb[1], A.reps[T.rep].zb[2]);
+    const uint32_t step0 = A.step0 + (C.step_base ? *C.step_base : 0u);
+    double3 mn[RY];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RY; ++r) {
+        mn[r] = make_double3(0.0, 0.0, 0.0);
+        if (x < T.Lx && yt + r < T.Ly) {
+            const int li = li0 + T.Lx * r;
+            mn[r] = make_double3(__ldcg(m + li), __ldcg(m + N + li), __ldcg(m + 2 * N + li));
+            ring.set(sm_s, own + r * G::PX, mn[r]);
+        }
+    }
+    // H of the thread's sites (own spins m0) from the staged tile
+    auto field = [&](const double3 (&m0)[RY], const double3 (&draw)[RY], double3 (&H)[RY]) {
+        double bx[RY], by[RY], bz[RY];
+#pragma unroll
+        for (int r = 0; r < RY; ++r) bx[r] = by[r] = bz[r] = 0.0;
+        all_columns<S, BYT, RY, SP>(P, sm_s, base, bx, by, bz, std::make_integer_sequence<int, 2 * S::R + 1>{});
+#pragma unroll
+        for (int r = 0; r < RY; ++r) {
+            double b0 = bx[r], b1 = by[r], b2 = bz[r];
+            if (P.has_onsite) {
+                const double* W = P.W0;
+                if constexpr (SP == SP_AXIAL) {
+                    b2 = fma(W[8], m0[r].z, b2);
+                } else {
+                    b0 = fma(W[0], m0[r].x, fma(W[1], m0[r].y, fma(W[2], m0[r].z, b0)));
+                    b1 = fma(W[3], m0[r].x, fma(W[4], m0[r].y, fma(W[5], m0[r].z, b1)));
+                    b2 = fma(W[6], m0[r].x, fma(W[7], m0[r].y, fma(W[8], m0[r].z, b2)));
+                }
+            }
+            H[r] = make_double3(b0 + zb.x, b1 + zb.y, b2 + zb.z);
+            if (thermal) H[r] = make_double3(H[r].x + draw[r].x, H[r].y + draw[r].y, H[r].z + draw[r].z);
+        }
+    };
+    // posted as pass `pass` (0: not), into the tile once every thread has read it
+    auto store = [&](const double3 (&v)[RY], unsigned int pass) {
+        if (pass)
+#pragma unroll
+            for (int r = 0; r < RY; ++r) ring.post(r, v[r], pass);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RY; ++r)
+            if (x < T.Lx && yt + r < T.Ly) ring.set(sm_s, own + r * G::PX, v[r]);
+    };
+    for (int k = 0; k < A.nsteps; ++k) {
+        double3 draw[RY], H[RY], v[RY];
+        if (thermal) {
+            const uint32_t step = step0 + static_cast<uint32_t>(k);
+            if constexpr (RY % 2 == 0) {
+#pragma unroll
+                for (int r = 0; r < RY; r += 2)
+                    philox_normals_x2(C.keys, C.noise_tab, step, stream, static_cast<uint32_t>(li0 + T.Lx * r),
+                                      static_cast<uint32_t>(li0 + T.Lx * (r + 1)), draw[r], draw[r + 1]);
+            } else {
+#pragma unroll
+                for (int r = 0; r < RY; ++r)
+                    draw[r] = philox_normals_tab(C.keys, C.noise_tab, step, stream, static_cast<uint32_t>(li0 + T.Lx * r));
+            }
+#pragma unroll
+            for (int r = 0; r < RY; ++r)
+                draw[r] = make_double3(sigma * draw[r].x, sigma * draw[r].y, sigma * draw[r].z);
+        }
+        if (k == 0) {
+            ring.load(m, N, sm_s);
+            __syncthreads();
+        } else if (!ring.fetch(static_cast<unsigned int>(2 * k), sm_s, A.status)) {
+            return;
+        }
+        field(mn, draw, H);
+#pragma unroll
+        for (int r = 0; r < RY; ++r) v[r] = sib_solve<true>(mn[r], mn[r], H[r], C.alpha, C.sib_hc);
+        store(v, static_cast<unsigned int>(2 * k + 1));
+        if (!ring.fetch(static_cast<unsigned int>(2 * k + 1), sm_s, A.status)) return;
+        field(v, draw, H);
+#pragma unroll
+        for (int r = 0; r < RY; ++r) mn[r] = sib_solve(mn[r], v[r], H[r], C.alpha, C.sib_hc);
+        if (k + 1 < A.nsteps) store(mn, static_cast<unsigned int>(2 * k + 2));
+    }
+#pragma unroll
+    for (int r = 0; r < RY; ++r)
+        if (x < T.Lx && yt + r < T.Ly) st3(m, li0 + T.Lx * r, N, mn[r]);
+}
+
 // sigma of every replica at its current temperature: the expression and the thermal
 // condition of the single-lattice coefficients
 __global__ void k_batch_sigma(const BatchRep* reps, int nrep, int thermal, double alpha, double dt, double* sigma) {
@@ -521,6 +656,64 @@ mj_status batch_pass(int shape, int variant, int ps, bool zaxial, const StencilP
     }
 }
 
+// tiles of 32 x 8 that are resident at once: one site a thread, two sites a thread
+template <class S>
+void batch_steps_capacity(int num_sms, int cap[2]) {
+    int n = 0;
+    cap[0] = cap[1] = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_steps<S, 8, 1, 2, SP_FULL>, 256,
+                                                      TileGeom<S, 8, 1>::buf_bytes) == cudaSuccess)
+        cap[0] = n * num_sms;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_steps<S, 4, 2, 8, SP_FULL>, 128,
+                                                      TileGeom<S, 4, 2>::buf_bytes) == cudaSuccess)
+        cap[1] = n * num_sms;
+    int a = 0, b = 0;  // the axial forms hold at least as many, or the smaller number counts
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_batch_steps<S, 8, 1, 2, SP_AXIAL>, 256,
+                                                      TileGeom<S, 8, 1>::buf_bytes) == cudaSuccess)
+        cap[0] = std::min(cap[0], a * num_sms);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batch_steps<S, 4, 2, 8, SP_AXIAL>, 128,
+                                                      TileGeom<S, 4, 2>::buf_bytes) == cudaSuccess)
+        cap[1] = std::min(cap[1], b * num_sms);
+}
+
+template <class S>
+mj_status batch_steps_shape(bool zaxial, bool one, const StencilParams& P, const DynCoef& C, const BatchStepArgs& A,
+                            int ntile, cudaStream_t s) {
+    mj_status st = cuda_status(cudaMemsetAsync(A.box, 0, sizeof(unsigned long long) * 12 * steps_box_sites(S::R) *
+                                                             static_cast<size_t>(ntile), s), "batch step boxes");
+    if (st != MJ_OK) return st;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ntile);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const bool axial = zaxial && stencil_axial<S>(P, true);
+    if (one) {
+        cfg.blockDim = dim3(32, 8);
+        cfg.dynamicSmemBytes = TileGeom<S, 8, 1>::buf_bytes;
+        return cuda_status(axial ? cudaLaunchKernelEx(&cfg, k_batch_steps<S, 8, 1, 2, SP_AXIAL>, P, C, A)
+                                 : cudaLaunchKernelEx(&cfg, k_batch_steps<S, 8, 1, 2, SP_FULL>, P, C, A), "k_batch_steps");
+    }
+    cfg.blockDim = dim3(32, 4);
+    cfg.dynamicSmemBytes = TileGeom<S, 4, 2>::buf_bytes;
+    return cuda_status(axial ? cudaLaunchKernelEx(&cfg, k_batch_steps<S, 4, 2, 8, SP_AXIAL>, P, C, A)
+                             : cudaLaunchKernelEx(&cfg, k_batch_steps<S, 4, 2, 8, SP_FULL>, P, C, A), "k_batch_steps");
+}
+
+// f(shape) with the batch's compile-time shape
+template <class Fn>
+auto with_shape(int shape, Fn&& f) {
+    switch (shape) {
+        case kShapeSquareNN: return f(ShapeSquareNN{});
+        case kShapeSquare2: return f(ShapeSquare2{});
+        case kShapeTriNN: return f(ShapeTriNN{});
+        default: return f(ShapeTri3{});
+    }
+}
+
 }  // namespace
 }  // namespace mj
 
@@ -551,6 +744,15 @@ struct mj_batch {
     double* d_noise_tab = nullptr;
     mj::BatchRep* d_reps = nullptr;
     mj::BatchTile* d_tiles = nullptr;
+    // many steps in one launch: the replicas in groups of resident tiles
+    struct StepGroup {
+        int first, count;  // tiles of the group in d_step_tiles
+        bool one;          // one site a thread
+    };
+    bool together = true;             // off once a program picks a pass configuration
+    std::vector<StepGroup> groups;    // empty: a replica is too large
+    mj::BatchStepTile* d_step_tiles = nullptr;
+    int* d_status = nullptr;          // kStatusTimeout of a bounded wait
     double* d_sigma = nullptr;        // per replica, of the current call's alpha and timestep
     int* d_image = nullptr;
     int* d_accept = nullptr;
@@ -589,6 +791,8 @@ void batch_free(mj_batch* b) {
     cudaFree(b->d_reps);
     cudaFree(b->d_tiles);
     cudaFree(b->d_sigma);
+    cudaFree(b->d_step_tiles);
+    cudaFree(b->d_status);
     cudaFree(b->d_image);
     cudaFree(b->d_accept);
     cudaFree(b->d_stepctr);
@@ -643,6 +847,64 @@ mj_status batch_tiles(mj_batch* b, bool upload_reps) {
     }
     return cuda_status(cudaMemcpy(b->d_reps, cur.data(), sizeof(BatchRep) * b->nrep, cudaMemcpyHostToDevice),
                        "batch table");
+}
+
+// The replicas packed into groups of at most the resident tiles (largest first,
+// each into the first group with room); *words the box words of the largest group.
+mj_status batch_groups(mj_batch* b, size_t* words) {
+    *words = 0;
+    int cap[2];
+    bool fits = true;
+    int R = 1;
+    with_shape(b->shape, [&](auto sh) {
+        using S = decltype(sh);
+        batch_steps_capacity<S>(b->num_sms, cap);
+        R = S::R;
+        for (const BatchRep& r : b->reps) fits = fits && !thin_last_tile<S>(b->sp.periodic, r.Lx, r.Ly);
+    });
+    struct Group {
+        std::vector<int> reps;
+        int tiles = 0;
+    };
+    std::vector<Group> groups;
+    std::vector<int> order(b->nrep), tiles(b->nrep);
+    for (int r = 0; r < b->nrep; ++r) {
+        const int64_t t = static_cast<int64_t>((b->reps[r].Lx + 31) / 32) * ((b->reps[r].Ly + kStepsTY - 1) / kStepsTY);
+        fits = fits && t <= cap[1];
+        tiles[r] = fits ? static_cast<int>(t) : 0;
+        order[r] = r;
+    }
+    if (!fits) return MJ_OK;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return tiles[a] > tiles[c]; });
+    size_t open = 0;  // the groups before it are full
+    for (int r : order) {
+        size_t g = open;
+        while (g < groups.size() && groups[g].tiles + tiles[r] > cap[1]) ++g;
+        if (g == groups.size()) groups.emplace_back();
+        groups[g].reps.push_back(r);
+        groups[g].tiles += tiles[r];
+        while (open < groups.size() && groups[open].tiles == cap[1]) ++open;
+    }
+    std::vector<BatchStepTile> all;
+    int most = 0;
+    for (const Group& g : groups) {
+        b->groups.push_back({static_cast<int>(all.size()), g.tiles, g.tiles <= cap[0]});
+        most = std::max(most, g.tiles);
+        int tile0 = 0;
+        for (int r : g.reps) {
+            const BatchRep& q = b->reps[r];
+            const int nx = (q.Lx + 31) / 32, ny = (q.Ly + kStepsTY - 1) / kStepsTY;
+            for (int ty = 0; ty < ny; ++ty)
+                for (int tx = 0; tx < nx; ++tx) all.push_back(BatchStepTile{q.off, q.Lx, q.Ly, tx, ty, nx, tile0, r, 0});
+            tile0 += nx * ny;
+        }
+    }
+    *words = 12 * static_cast<size_t>(steps_box_sites(R)) * most;
+    mj_status st = cuda_status(cudaMalloc(&b->d_step_tiles, sizeof(BatchStepTile) * all.size()), "batch step tiles");
+    if (st == MJ_OK)
+        st = cuda_status(cudaMemcpy(b->d_step_tiles, all.data(), sizeof(BatchStepTile) * all.size(), cudaMemcpyHostToDevice),
+                         "batch step tiles");
+    return st;
 }
 
 mj_status batch_coef(const mj_batch* b, const mj_dyn_params* d, DynCoef& c, double& dt) {
@@ -718,13 +980,39 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
         return cuda_status(cudaGetLastError(), "k_batch_sigma");
     };
     if (nsteps > 0 && (st = sigmas()) != MJ_OK) return st;
+    const bool together = b->together && !b->groups.empty();
     for (int32_t k = 0; k < nsteps; ++k) {
-        const uint32_t step = step0 + static_cast<uint32_t>(k);
-        BatchArgs A = batch_args(b, step);
-        if ((st = batch_pass(b->shape, b->variant, BPASS_SIB1, b->zaxial, b->sp, c, A, nb, s)) != MJ_OK) return st;
-        A.ms = b->d_mid;
-        A.out = b->d_m;
-        if ((st = batch_pass(b->shape, b->variant, BPASS_SIB2, b->zaxial, b->sp, c, A, nb, s)) != MJ_OK) return st;
+        uint32_t step = step0 + static_cast<uint32_t>(k);
+        if (together) {
+            // the steps up to the next swap round, group after group
+            int32_t n = std::min<int32_t>(nsteps - k, 4096);
+            if (swap_every > 0)
+                n = static_cast<int32_t>(std::min<uint32_t>(n, static_cast<uint32_t>(swap_every) - step % static_cast<uint32_t>(swap_every)));
+            for (const mj_batch::StepGroup& g : b->groups) {
+                BatchStepArgs A;
+                A.tiles = b->d_step_tiles + g.first;
+                A.reps = b->d_reps;
+                A.sigma = b->d_sigma;
+                A.m = b->d_m;
+                A.Ntot = b->Ntot;
+                A.step0 = step;
+                A.nsteps = n;
+                A.box = reinterpret_cast<unsigned long long*>(b->d_mid);
+                A.status = b->d_status;
+                st = with_shape(b->shape, [&](auto sh) {
+                    return batch_steps_shape<decltype(sh)>(b->zaxial, g.one, b->sp, c, A, g.count, s);
+                });
+                if (st != MJ_OK) return st;
+            }
+            k += n - 1;
+            step += static_cast<uint32_t>(n - 1);
+        } else {
+            BatchArgs A = batch_args(b, step);
+            if ((st = batch_pass(b->shape, b->variant, BPASS_SIB1, b->zaxial, b->sp, c, A, nb, s)) != MJ_OK) return st;
+            A.ms = b->d_mid;
+            A.out = b->d_m;
+            if ((st = batch_pass(b->shape, b->variant, BPASS_SIB2, b->zaxial, b->sp, c, A, nb, s)) != MJ_OK) return st;
+        }
         if (swap_every > 0 && ((step + 1) % static_cast<uint32_t>(swap_every)) == 0) {
             if ((st = batch_energy(b, c, b->d_E, s)) != MJ_OK) return st;
             // round index (step + 1) / swap_every; in a graph the device counter (a multiple of
@@ -738,6 +1026,15 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
     }
     if (E_out) return batch_energy(b, c, E_out, s);
     return MJ_OK;
+}
+
+// MJ_ERR_TIMEOUT once when a bounded wait of a many-step launch gave up (synchronous).
+mj_status batch_status(const mj_batch* b) {
+    int word = 0;
+    mj_status st = cuda_status(cudaMemcpy(&word, b->d_status, sizeof(int), cudaMemcpyDeviceToHost), "batch status");
+    if (st != MJ_OK || word == 0) return st;
+    cudaMemset(b->d_status, 0, sizeof(int));
+    return set_error(MJ_ERR_TIMEOUT, "a bounded device wait of the batch's steps gave up; its spins are invalid");
 }
 
 // The field of the images for gneb_relax: the batch's field pass with the
@@ -859,7 +1156,14 @@ mj_status mj_batch_create(const mj_lattice_desc* cell, const mj_hamiltonian_desc
     b->Ntot = off;
     auto dal = [&](auto** p, size_t n, const char* w) { return cuda_status(cudaMalloc(reinterpret_cast<void**>(p), n), w); };
     const size_t f3 = sizeof(double) * 3 * static_cast<size_t>(b->Ntot);
-    if ((st = dal(&b->d_m, f3, "batch m")) != MJ_OK || (st = dal(&b->d_mid, f3, "batch mid")) != MJ_OK ||
+    size_t words = 0;  // the many-step launches keep their boxes in the midpoint buffer
+    if ((st = batch_groups(b, &words)) != MJ_OK) {
+        batch_free(b);
+        return st;
+    }
+    if ((st = dal(&b->d_m, f3, "batch m")) != MJ_OK ||
+        (st = dal(&b->d_mid, std::max(f3, sizeof(unsigned long long) * words), "batch mid")) != MJ_OK ||
+        (st = dal(&b->d_status, sizeof(int), "batch status")) != MJ_OK ||
         (st = dal(&b->d_aux, f3, "batch aux")) != MJ_OK || (st = dal(&b->d_E, sizeof(double) * nrep, "batch E")) != MJ_OK ||
         (st = dal(&b->d_slot_kT, sizeof(double) * nrep, "batch ladder")) != MJ_OK ||
         (st = dal(&b->d_noise_tab, sizeof(double) * kNoiseTabDoubles, "batch tables")) != MJ_OK ||
@@ -879,6 +1183,7 @@ mj_status mj_batch_create(const mj_lattice_desc* cell, const mj_hamiltonian_desc
     cudaMemcpy(b->d_slot_kT, b->slot_kT.data(), sizeof(double) * nrep, cudaMemcpyHostToDevice);
     cudaMemcpy(b->d_image, image.data(), sizeof(int) * nrep, cudaMemcpyHostToDevice);
     cudaMemset(b->d_accept, 0, sizeof(int) * nrep);
+    cudaMemset(b->d_status, 0, sizeof(int));
     cudaMemset(b->d_m, 0, f3);
     if ((st = batch_tiles(b, true)) != MJ_OK) {
         batch_free(b);
@@ -940,7 +1245,8 @@ mj_status mj_batch_download(const mj_batch* bc, double* m, void* stream) {
     if ((st = cuda_status(cudaMemcpyAsync(m, b->d_stage, sizeof(double) * 3 * b->Ntot, cudaMemcpyDeviceToHost, s),
                           "batch download")) != MJ_OK)
         return st;
-    return cuda_status(cudaStreamSynchronize(s), "batch download");
+    if ((st = cuda_status(cudaStreamSynchronize(s), "batch download")) != MJ_OK) return st;
+    return batch_status(b);
 }
 
 mj_status mj_batch_step(mj_batch* b, const mj_dyn_params* p, int32_t nsteps, int32_t swap_every, double* E_dev,
@@ -971,7 +1277,7 @@ mj_status mj_batch_graph_run(mj_batch* b, const mj_dyn_params* p, int32_t steps_
         (st = cuda_status(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking), "capture stream")) != MJ_OK)
         return st;
     std::string key(reinterpret_cast<const char*>(&c), sizeof(c));
-    key += std::to_string(sc) + "/" + std::to_string(steps_per_graph) + "/" + std::to_string(swap_every) + "/" +
+    key += std::to_string(b->together) + "/" + std::to_string(sc) + "/" + std::to_string(steps_per_graph) + "/" + std::to_string(swap_every) + "/" +
            std::to_string(reinterpret_cast<uintptr_t>(E_dev)) + "/" + std::to_string(b->variant) + "/" +
            std::to_string(b->blocks_per_sm);
     if (!b->graph || b->graph_key != key) {
@@ -1013,7 +1319,10 @@ mj_status mj_batch_energies(mj_batch* b, double* E_host) {
     std::memset(&c, 0, sizeof(c));
     mj_status st = batch_energy(b, c, b->d_E, 0);
     if (st != MJ_OK) return st;
-    return cuda_status(cudaMemcpy(E_host, b->d_E, sizeof(double) * b->nrep, cudaMemcpyDeviceToHost), "batch energies");
+    if ((st = cuda_status(cudaMemcpy(E_host, b->d_E, sizeof(double) * b->nrep, cudaMemcpyDeviceToHost), "batch energies")) !=
+        MJ_OK)
+        return st;
+    return batch_status(b);
 }
 
 mj_status mj_batch_temperatures(const mj_batch* b, double* T_host, int32_t* accepted) {
@@ -1069,7 +1378,7 @@ mj_status mj_batch_gneb_tangent(mj_batch* b, const double* E_dev, int32_t mode, 
     return cuda_status(cudaGetLastError(), "k_gneb_scale");
 }
 
-mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm) {
+static mj_status batch_configure(mj_batch* b, int32_t variant, int32_t blocks_per_sm) {
     if (!b || variant < 0 || variant >= kBatchVariants || blocks_per_sm < 1 || blocks_per_sm > 64)
         return set_error(MJ_ERR_ARG, "variant 0..4 and blocks_per_sm 1..64");
     cudaSetDevice(b->device);
@@ -1082,6 +1391,12 @@ mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_s
         b->graph_key.clear();
     }
     return retile ? batch_tiles(b, false) : MJ_OK;
+}
+
+mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm) {
+    const mj_status st = batch_configure(b, variant, blocks_per_sm);
+    if (st == MJ_OK) b->together = false;  // the program asked for those passes
+    return st;
 }
 
 mj_status mj_batch_autotune(mj_batch* b, const mj_dyn_params* p, int32_t steps, int32_t* best_variant,
@@ -1100,12 +1415,14 @@ mj_status mj_batch_autotune(mj_batch* b, const mj_dyn_params* p, int32_t steps, 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
+    const bool together = b->together;  // the passes are timed; a batch that steps together keeps doing so
+    b->together = false;
     double best = 1e300;
     int bv = b->variant, bb = b->blocks_per_sm;
     int k = 0;
     for (int v = 0; v < kBatchVariants && st == MJ_OK; ++v)
         for (int q = 0; q < 5 && st == MJ_OK; ++q, ++k) {
-            if ((st = mj_batch_set_config(b, v, bps_list[q])) != MJ_OK) break;
+            if ((st = batch_configure(b, v, bps_list[q])) != MJ_OK) break;
             if ((st = batch_sequence(b, c, sc, p->step0, 1, 0, false, nullptr, 0)) != MJ_OK) break;
             cudaEventRecord(e0, 0);
             if ((st = batch_sequence(b, c, sc, p->step0, steps, 0, false, nullptr, 0)) != MJ_OK) break;
@@ -1125,8 +1442,9 @@ mj_status mj_batch_autotune(mj_batch* b, const mj_dyn_params* p, int32_t steps, 
     cudaEventDestroy(e1);
     cudaMemcpy(b->d_m, save, sizeof(double) * 3 * b->Ntot, cudaMemcpyDeviceToDevice);
     cudaFree(save);
+    b->together = together;
     if (st != MJ_OK) return st;
-    if ((st = mj_batch_set_config(b, bv, bb)) != MJ_OK) return st;
+    if ((st = batch_configure(b, bv, bb)) != MJ_OK) return st;
     *best_variant = bv;
     *best_bps = bb;
     return cuda_status(cudaDeviceSynchronize(), "batch autotune");

@@ -55,8 +55,7 @@ struct StepsArgs {
 
 constexpr uint32_t kStepsWaitPolls = 1u << 20;
 
-// The halo of a block's tile (TileGeom layout; grid x, y over the tiles, z over
-// the layers) and the boxes its cells come from.  A tile's box: [parity][word][kN]
+// The halo of a block's tile (TileGeom layout) and the boxes its cells come from.  A tile's box: [parity][word][kN]
 // over the sites within R of the tile's edge (box_index), word 2 c and 2 c + 1
 // the low and high half of component c.
 template <class S, int BYT, int RY>
@@ -79,13 +78,13 @@ struct TileRing {
         if (lx >= w - R) return 64 * R + (ly - R) * 2 * R + R + lx - (w - R);
         return -1;
     }
-    __device__ __forceinline__ void init(const StencilParams& P, unsigned long long* boxes) {
-        const int Lx = P.L[0], Ly = P.L[1];
+    // tile (bx, by) of the nx tiles a row of an Lx x Ly layer whose first box is number tile0
+    __device__ __forceinline__ void init(const int* periodic, int Lx, int Ly, int bx, int by, int nx, int tile0,
+                                         unsigned long long* boxes) {
         const int tid = threadIdx.x + 32 * threadIdx.y;
-        const int x0 = blockIdx.x * G::TX, y0 = blockIdx.y * G::TY;
+        const int x0 = bx * G::TX, y0 = by * G::TY;
         const int w = min(G::TX, Lx - x0), h = min(G::TY, Ly - y0);
-        const int nx = gridDim.x, ny = gridDim.y, z = blockIdx.z;
-        auto base_of = [&](int tx, int ty) { return 12 * kN * (tx + nx * (ty + ny * z)); };
+        auto base_of = [&](int tx, int ty) { return 12 * kN * (tile0 + tx + nx * ty); };
         box = boxes;
         // the ring of width R about the tile's w x h sites: rows below and above, then the sides
         const int full = w + 2 * R;
@@ -111,7 +110,7 @@ struct TileRing {
             if (c < 2 * R * (full + h)) {
                 int gx = x0 + lx, gy = y0 + ly;
                 const bool outx = gx < 0 || gx >= Lx, outy = gy < 0 || gy >= Ly;
-                if (!((outx && !P.periodic[0]) || (outy && !P.periodic[1]))) {
+                if (!((outx && !periodic[0]) || (outy && !periodic[1]))) {
                     if (outx) gx = ((gx % Lx) + Lx) % Lx;
                     if (outy) gy = ((gy % Ly) + Ly) % Ly;
                     hsrc[q] = gx + Lx * gy;
@@ -125,7 +124,7 @@ struct TileRing {
         for (int r = 0; r < RY; ++r) {
             const int lx = threadIdx.x, ly = threadIdx.y * RY + r;
             const int b = lx < w && ly < h ? box_index(lx, ly, w, h) : -1;
-            obox[r] = b < 0 ? -1 : base_of(blockIdx.x, blockIdx.y) + b;
+            obox[r] = b < 0 ? -1 : base_of(bx, by) + b;
         }
     }
     // the halo cells of a layer of `src` (component stride N) into the tile
@@ -211,7 +210,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
     // cells across an open edge stay zero
     for (int q = tid; q < 3 * G::NS; q += NT) sm[q] = 0.0;
     TileRing<S, BYT, RY> ring;
-    ring.init(P, A.box);
+    ring.init(P.periodic, Lx, Ly, blockIdx.x, blockIdx.y, gridDim.x, gridDim.x * gridDim.y * z, A.box);
     const int x = x0 + static_cast<int>(threadIdx.x), yt = y0 + static_cast<int>(threadIdx.y) * RY;
     const int64_t i0 = layer * z + x + static_cast<int64_t>(Lx) * yt;
     const int base = static_cast<int>(threadIdx.y) * RY * G::PX + static_cast<int>(threadIdx.x);
@@ -398,9 +397,9 @@ mj_status launch_steps_cfg(mj_plan* p, const DynCoef& C, const StepsArgs& A, dim
 // A halo reaches the next tile alone, unless a last tile is thinner than the
 // reach: the one before it is then in reach of the periodic images too.
 template <class S>
-bool thin_last_tile(const StencilParams& P) {
-    auto thin = [&](int d, int t) { return P.periodic[d] && P.L[d] > t && P.L[d] % t != 0 && P.L[d] % t < S::R; };
-    return thin(0, 32) || thin(1, kStepsTY);
+bool thin_last_tile(const int* periodic, int Lx, int Ly) {
+    auto thin = [](bool per, int L, int t) { return per && L > t && L % t != 0 && L % t < S::R; };
+    return thin(periodic[0] != 0, Lx, 32) || thin(periodic[1] != 0, Ly, kStepsTY);
 }
 
 // Resident tiles of a configuration on the plan's device.
@@ -420,7 +419,7 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     const dim3 grid((p->sp.L[0] + 31) / 32, (p->sp.L[1] + kStepsTY - 1) / kStepsTY, p->sp.L[2]);
     const int64_t tiles = static_cast<int64_t>(grid.x) * grid.y * grid.z;
     fits = false;
-    if (thin_last_tile<S>(p->sp)) return MJ_OK;
+    if (thin_last_tile<S>(p->sp.periodic, p->sp.L[0], p->sp.L[1])) return MJ_OK;
     // one site per thread while the blocks of eight warps that are resident hold
     // the lattice (the shortest chain per pass), two sites per thread above: at
     // six blocks per SM, then at eight with the registers that leaves (64; 512^2
