@@ -415,8 +415,8 @@ def run_adjoint(dev: int, reps: int = 3) -> dict:
             "checkpoint_every": d["checkpoint_every"], "forward_ms": f, "forward_graph_ms": fg,
             "forward_backward_ms": a, "cost_ratio": a / f, "cost_ratio_vs_graph_forward": a / fg,
             "gradients": "m0 (3N), J, D, K, per-site B (3N)",
-            "launches_per_step": {"forward": 2, "adjoint": 6},
-            "adjoint_path": "forward and backward sweeps replayed as CUDA graphs"}
+            "launches_per_segment": {"forward": 1, "recompute": 1, "backward": 1},
+            "adjoint_path": "forward, recompute and backward of a segment as one launch of many steps each"}
 
 
 def dipolar_alg_bytes(N: int, nrep) -> float:
@@ -867,7 +867,8 @@ def run_integrator_key(dev, wname, integrator, K, W, noise=None, inject_steps=0)
         bytes_site = {"k_sib1": 48.0 + extra, "k_sib2": 72.0 + extra, "k_sib_fused": 120.0 + 2 * extra}
         step_b = 120.0 + 2 * extra
     else:
-        bytes_site = {"k_heun1": 72.0 + (24.0 if thermal else 0.0), "k_heun2": 72.0 + (24.0 if thermal else 0.0)}
+        # predictor: m in, the prediction and D1/2 (+ the thermal part, one vector) out; corrector: both in, m out
+        bytes_site = {"k_heun1": 72.0, "k_heun2": 72.0}
         step_b = sum(bytes_site.values())
     sec = ms / K / 1e3
     return {"workload": wname, "integrator": integrator, "noise": dyn.get("noise", "off"), "kernels_config": cfg,
