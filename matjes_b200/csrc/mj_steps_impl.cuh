@@ -421,10 +421,20 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     fits = false;
     if (thin_last_tile<S>(p->sp.periodic, p->sp.L[0], p->sp.L[1])) return MJ_OK;
     // one site per thread while the blocks of eight warps that are resident hold
-    // the lattice (the shortest chain per pass), two sites per thread above: at
-    // six blocks per SM, then at eight with the registers that leaves (64; 512^2
-    // 10.3 us a step where the two launches take 15.5)
-    const bool one = tiles <= steps_capacity<S, 8, 1, 2, SP, INTEG>(p);
+    // the lattice (the shortest chain per pass): at two blocks per SM, then three
+    // (80 registers) and four (64).  Two sites per thread above: at six blocks per
+    // SM, then at eight with the registers that leaves (64; 512^2 10.3 us a step
+    // where the two launches take 15.5).  us per SIB step at 10 K, one site at
+    // three or four blocks against two sites at six: square 288^2 4.7 / 5.4, 352 x
+    // 320 4.9 / 5.7, 384^2 5.7 / 6.1 (T = 0 5.4 / 6.2).  A longer reach (three
+    // triangular shells) keeps more in registers: three blocks gain where the
+    // draw gives the eight warps work (352 x 320 6.3 / 6.8, T = 0 5.7 / 5.7 and
+    // 288^2 5.7 / 5.5), four spill (384^2 T = 0 7.1 / 6.4).
+    const bool one2 = tiles <= steps_capacity<S, 8, 1, 2, SP, INTEG>(p);
+    const bool one3 = !one2 && (S::R == 1 || C.thermal) && tiles <= steps_capacity<S, 8, 1, 3, SP, INTEG>(p);
+    bool one4 = false;
+    if constexpr (S::R == 1) one4 = !one2 && !one3 && tiles <= steps_capacity<S, 8, 1, 4, SP, INTEG>(p);
+    const bool one = one2 || one3 || one4;
     const bool six = tiles <= steps_capacity<S, 4, 2, 6, SP, INTEG>(p);
     if (!one && !six && tiles > steps_capacity<S, 4, 2, 8, SP, INTEG>(p)) return MJ_OK;
     fits = true;
@@ -451,7 +461,10 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     mj_status st = cuda_status(cudaMemsetAsync(job->box, 0, sizeof(unsigned long long) * 12 * steps_box_sites(S::R) * tiles, s),
                                "step boxes");
     if (st != MJ_OK) return st;
-    if (one) return launch_steps_cfg<S, 8, 1, 2, SP, INTEG>(p, C, A, grid, s);
+    if (one2) return launch_steps_cfg<S, 8, 1, 2, SP, INTEG>(p, C, A, grid, s);
+    if (one3) return launch_steps_cfg<S, 8, 1, 3, SP, INTEG>(p, C, A, grid, s);
+    if constexpr (S::R == 1)
+        if (one4) return launch_steps_cfg<S, 8, 1, 4, SP, INTEG>(p, C, A, grid, s);
     if (six) return launch_steps_cfg<S, 4, 2, 6, SP, INTEG>(p, C, A, grid, s);
     return launch_steps_cfg<S, 4, 2, 8, SP, INTEG>(p, C, A, grid, s);
 }
