@@ -21,14 +21,14 @@
 // product is kept whenever they exceed 1e-13.  The unpack is fused into the consumers: the field and
 // step kernels read H on the padded (y, x) grid of the lattice planes.
 //
-// With few lattice planes (kZdirMax) the z part is not transformed at all: k_zdirect
+// With few lattice planes (zdirect_pays) the z part is not transformed at all: k_zdirect
 // sums H_z = sum_z' K(ky, kx, z - z') M_z' over the planes for every (ky, kx)
 // column, with K transformed along y and x only.  It serves every N_rep,z, reads
 // and writes the Lz planes alone, and for an open z axis uses the mirror symmetry
 // of K (K_xz and K_yz odd in z, the others even) to read half of K.
 //
-// With more planes than that, when N_rep,z is a power of two up to 32, the z
-// transforms and the pointwise product are one kernel (k_zconv): one warp per (ky, kx) column, lane = z,
+// Otherwise, when N_rep,z is a power of two from 2 to 32, the z transforms and the
+// pointwise product are one kernel (k_zconv): one warp per (ky, kx) column, lane = z,
 // a radix-2 FFT across the lanes by shuffles (forward in decimation in
 // frequency, which leaves the spectrum in bit-reversed order, K_F stored per
 // column in that order, inverse in decimation in time back to natural order).
@@ -261,12 +261,44 @@ __global__ void __launch_bounds__(256) k_zconv(const double2* __restrict__ in, d
 // 16 planes of 128 x 65 columns).  Bound by FP64 (36 fma a pair, Lz^2 pairs a
 // column) and the shared memory reads behind them.
 enum ZdirMode { kZdirMirror = 0, kZdirOpen = 1, kZdirCircular = 2 };
-// Planes it is taken for: up to 16, but up to 8 where k_zconv serves N_rep,z too.
-// us of a field call with this / with k_zconv: 8 planes of 64^2 33.8 / 35.9 and of
-// 128^2 42.1 / 43.9, but 16 planes of 32^2 37.8 / 35.9; with this / with the cuFFT
-// transforms and the separate product: 13 planes of 128^2 48.1 / 63.2 and of
-// 100 x 90 45.9 / 55.0, 6 planes of 64^2 33.8 / 42.2.
-constexpr int kZdirMax = 16, kZdirPow2Max = 8;
+constexpr int kZdirMax = 16;  // planes: two per warp, the spectra in 24 KB of shared memory
+// Whether the direct sum is taken for lz planes of pc columns; `even`: K(-r) = K(r)
+// on the grid, `pow2`: k_zconv serves N_rep,z.  On small planes every route waits for
+// its launches and the one with fewer wins.  On large ones the bytes of K decide:
+// k_zdirect reads complex K, per column and component Lz values with the mirror
+// symmetry, 2 Lz (open) or Lz (circular) without; the transforms read N_rep,z values,
+// real ones when K is even (with images a truncated sum leaves K uneven: complex).
+// us of a field call, direct / k_zconv or cuFFT z and product, n^2 cells (x and y open
+// except where noted; open axes double the columns):
+//   mirror, pow2: 2 planes 192^2 58.8 / 58.9, 256^2 68.6 / 66.3; 4 planes 128^2 41.5 /
+//     43.6, 192^2 89.3 / 87.1; 8 planes 96^2 48.5 / 48.8, 128^2 76.4 / 66.2; uneven
+//     (periodic x, y) 4 planes 512^2 127 / 132, 8 planes 192^2 52.8 / 55.5, 256^2 88.7 / 78.6
+//   mirror, else: 3 planes 384^2 266 / 305; 5 planes 192^2 128 / 131, 256^2 172 / 170;
+//     15 planes 96^2 80 / 83, 128^2 128 / 121; 7 planes 256^2 224 / 257 (cuFFT is slow at
+//     lengths with a factor of 7 or more); uneven 6 planes 512^2 222 / 224, 15 256^2 140 / 149
+//   open (third vector not normal), pow2: 2 planes 96^2 in x, y periodic 33 / 35, 256^2 40.4 /
+//     39.3, 4 planes 64^2 32.2 / 31.5; else: 3 planes 256^2 104 / 107, 5 planes 128^2 55 / 60,
+//     192^2 137 / 131, 7 planes 192^2 180 / 190, 9 planes 96^2 68 / 64; uneven 6 planes 256^2
+//     75 / 79, 384^2 170 / 165, 11 planes 128^2 53 / 61, 9 planes 192^2 74 / 72
+//   circular, pow2: 4 planes 192^2 41.6 / 41.6, 384^2 100 / 95, 8 planes 128^2 41.5 / 39.5;
+//     else: 3 planes 384^2 84 / 86, 512^2 97.7 / 96.0, 9 planes 192^2 60.6 / 61.1,
+//     5 planes 256^2 56.8 / 54.9, 12 planes 192^2 75.5 / 71.6
+// One plane has no z part to transform: the real product is never slower (1024^2 open
+// 348 us, 473 by the direct sum's complex K).
+bool zdirect_pays(int mode, int lz, int64_t pc, bool even, bool pow2) {
+    if (lz < 2 || lz > kZdirMax) return false;
+    const int64_t w = lz * pc;
+    if (mode == kZdirMirror) {
+        if (pow2) return lz <= 4 ? !even || pc <= 40000 : lz <= 8 && pc <= 20000;
+        return !even || lz <= 3 || w <= 400000 || lz % 7 == 0 || lz % 11 == 0 || lz % 13 == 0;
+    }
+    if (mode == kZdirOpen) {
+        if (pow2) return lz <= 2 && pc <= 20000;
+        return lz == 3 || lz == 7 || (lz <= 7 && w <= (even ? 170000 : 400000)) || (lz <= 11 && pc <= 10000);
+    }
+    if (pow2) return lz <= 4 && pc <= 20000;
+    return lz <= 3 ? pc <= 100000 : w <= 160000;
+}
 
 struct KSix {
     double2 xx, xy, xz, yy, yz, zz;
@@ -415,19 +447,35 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
             return fail(st);
         }
         int dims[3] = {nz, ny, nx}, inembed[3] = {nz, ny, nx}, onembed[3] = {nz, ny, nkx};
-        if (d->lz <= kZdirPow2Max || (d->lz <= kZdirMax && !pow2)) {
-            // K along y and x only, for the direct z sum; its mirror symmetry in z
-            // checked value by value
-            bool mirror = nz >= 2 * d->lz;
-            for (int c = 0; c < 6 && mirror; ++c) {
-                const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
-                for (int z = 1; z < d->lz && mirror; ++z) {
-                    const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
-                    const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
-                    for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
-                }
+        // K's symmetries, checked value by value: the mirror in z (open axis), and K(-r) = K(r)
+        bool mirror = nz >= 2 * d->lz, even = true;
+        for (int c = 0; c < 6 && mirror; ++c) {
+            const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
+            for (int z = 1; z < d->lz && mirror; ++z) {
+                const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
+                const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
+                for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
             }
-            d->zdir = 1 + (nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular);
+        }
+        if (d->lz >= 2 && d->lz <= kZdirMax) {
+            double top = 0.0, odd = 0.0;
+            for (int c = 0; c < 6; ++c)
+                for (int z = 0; z < nz; ++z)
+                    for (int y = 0; y < ny; ++y) {
+                        const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr + static_cast<size_t>(y) * nx];
+                        const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>((nz - z) % nz) * d->pr +
+                                              static_cast<size_t>((ny - y) % ny) * nx];
+                        for (int x = 0; x < nx; ++x) {
+                            top = std::max(top, std::fabs(a[x]));
+                            odd = std::max(odd, std::fabs(a[x] - b[x == 0 ? 0 : nx - x]));
+                        }
+                    }
+            even = odd <= 1e-12 * top;
+        }
+        const int zmode = nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular;
+        if (zdirect_pays(zmode, d->lz, d->pc, even, pow2)) {
+            // K along y and x only, for the direct z sum
+            d->zdir = 1 + zmode;
             cufftHandle p2;
             cufftResult r2 = CUFFT_EXEC_FAILED;
             if ((st = al(&d->d_kd, sizeof(cufftDoubleComplex) * 6 * nkc, "dipolar K planes")) == MJ_OK &&
