@@ -178,11 +178,13 @@ mj_status mj_plan_set_fused(mj_plan* plan, int32_t enable);
  *                              launch asks for enough shared memory), so that
  *                              the tiles of a lattice fill the last wave of
  *                              the GPU better;
- *   MJ_OPT_DIP_ZCONV (default 1)  FFT dipolar term with up to 16 lattice
- *                              planes, or a z grid of a power of two up to 32:
- *                              the z part as one kernel, a direct sum or
- *                              transforms with the product (0: cuFFT z
- *                              transforms and a separate product);
+ *   MJ_OPT_DIP_ZCONV (default 1)  FFT dipolar term with few lattice planes, or
+ *                              a z grid of a power of two up to 32: the z part
+ *                              as one kernel, a direct sum or transforms with
+ *                              the product (0: cuFFT z transforms and a
+ *                              separate product; a plan on the direct sum
+ *                              makes their K_F at the first 0, so not inside
+ *                              a stream capture);
  *   MJ_OPT_HOST_ZEROCOPY (default 1)  striped mj_step_host with a mapped pinned
  *                              buffer: kernels write the stepped spins into it
  *                              directly (0: device transposes and copies). */

@@ -1200,7 +1200,15 @@ mj_status mj_plan_set_option(mj_plan* plan, int32_t option, int32_t value) {
             if (value < 0 || value > 64) return set_error(MJ_ERR_ARG, "host stripes must be in [0, 64]");
             plan->host_stripes = value;
             break;
-        case MJ_OPT_DIP_ZCONV: plan->dip_zconv = value != 0; break;
+        case MJ_OPT_DIP_ZCONV: {
+            if (value == 0) {
+                cudaSetDevice(plan->device);
+                const mj_status st = dipolar_transforms(plan);
+                if (st != MJ_OK) return st;
+            }
+            plan->dip_zconv = value != 0;
+            break;
+        }
         case MJ_OPT_HOST_ZEROCOPY: plan->host_zerocopy = value != 0; break;
         case MJ_OPT_BLOCKS_PER_SM: {
             if (value != 0 && (value < 4 || value > 32))

@@ -60,8 +60,11 @@ struct DipolarPlan {
     cufftDoubleComplex* d_kfc = nullptr;   // complex K_F when it is not real
     cufftHandle f2d = 0, fz = 0, b2d = 0;
     bool have_f2d = false, have_fz = false, have_b2d = false;
-    // the direct z sum: K transformed along y and x, [6][nz][y][kx]
+    // the direct z sum: K transformed along y and x, [6][nkd][y][kx] (the lz distances of one sign
+    // when the mirror gives the others, else all nz).  K_F above is then made only when the
+    // cuFFT z transforms are asked for (dipolar_transforms)
     int zdir = 0;                          // 0: not used, else 1 + its mode (ZdirMode)
+    int nkd = 0;
     cufftDoubleComplex* d_kd = nullptr;
     // the fused z convolution: K_F per column [pc][nz][6] (kz in bit-reversed
     // order), real or complex, and the twiddles exp(-2 pi i m / nz), m < nz / 2
@@ -325,7 +328,8 @@ __device__ __forceinline__ void k6_mac(double2 (&h)[3], const KSix& K, double2 m
 
 template <int NW, int ZPT, int MODE>
 __global__ void __launch_bounds__(32 * NW, 2) k_zdirect(const double2* __restrict__ in, double2* __restrict__ out,
-                                                        const double2* __restrict__ kd, int64_t pc, int lz, int nz) {
+                                                        const double2* __restrict__ kd, int64_t pc, int lz, int nz,
+                                                        int nk) {
     extern __shared__ double2 zs[];  // [lz][3][32]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t col = static_cast<int64_t>(blockIdx.x) * 32 + lane;
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(32 * NW, 2) k_zdirect(const double2* __restric
     double2 h[ZPT][3];
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) h[q][0] = h[q][1] = h[q][2] = make_double2(0.0, 0.0);
-    const int64_t ks = static_cast<int64_t>(nz) * pc;  // component stride
+    const int64_t ks = static_cast<int64_t>(nk) * pc;  // component stride (nk planes of K kept)
     const double2* k = kd + (act ? col : 0);
     const int nd = MODE == kZdirCircular ? nz : lz;
     KSix kp = load_k6(k, ks), km = kp;
@@ -402,6 +406,109 @@ void free_plan(DipolarPlan* d) {
     delete d;
 }
 
+// K_F (device, complex, taken over) kept as 6 real values per wave vector when its imaginary
+// parts are rounding, else as it is; with `columns` also in k_zconv's layout.
+mj_status keep_kf(DipolarPlan* d, cufftDoubleComplex* kf, bool columns) {
+    const int nz = d->nrep[2];
+    const int64_t nkc = d->pc * nz;
+    mj_status st = MJ_OK;
+    auto al = [&](auto** ptr, size_t bytes, const char* what) {
+        return cuda_status(cudaMalloc(reinterpret_cast<void**>(ptr), bytes), what);
+    };
+    std::vector<cufftDoubleComplex> h(static_cast<size_t>(6) * nkc);
+    if ((st = cuda_status(cudaMemcpy(h.data(), kf, sizeof(cufftDoubleComplex) * h.size(), cudaMemcpyDeviceToHost),
+                          "K_F download")) != MJ_OK) {
+        cudaFree(kf);
+        return st;
+    }
+    double re = 0.0, im = 0.0;
+    for (const cufftDoubleComplex& c : h) {
+        re = std::max(re, std::fabs(c.x));
+        im = std::max(im, std::fabs(c.y));
+    }
+    d->real_kf = im <= 1e-13 * re;
+    // the fused z convolution's K_F: per column, kz in the lanes' bit-reversed order
+    if (columns) {
+        int bits = 0;
+        while ((1 << bits) < nz) ++bits;
+        auto bitrev = [&](int l) {
+            int r = 0;
+            for (int b = 0; b < bits; ++b) r |= ((l >> b) & 1) << (bits - 1 - b);
+            return r;
+        };
+        const size_t ncol = static_cast<size_t>(d->pc);
+        if (d->real_kf) {
+            std::vector<double> kz(ncol * nz * 6);
+            for (size_t col = 0; col < ncol; ++col)
+                for (int c = 0; c < 6; ++c)
+                    for (int l = 0; l < nz; ++l)
+                        kz[(col * 6 + c) * nz + l] =
+                            h[static_cast<size_t>(c) * nkc + static_cast<size_t>(bitrev(l)) * ncol + col].x;
+            st = al(&d->d_kzr, sizeof(double) * kz.size(), "dipolar K_F columns");
+            if (st == MJ_OK)
+                st = cuda_status(cudaMemcpy(d->d_kzr, kz.data(), sizeof(double) * kz.size(), cudaMemcpyHostToDevice),
+                                 "K_F columns upload");
+        } else {
+            std::vector<cufftDoubleComplex> kz(ncol * nz * 6);
+            for (size_t col = 0; col < ncol; ++col)
+                for (int c = 0; c < 6; ++c)
+                    for (int l = 0; l < nz; ++l)
+                        kz[(col * 6 + c) * nz + l] =
+                            h[static_cast<size_t>(c) * nkc + static_cast<size_t>(bitrev(l)) * ncol + col];
+            st = al(&d->d_kzc, sizeof(cufftDoubleComplex) * kz.size(), "dipolar K_F columns");
+            if (st == MJ_OK)
+                st = cuda_status(cudaMemcpy(d->d_kzc, kz.data(), sizeof(cufftDoubleComplex) * kz.size(),
+                                            cudaMemcpyHostToDevice),
+                                 "K_F columns upload");
+        }
+        if (st != MJ_OK) {
+            cudaFree(kf);
+            return st;
+        }
+        // exp(-2 pi i m / nz), m < nz / 2, rounded once from long double
+        const long double pi = 3.141592653589793238462643383279502884L;
+        for (int m = 0; m < nz / 2; ++m) {
+            const long double a = 2.0L * pi * static_cast<long double>(m) / static_cast<long double>(nz);
+            d->tw[m] = static_cast<double>(std::cos(a));
+            d->tw[16 + m] = static_cast<double>(-std::sin(a));
+        }
+        d->zconv = true;
+    }
+    if (d->real_kf) {
+        std::vector<double> r(h.size());
+        for (size_t q = 0; q < h.size(); ++q) r[q] = h[q].x;
+        if ((st = al(&d->d_kfr, sizeof(double) * r.size(), "dipolar K_F")) != MJ_OK ||
+            (st = cuda_status(cudaMemcpy(d->d_kfr, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice),
+                              "K_F upload")) != MJ_OK) {
+            cudaFree(kf);
+            cudaFree(d->d_kfr);
+            d->d_kfr = nullptr;
+            return st;
+        }
+        cudaFree(kf);
+    } else {
+        d->d_kfc = kf;
+    }
+    return MJ_OK;
+}
+
+// K_F's z transform input from the planes that the direct sum keeps: plane z, or with the
+// mirror plane nz - z with xz and yz negated (no pair of sites is lz planes apart: zero).
+__global__ void k_unfold(const cufftDoubleComplex* __restrict__ kd, cufftDoubleComplex* __restrict__ kf, int64_t pc, int nz,
+                         int nkd, double f) {
+    const int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (q >= 6 * pc * nz) return;
+    const int c = static_cast<int>(q / (pc * nz)), z = static_cast<int>(q / pc % nz);
+    const int zs = z < nkd ? z : nz - z;
+    if (zs >= nkd) {
+        kf[q] = make_cuDoubleComplex(0.0, 0.0);
+        return;
+    }
+    const double g = z >= nkd && (c == 2 || c == 4) ? -f : f;
+    const cufftDoubleComplex v = kd[(static_cast<int64_t>(c) * nkd + zs) * pc + q % pc];
+    kf[q] = make_cuDoubleComplex(g * v.x, g * v.y);
+}
+
 }  // namespace
 
 mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t s) {
@@ -433,79 +540,67 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
         (st = cuda_status(cudaMemsetAsync(d->d_cx, 0, sizeof(cufftDoubleComplex) * 3 * nkc, s), "dipolar memset")) != MJ_OK)
         return fail(st);
 
-    // K_F of the six unique components on the full grid (3D transform, once), scaled by 1/prod(N_rep)
-    cufftDoubleComplex* kf = nullptr;
-    {
-        std::vector<double> k6(static_cast<size_t>(6) * nk);
-        const int sel[6] = {0, 1, 2, 4, 5, 8};
+    // K of the six unique components: its transform along y and x (direct z sum), or K_F on
+    // the full grid (3D transform), each scaled by one over the points transformed, once
+    std::vector<double> k6(static_cast<size_t>(6) * nk);
+    const int sel[6] = {0, 1, 2, 4, 5, 8};
+    for (int c = 0; c < 6; ++c)
+        for (int64_t q = 0; q < nk; ++q) k6[static_cast<size_t>(c) * nk + q] = K[static_cast<size_t>(q) * 9 + sel[c]];
+    // K's symmetries, checked value by value: the mirror in z (open axis), and K(-r) = K(r)
+    bool mirror = nz >= 2 * d->lz, even = true;
+    for (int c = 0; c < 6 && mirror; ++c) {
+        const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
+        for (int z = 1; z < d->lz && mirror; ++z) {
+            const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
+            const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
+            for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
+        }
+    }
+    if (d->lz >= 2 && d->lz <= kZdirMax) {
+        double top = 0.0, odd = 0.0;
         for (int c = 0; c < 6; ++c)
-            for (int64_t q = 0; q < nk; ++q) k6[static_cast<size_t>(c) * nk + q] = K[static_cast<size_t>(q) * 9 + sel[c]];
+            for (int z = 0; z < nz; ++z)
+                for (int y = 0; y < ny; ++y) {
+                    const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr + static_cast<size_t>(y) * nx];
+                    const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>((nz - z) % nz) * d->pr +
+                                          static_cast<size_t>((ny - y) % ny) * nx];
+                    for (int x = 0; x < nx; ++x) {
+                        top = std::max(top, std::fabs(a[x]));
+                        odd = std::max(odd, std::fabs(a[x] - b[x == 0 ? 0 : nx - x]));
+                    }
+                }
+        even = odd <= 1e-12 * top;
+    }
+    const int zmode = nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular;
+    const bool direct = zdirect_pays(zmode, d->lz, d->pc, even, pow2);
+    const int planes = direct && zmode == kZdirMirror ? d->lz : nz;  // of K that are transformed
+    {
         double* d_k6 = nullptr;
-        if ((st = al(&d_k6, sizeof(double) * 6 * nk, "dipolar K")) != MJ_OK) return fail(st);
-        if ((st = al(&kf, sizeof(cufftDoubleComplex) * 6 * nkc, "dipolar K_F")) != MJ_OK) {
+        cufftDoubleComplex* kf = nullptr;
+        if ((st = al(&d_k6, sizeof(double) * 6 * planes * d->pr, "dipolar K")) != MJ_OK) return fail(st);
+        if ((st = al(&kf, sizeof(cufftDoubleComplex) * 6 * planes * d->pc, "dipolar K_F")) != MJ_OK) {
             cudaFree(d_k6);
             return fail(st);
         }
+        const size_t part = sizeof(double) * static_cast<size_t>(planes) * d->pr;  // a component's planes
+        cudaError_t up = cudaSuccess;
+        for (int c = 0; c < 6 && up == cudaSuccess; ++c)
+            up = cudaMemcpyAsync(d_k6 + static_cast<int64_t>(c) * planes * d->pr, &k6[static_cast<size_t>(c) * nk], part,
+                                 cudaMemcpyHostToDevice, s);
         int dims[3] = {nz, ny, nx}, inembed[3] = {nz, ny, nx}, onembed[3] = {nz, ny, nkx};
-        // K's symmetries, checked value by value: the mirror in z (open axis), and K(-r) = K(r)
-        bool mirror = nz >= 2 * d->lz, even = true;
-        for (int c = 0; c < 6 && mirror; ++c) {
-            const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
-            for (int z = 1; z < d->lz && mirror; ++z) {
-                const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
-                const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
-                for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
-            }
-        }
-        if (d->lz >= 2 && d->lz <= kZdirMax) {
-            double top = 0.0, odd = 0.0;
-            for (int c = 0; c < 6; ++c)
-                for (int z = 0; z < nz; ++z)
-                    for (int y = 0; y < ny; ++y) {
-                        const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr + static_cast<size_t>(y) * nx];
-                        const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>((nz - z) % nz) * d->pr +
-                                              static_cast<size_t>((ny - y) % ny) * nx];
-                        for (int x = 0; x < nx; ++x) {
-                            top = std::max(top, std::fabs(a[x]));
-                            odd = std::max(odd, std::fabs(a[x] - b[x == 0 ? 0 : nx - x]));
-                        }
-                    }
-            even = odd <= 1e-12 * top;
-        }
-        const int zmode = nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular;
-        if (zdirect_pays(zmode, d->lz, d->pc, even, pow2)) {
-            // K along y and x only, for the direct z sum
-            d->zdir = 1 + zmode;
-            cufftHandle p2;
-            cufftResult r2 = CUFFT_EXEC_FAILED;
-            if ((st = al(&d->d_kd, sizeof(cufftDoubleComplex) * 6 * nkc, "dipolar K planes")) == MJ_OK &&
-                cudaMemcpyAsync(d_k6, k6.data(), sizeof(double) * 6 * nk, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                (r2 = cufftPlanMany(&p2, 2, dims + 1, inembed + 1, 1, static_cast<int>(d->pr), onembed + 1, 1,
-                                    static_cast<int>(d->pc), CUFFT_D2Z, 6 * nz)) == CUFFT_SUCCESS) {
-                cufftSetStream(p2, s);
-                r2 = cufftExecD2Z(p2, d_k6, d->d_kd);
-                if (r2 == CUFFT_SUCCESS)
-                    k_scale<<<static_cast<unsigned>((6 * nkc + 255) / 256), 256, 0, s>>>(d->d_kd, 6 * nkc,
-                                                                                         1.0 / static_cast<double>(d->pr));
-                cudaStreamSynchronize(s);
-                cufftDestroy(p2);
-            }
-            if (st != MJ_OK || r2 != CUFFT_SUCCESS) {
-                cudaFree(d_k6);
-                cudaFree(kf);
-                return fail(st != MJ_OK ? st : cufft_status(r2, "K plane transforms"));
-            }
-        }
+        const int rank = direct ? 2 : 3, batch = direct ? 6 * planes : 6, o = 3 - rank;
+        const int64_t npc = static_cast<int64_t>(planes) * d->pc;
         cufftHandle pk;
-        cufftResult r = cudaMemcpyAsync(d_k6, k6.data(), sizeof(double) * 6 * nk, cudaMemcpyHostToDevice, s) == cudaSuccess
-                            ? cufftPlanMany(&pk, 3, dims, inembed, 1, static_cast<int>(nk), onembed, 1,
-                                            static_cast<int>(nkc), CUFFT_D2Z, 6)
+        cufftResult r = up == cudaSuccess
+                            ? cufftPlanMany(&pk, rank, dims + o, inembed + o, 1, static_cast<int>(direct ? d->pr : nk),
+                                            onembed + o, 1, static_cast<int>(direct ? d->pc : nkc), CUFFT_D2Z, batch)
                             : CUFFT_EXEC_FAILED;
         if (r == CUFFT_SUCCESS) {
             cufftSetStream(pk, s);
             r = cufftExecD2Z(pk, d_k6, kf);
             if (r == CUFFT_SUCCESS)
-                k_scale<<<static_cast<unsigned>((6 * nkc + 255) / 256), 256, 0, s>>>(kf, 6 * nkc, 1.0 / static_cast<double>(nk));
+                k_scale<<<static_cast<unsigned>((6 * npc + 255) / 256), 256, 0, s>>>(
+                    kf, 6 * npc, 1.0 / static_cast<double>(direct ? d->pr : nk));
             cudaStreamSynchronize(s);
             cufftDestroy(pk);
         }
@@ -514,80 +609,12 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
             cudaFree(kf);
             return fail(cufft_status(r, "K transform"));
         }
-    }
-    // real when the imaginary parts are rounding: keep 6 real values per wave vector
-    {
-        std::vector<cufftDoubleComplex> h(static_cast<size_t>(6) * nkc);
-        if ((st = cuda_status(cudaMemcpy(h.data(), kf, sizeof(cufftDoubleComplex) * h.size(), cudaMemcpyDeviceToHost),
-                              "K_F download")) != MJ_OK) {
-            cudaFree(kf);
+        if (direct) {
+            d->zdir = 1 + zmode;
+            d->nkd = planes;
+            d->d_kd = kf;
+        } else if ((st = keep_kf(d, kf, pow2)) != MJ_OK) {
             return fail(st);
-        }
-        double re = 0.0, im = 0.0;
-        for (const cufftDoubleComplex& c : h) {
-            re = std::max(re, std::fabs(c.x));
-            im = std::max(im, std::fabs(c.y));
-        }
-        d->real_kf = im <= 1e-13 * re;
-        // the fused z convolution's K_F: per column, kz in the lanes' bit-reversed order
-        if (d->zdir == 0 && pow2) {
-            int bits = 0;
-            while ((1 << bits) < nz) ++bits;
-            auto bitrev = [&](int l) {
-                int r = 0;
-                for (int b = 0; b < bits; ++b) r |= ((l >> b) & 1) << (bits - 1 - b);
-                return r;
-            };
-            const size_t ncol = static_cast<size_t>(d->pc);
-            if (d->real_kf) {
-                std::vector<double> kz(ncol * nz * 6);
-                for (size_t col = 0; col < ncol; ++col)
-                    for (int c = 0; c < 6; ++c)
-                        for (int l = 0; l < nz; ++l)
-                            kz[(col * 6 + c) * nz + l] =
-                                h[static_cast<size_t>(c) * nkc + static_cast<size_t>(bitrev(l)) * ncol + col].x;
-                st = al(&d->d_kzr, sizeof(double) * kz.size(), "dipolar K_F columns");
-                if (st == MJ_OK)
-                    st = cuda_status(cudaMemcpy(d->d_kzr, kz.data(), sizeof(double) * kz.size(), cudaMemcpyHostToDevice),
-                                     "K_F columns upload");
-            } else {
-                std::vector<cufftDoubleComplex> kz(ncol * nz * 6);
-                for (size_t col = 0; col < ncol; ++col)
-                    for (int c = 0; c < 6; ++c)
-                        for (int l = 0; l < nz; ++l)
-                            kz[(col * 6 + c) * nz + l] =
-                                h[static_cast<size_t>(c) * nkc + static_cast<size_t>(bitrev(l)) * ncol + col];
-                st = al(&d->d_kzc, sizeof(cufftDoubleComplex) * kz.size(), "dipolar K_F columns");
-                if (st == MJ_OK)
-                    st = cuda_status(cudaMemcpy(d->d_kzc, kz.data(), sizeof(cufftDoubleComplex) * kz.size(),
-                                                cudaMemcpyHostToDevice),
-                                     "K_F columns upload");
-            }
-            if (st != MJ_OK) {
-                cudaFree(kf);
-                return fail(st);
-            }
-            // exp(-2 pi i m / nz), m < nz / 2, rounded once from long double
-            const long double pi = 3.141592653589793238462643383279502884L;
-            for (int m = 0; m < nz / 2; ++m) {
-                const long double a = 2.0L * pi * static_cast<long double>(m) / static_cast<long double>(nz);
-                d->tw[m] = static_cast<double>(std::cos(a));
-                d->tw[16 + m] = static_cast<double>(-std::sin(a));
-            }
-            d->zconv = true;
-        }
-        if (d->real_kf) {
-            std::vector<double> r(h.size());
-            for (size_t q = 0; q < h.size(); ++q) r[q] = h[q].x;
-            if ((st = al(&d->d_kfr, sizeof(double) * r.size(), "dipolar K_F")) != MJ_OK ||
-                (st = cuda_status(cudaMemcpy(d->d_kfr, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice),
-                                  "K_F upload")) != MJ_OK) {
-                cudaFree(kf);
-                return fail(st);
-            }
-            cudaFree(kf);
-        } else {
-            d->d_kfc = kf;
         }
     }
     // 2D real transforms over (y, x) of the lattice planes, batched over (z < Lz, component)
@@ -612,6 +639,36 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
     }
     p->dip = d;
     return MJ_OK;
+}
+
+mj_status dipolar_transforms(mj_plan* p) {
+    DipolarPlan* d = static_cast<DipolarPlan*>(p->dip);
+    if (!d || !d->zdir || d->d_kfr || d->d_kfc) return MJ_OK;
+    const int nz = d->nrep[2];
+    const int64_t nkc = d->pc * nz;
+    cufftDoubleComplex* kf = nullptr;
+    mj_status st = cuda_status(cudaMalloc(&kf, sizeof(cufftDoubleComplex) * 6 * nkc), "dipolar K_F");
+    if (st != MJ_OK) return st;
+    k_unfold<<<static_cast<unsigned>((6 * nkc + 255) / 256), 256>>>(d->d_kd, kf, d->pc, nz, d->nkd,
+                                                                    1.0 / static_cast<double>(nz));
+    st = cuda_status(cudaGetLastError(), "k_unfold");
+    if (st == MJ_OK && nz > 1) {  // along z, a line per column
+        int n1[1] = {nz}, emb[1] = {nz};
+        const int stride = static_cast<int>(d->pc);
+        cufftHandle pz;
+        cufftResult r = cufftPlanMany(&pz, 1, n1, emb, stride, 1, emb, stride, 1, CUFFT_Z2Z, stride);
+        if (r == CUFFT_SUCCESS) {
+            for (int c = 0; c < 6 && r == CUFFT_SUCCESS; ++c) r = cufftExecZ2Z(pz, kf + c * nkc, kf + c * nkc, CUFFT_FORWARD);
+            cudaStreamSynchronize(0);
+            cufftDestroy(pz);
+        }
+        if (r != CUFFT_SUCCESS) st = cufft_status(r, "K z transform");
+    }
+    if (st != MJ_OK) {
+        cudaFree(kf);
+        return st;
+    }
+    return keep_kf(d, kf, false);
 }
 
 void dipolar_destroy(mj_plan* p) {
@@ -648,7 +705,7 @@ mj_status dipolar_apply(mj_plan* p, const double* m, double* /*H unused: consume
         auto go = [&](auto nw, auto zpt) {
             constexpr int W = decltype(nw)::value, Z = decltype(zpt)::value;
             auto run = [&](auto mode) {
-                k_zdirect<W, Z, decltype(mode)::value><<<nb, 32 * W, smem, s>>>(in, out, kd, d->pc, d->lz, nz);
+                k_zdirect<W, Z, decltype(mode)::value><<<nb, 32 * W, smem, s>>>(in, out, kd, d->pc, d->lz, nz, d->nkd);
             };
             switch (d->zdir - 1) {
                 case kZdirMirror: run(std::integral_constant<int, kZdirMirror>{}); break;

@@ -375,6 +375,8 @@ void drop_graph(mj_plan* p);
 
 // dipolar (mj_dipolar.cu)
 mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t s);
+// K_F for the cuFFT z transforms of a plan that sums over the planes directly, on first use (synchronous)
+mj_status dipolar_transforms(mj_plan* p);
 void dipolar_destroy(mj_plan* p);
 // H = K * m on the padded grid; consumers read it through dipolar_view and fold B -= 2H.
 mj_status dipolar_apply(mj_plan* p, const double* m, double* H_unused, cudaStream_t s);
