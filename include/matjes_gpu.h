@@ -530,8 +530,10 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
  * resident blocks of 4 warps; 4: 32x16, 2 per thread, capped for 4 blocks of 8
  * warps) and persistent blocks per SM (1..64).  A batch left at its default runs
  * its steps as launches of many steps over groups of replicas whose tiles are all
- * resident at once (when each replica alone fits: about 300,000 sites); setting a
- * configuration makes it run these passes, two launches a step.  The spins are
+ * resident at once (when each replica alone fits: about 300,000 sites), where there
+ * are enough steps between two swap rounds to pay for the groups' launches (one to
+ * five, more where the groups are half full); setting a configuration makes it run
+ * these passes, two launches a step, always.  The spins are
  * the same bit for bit. */
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
 /* Times `steps` steps of every (variant, blocks per SM in {2,4,8,16,32}) on the

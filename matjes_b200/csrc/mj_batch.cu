@@ -907,6 +907,20 @@ mj_status batch_groups(mj_batch* b, size_t* words) {
     return st;
 }
 
+// Whether n steps run as many-step launches, group after group, or as passes: a group
+// costs its launch and staging (10.8 us) and then 3.4 us a step and 5 to 6 ns per tile
+// and step, a step of passes 11 us and 10 to 12 ns per tile.  us a step of n = 1, 2, 4, 8,
+// many-step / passes: 4 replicas (1 group, 176 tiles) 19.7 10.8 7.1 5.4 / 18.8 16.5 15.0
+// 14.5; 16 (2, 1272) 42 29.6 22.9 19.6 / 32 29.2 27.9 27.2; 64 (5, 5460) 84 59 48 41 / 55 51
+// 50 49; 256 (17, 19920) 362 274 226 198 / 233 230 239 247; 8 of 320 x 480 (8, 4800: groups
+// half full) 152 109 84 72 / 70 66 65 64; 2048 of 16^2 (4, 4096) 78 56 44 37 / 59 52 51 50.
+bool batch_together_pays(const mj_batch* b, int32_t n) {
+    const double groups = static_cast<double>(b->groups.size());
+    double tiles = 0.0;
+    for (const mj_batch::StepGroup& g : b->groups) tiles += g.count;
+    return n * (11.0 + 0.0046 * tiles - 3.4 * groups) > 10.8 * groups - 6.0;
+}
+
 mj_status batch_coef(const mj_batch* b, const mj_dyn_params* d, DynCoef& c, double& dt) {
     if (!d) return set_error(MJ_ERR_ARG, "null dynamics parameters");
     if (d->integrator != MJ_SIB) return set_error(MJ_ERR_UNSUPPORTED, "batches run the SIB integrator");
@@ -983,11 +997,12 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
     const bool together = b->together && !b->groups.empty();
     for (int32_t k = 0; k < nsteps; ++k) {
         uint32_t step = step0 + static_cast<uint32_t>(k);
-        if (together) {
-            // the steps up to the next swap round, group after group
-            int32_t n = std::min<int32_t>(nsteps - k, 4096);
-            if (swap_every > 0)
-                n = static_cast<int32_t>(std::min<uint32_t>(n, static_cast<uint32_t>(swap_every) - step % static_cast<uint32_t>(swap_every)));
+        // the steps up to the next swap round
+        int32_t n = std::min<int32_t>(nsteps - k, 4096);
+        if (swap_every > 0)
+            n = static_cast<int32_t>(std::min<uint32_t>(n, static_cast<uint32_t>(swap_every) - step % static_cast<uint32_t>(swap_every)));
+        if (together && batch_together_pays(b, n)) {
+            // group after group
             for (const mj_batch::StepGroup& g : b->groups) {
                 BatchStepArgs A;
                 A.tiles = b->d_step_tiles + g.first;
