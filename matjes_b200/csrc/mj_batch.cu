@@ -195,7 +195,7 @@ __device__ __forceinline__ double compute_tile_b(const StencilParams& P, const D
                     const bool up = rep + 1 < A.gneb_nimg, down = rep > 0;
                     const double3 mp = up ? ld3(A.ms, i + A.gneb_n, Nt) : m0;
                     const double3 mm = down ? ld3(A.ms, i - A.gneb_n, Nt) : m0;
-                    gneb_path_terms(m0, mp, mm, up, Bv, gs);
+                    gneb_path_terms(m0, mp, mm, gneb_segment(rep, A.gneb_nimg), Bv, gs);
                 }
             } else if constexpr (PASS == BPASS_SIB1) {
                 e += total_energy_part(f, m0, zero);

@@ -424,10 +424,27 @@ __device__ __forceinline__ double unit_angle2(double u2, double3 a, double3 b) {
     return l * l;
 }
 
+// The same for spins that may be off unit length (a path's end images, which the
+// relaxation never moves: it normalises the others): by the norms' deviation d the
+// series would be wrong by d.  Norms within a rounding of 1 keep it.
+__device__ __forceinline__ double any_angle2(double u2, double3 a, double3 b) {
+    if (fabs(dot(a, a) - 1.0) < 2e-15 && fabs(dot(b, b) - 1.0) < 2e-15) return unit_angle2(u2, a, b);
+    const double3 c = cross(a, b);
+    const double l = atan2(sqrt(dot(c, c)), dot(a, b));
+    return l * l;
+}
+
+// Image r's segment to image r + 1: none, between moved images, or with an end image.
+enum GnebSegment { kSegNone = 0, kSegInner = 1, kSegEnd = 2 };
+__device__ __forceinline__ int gneb_segment(int r, int nimg) {
+    if (r + 1 >= nimg) return kSegNone;
+    return r == 0 || r + 2 == nimg ? kSegEnd : kSegInner;
+}
+
 // The six GNEB path sums of one site (GNEB/tangent.f90, gneb_utils.f90):
 // A = P(m_{r+1} - m), B = P(m - m_{r-1}) (zero at the ends), |A|^2, A.B, |B|^2,
-// F.A, F.B, squared angle to image r + 1.
-__device__ __forceinline__ void gneb_path_terms(double3 m0, double3 mp, double3 mm, bool up, double3 F, double (&g)[6]) {
+// F.A, F.B, squared angle to image r + 1 (seg: gneb_segment).
+__device__ __forceinline__ void gneb_path_terms(double3 m0, double3 mp, double3 mm, int seg, double3 F, double (&g)[6]) {
     double3 u = make_double3(mp.x - m0.x, mp.y - m0.y, mp.z - m0.z);
     double3 w = make_double3(m0.x - mm.x, m0.y - mm.y, m0.z - mm.z);
     const double u2 = dot(u, u);
@@ -439,7 +456,8 @@ __device__ __forceinline__ void gneb_path_terms(double3 m0, double3 mp, double3 
     g[2] += dot(w, w);
     g[3] += dot(F, u);
     g[4] += dot(F, w);
-    if (up) g[5] += unit_angle2(u2, m0, mp);
+    if (seg == kSegInner) g[5] += unit_angle2(u2, m0, mp);
+    else if (seg == kSegEnd) g[5] += any_angle2(u2, m0, mp);
 }
 
 }  // namespace mj

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) k_gneb_sums(const double* __restrict__ m,
             f = make_double3(f.x - d * m0.x, f.y - d * m0.y, f.z - d * m0.z);
             st3(F, i, X.cs, f);
             double g6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            gneb_path_terms(m0, mp, mm, up, f, g6);
+            gneb_path_terms(m0, mp, mm, gneb_segment(r, nrep), f, g6);
             for (int k = 0; k < 6; ++k) g[k] += g6[k];
             if (esite) g[6] += esite[r * X.n + li];
         }

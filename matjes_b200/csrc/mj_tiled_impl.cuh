@@ -78,7 +78,7 @@ struct TiledArgs {
     int smem_bytes;     // host side: dynamic shared memory of the launch when above the
                         // tile's (caps the resident blocks per SM; the excess is unused)
     const int* stop;    // PASS_GNEB: device flag, the launch does nothing when set (may be null)
-    int img_up, img_dn; // PASS_GNEB, set per block: the image has a next / a previous one
+    int img_up, img_dn; // PASS_GNEB, set per block: the segment to the next image (GnebSegment) / has a previous one
 };
 
 // Programmatic dependent launch: a kernel lets the next one in its stream launch
@@ -492,7 +492,7 @@ __device__ __forceinline__ double sites_epilogue(const StencilParams& P, const D
                 st3(A.out, i, N, f);
                 const double3 mp = A.img_up ? ld3(A.ms + 3 * N, i, N) : m0;
                 const double3 mm = A.img_dn ? ld3(A.ms - 3 * N, i, N) : m0;
-                gneb_path_terms(m0, mp, mm, A.img_up != 0, f, g6);
+                gneb_path_terms(m0, mp, mm, A.img_up, f, g6);
             } else {
                 double3 hd = make_double3(0.0, 0.0, 0.0);
                 if constexpr (HD) hd = ld_dip(A.Hd, x, y, z);
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_tiled(const __grid_constant_
         if (A.out) A.out += 3 * n * img;
         if (A.aux) A.aux += n * img;
     }
-    A.img_up = img + 1 < A0.nimg ? 1 : 0;
+    A.img_up = gneb_segment(static_cast<int>(img), A0.nimg);
     A.img_dn = img > 0 ? 1 : 0;
     const int x0 = blockIdx.x * G::TX, y0 = by * G::TY;
     const int bid = blockIdx.x + gridDim.x * (by + nty * blockIdx.z);
