@@ -187,7 +187,14 @@ mj_status mj_plan_set_fused(mj_plan* plan, int32_t enable);
  *                              a stream capture);
  *   MJ_OPT_HOST_ZEROCOPY (default 1)  striped mj_step_host with a mapped pinned
  *                              buffer: kernels write the stepped spins into it
- *                              directly (0: device transposes and copies). */
+ *                              directly (0: device transposes and copies);
+ *   MJ_OPT_TEST_TIMEOUT (default 0)  1: the tiles of the many-step launches post
+ *                              nothing to each other, so that every wait between
+ *                              them runs out (about a second a launch): a test of
+ *                              the failure path and of a program's handling of
+ *                              it.  A wait that runs out is reported as
+ *                              MJ_ERR_TIMEOUT; until then the energies and
+ *                              gradients are NaN, the spins invalid. */
 enum {
     MJ_OPT_TMA = 0,
     MJ_OPT_FUSED = 1,
@@ -196,7 +203,8 @@ enum {
     MJ_OPT_HOST_STRIPES = 4,
     MJ_OPT_BLOCKS_PER_SM = 5,
     MJ_OPT_DIP_ZCONV = 6,
-    MJ_OPT_HOST_ZEROCOPY = 7
+    MJ_OPT_HOST_ZEROCOPY = 7,
+    MJ_OPT_TEST_TIMEOUT = 8
 };
 mj_status mj_plan_set_option(mj_plan* plan, int32_t option, int32_t value);
 /* Autotuner: times `steps` steps of `p` for every kernel configuration of the
@@ -536,6 +544,8 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
  * these passes, two launches a step, always.  The spins are
  * the same bit for bit. */
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
+/* Options of a batch, as mj_plan_set_option's: MJ_OPT_TEST_TIMEOUT. */
+mj_status mj_batch_set_option(mj_batch* b, int32_t option, int32_t value);
 /* Times `steps` steps of every (variant, blocks per SM in {2,4,8,16,32}) on the
  * current state (restored afterwards), keeps the fastest; ms_table (25 doubles,
  * may be NULL) gets ms per step in variant-major order. */

@@ -29,7 +29,7 @@ MJ_NOISE_PHILOX = 1
 MJ_NOISE_INJECT = 2
 MJ_MAX_ATOMS = 16
 MJ_OPT_TMA, MJ_OPT_FUSED, MJ_OPT_PDL, MJ_OPT_STORE_DRAW, MJ_OPT_HOST_STRIPES, MJ_OPT_BLOCKS_PER_SM = 0, 1, 2, 3, 4, 5
-MJ_OPT_DIP_ZCONV, MJ_OPT_HOST_ZEROCOPY = 6, 7
+MJ_OPT_DIP_ZCONV, MJ_OPT_HOST_ZEROCOPY, MJ_OPT_TEST_TIMEOUT = 6, 7, 8
 
 INTEGRATORS = {"euler": MJ_EULER, "heun": MJ_HEUN_MATJES, "heun_matjes": MJ_HEUN_MATJES, "sib": MJ_SIB}
 NOISES = {"off": MJ_NOISE_OFF, "philox": MJ_NOISE_PHILOX, "inject": MJ_NOISE_INJECT}
@@ -194,6 +194,7 @@ SIGNATURES = {
     "mj_batch_gneb_path": (C.c_int32, [P, P, P, P, P, P, P, P]),
     "mj_gneb_path": (C.c_int32, [P, P, C.c_int32, P, P, P, P, P, P, P, P]),
     "mj_batch_set_config": (C.c_int32, [P, C.c_int32, C.c_int32]),
+    "mj_batch_set_option": (C.c_int32, [P, C.c_int32, C.c_int32]),
     "mj_batch_autotune": (C.c_int32, [P, C.POINTER(DynParams), C.c_int32, C.POINTER(C.c_int32),
                                       C.POINTER(C.c_int32), P]),
     "mj_batch_mc": (C.c_int32, [P, C.POINTER(McParams), C.c_int32, C.c_int32, C.c_int32, P, P, P,

@@ -33,7 +33,8 @@ mj_status status_from_word(mj_plan* p, int word) {
     cudaMemset(p->d_status, 0, sizeof(int));
     cudaMemset(p->d_counter, 0, 4 * sizeof(unsigned int));
     if (word & kStatusTimeout)
-        return set_error(MJ_ERR_TIMEOUT, "a bounded device wait (TMA mbarrier) gave up; results of that launch are invalid");
+        return set_error(MJ_ERR_TIMEOUT, "a bounded device wait (TMA mbarrier, or between the tiles of a many-step launch) gave up; "
+                                          "results of that launch are invalid");
     return set_error(MJ_ERR_NAN, "a time step wrote a non-finite spin component; the state is invalid from that step on");
 }
 
@@ -501,7 +502,7 @@ mj_status steps_together(mj_plan* p, double* m, const DynCoef& c, int energy_mod
         st = launch_steps(p, &j, c, &warps, used, s);
         prof_end(p, rec, s);
         if (st != MJ_OK) return st;
-        if (slots > 0 && (st = launch_steps_energy(p->d_aux, warps, slots, E, s)) != MJ_OK) return st;
+        if (slots > 0 && (st = launch_steps_energy(p->d_aux, warps, slots, E, p->d_status, s)) != MJ_OK) return st;
     }
     return MJ_OK;
 }
@@ -1210,6 +1211,7 @@ mj_status mj_plan_set_option(mj_plan* plan, int32_t option, int32_t value) {
             break;
         }
         case MJ_OPT_HOST_ZEROCOPY: plan->host_zerocopy = value != 0; break;
+        case MJ_OPT_TEST_TIMEOUT: plan->mute_tiles = value != 0; break;
         case MJ_OPT_BLOCKS_PER_SM: {
             if (value != 0 && (value < 4 || value > 32))
                 return set_error(MJ_ERR_ARG, "blocks per SM must be 0 or in [4, 32]");

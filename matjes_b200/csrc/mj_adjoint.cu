@@ -596,6 +596,7 @@ struct SegArgs {
     const double* bmap;
     const double* unit;
     unsigned long long* box;
+    int mute;            // 1: nothing is posted (a test of the waits)
     int* status;
     AdjReduce R;
 };
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
     for (int q = tid; q < 9 * G::NS; q += 32 * kTBYT) smem_s[q] = 0.0;
     stage_units<S, kTBYT, kTRY>(A.unit, M, Us);
     TileRing<S, kTBYT, kTRY> ring;
-    ring.init(P.periodic, P.L[0], P.L[1], blockIdx.x, blockIdx.y, gridDim.x, 0, A.box);
+    ring.init(P.periodic, P.L[0], P.L[1], blockIdx.x, blockIdx.y, gridDim.x, 0, A.box, A.mute);
     auto put = [&](double* t, double3 v) {
         if (act[0]) {
             t[own] = v.x;
@@ -647,9 +648,10 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
         ring.load(A.gH1, N, tA);
     }
     unsigned int pass = 0;
-    bool ok = true;               // no wait gave up
+    bool ok = !timed_out(A.status);  // no wait gave up, here or in the launches that made the segment
     bool more = A.with_gH1 != 0;  // gH1 of the step after adds to dL/dm
-    for (int k = A.len - 1; k >= 0; --k) {
+    ok = __syncthreads_and(ok);
+    for (int k = A.len - 1; k >= 0 && ok; --k) {
         const double* mk = k == 0 ? A.m0 : A.segm + k * n3;
         const double* bk = A.segb + k * n3;
         const double3 m0 = act[0] ? ld3(mk, i, N) : zero, b0 = act[0] ? ld3(bk, i, N) : zero;
@@ -686,8 +688,14 @@ __global__ void __launch_bounds__(32 * kTBYT, 2) k_adj_segment(const __grid_cons
         if (M.nterm > 0) tiled_term_grads<S, kTBYT, kTRY>(Us, M, tC, base, gh1, act, acc);
         __syncthreads();  // the tiles of m_n and mb have been read
     }
-    // after a timeout the results are invalid, but every block still takes part in the reduction
-    if (act[0] && ok) {
+    // after a timeout the results are NaN, and every block still takes part in the reduction
+    if (!ok) {
+        const double n = no_number();
+        part = gbs = make_double3(n, n, n);
+#pragma unroll
+        for (int t = 0; t < kMaxTerms; ++t) acc[t] = n;
+    }
+    if (act[0]) {
         st3(A.mpart, i, N, part);
         if (A.gb) st3(A.gb, i, N, gbs);
     }
@@ -1084,6 +1092,7 @@ void backward_launches(mj_adjoint* a, const DynCoef& c, uint32_t step0, bool wan
             g.bmap = plan->d_bmap;
             g.unit = plan->d_unit;
             g.box = a->d_box;
+            g.mute = plan->mute_tiles ? 1 : 0;
             g.status = plan->d_status;
             g.acc = a->d_acc;
             g.acc_in = first ? 0 : 1;
@@ -1127,7 +1136,8 @@ std::string sweep_key(const mj_adjoint* a, const DynCoef& c, uint32_t step0, int
     k.append(reinterpret_cast<const char*>(&a->plan->sp), sizeof(StencilParams));
     const void* ptrs[2] = {a->plan->d_bmap, a->plan->d_unit};
     k.append(reinterpret_cast<const char*>(ptrs), sizeof(ptrs));
-    k += "/" + std::to_string(step0) + "/" + std::to_string(flags) + "/" + std::to_string(a->plan->steps_together);
+    k += "/" + std::to_string(step0) + "/" + std::to_string(flags) + "/" + std::to_string(a->plan->steps_together) +
+         "/" + std::to_string(a->plan->mute_tiles);
     return k;
 }
 

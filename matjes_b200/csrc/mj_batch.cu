@@ -307,6 +307,7 @@ struct BatchStepArgs {
     uint32_t step0;
     int nsteps;
     unsigned long long* box;
+    int mute;        // 1: nothing is posted (a test of the waits)
     int* status;
 };
 
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_batch_steps(const __grid_con
     const int tid = threadIdx.x + 32 * threadIdx.y;
     for (int q = tid; q < 3 * G::NS; q += 32 * BYT) sm_s[q] = 0.0;  // cells across an open edge stay zero
     TileRing<S, BYT, RY> ring;
-    ring.init(P.periodic, T.Lx, T.Ly, T.tx, T.ty, T.nx, T.tile0, A.box);
+    ring.init(P.periodic, T.Lx, T.Ly, T.tx, T.ty, T.nx, T.tile0, A.box, A.mute);
     const int x = T.tx * G::TX + static_cast<int>(threadIdx.x), yt = T.ty * G::TY + static_cast<int>(threadIdx.y) * RY;
     const int li0 = x + T.Lx * yt;  // the first site within its replica
     double* m = A.m + T.off;
@@ -424,8 +425,9 @@ __global__ void k_batch_sigma(const BatchRep* reps, int nrep, int thermal, doubl
     sigma[r] = thermal && (kT * alpha > 1e-10) && (kT > 1e-8) ? sqrt(alpha * kT * kHbar / dt) : 0.0;
 }
 
-// per-replica energies: tile partials summed in tile order, one block per replica
-__global__ void k_batch_energy(const BatchRep* reps, int nrep, const double* tile_e, double* E) {
+// per-replica energies: tile partials summed in tile order, one block per replica; NaN
+// while a timeout stands unreported (a swap round on it moves nothing)
+__global__ void k_batch_energy(const BatchRep* reps, int nrep, const double* tile_e, double* E, const int* status) {
     const int r = blockIdx.x;
     if (r >= nrep) return;
     __shared__ double part[256];
@@ -437,7 +439,7 @@ __global__ void k_batch_energy(const BatchRep* reps, int nrep, const double* til
     if (threadIdx.x == 0) {
         double tot = 0.0;
         for (int k = 0; k < static_cast<int>(blockDim.x); ++k) tot += part[k];
-        E[r] = tot;
+        E[r] = timed_out(status) ? no_number() : tot;
     }
 }
 
@@ -753,6 +755,7 @@ struct mj_batch {
     std::vector<StepGroup> groups;    // empty: a replica is too large
     mj::BatchStepTile* d_step_tiles = nullptr;
     int* d_status = nullptr;          // kStatusTimeout of a bounded wait
+    bool mute_tiles = false;          // the many-step launches' tiles post nothing (a test of the waits)
     double* d_sigma = nullptr;        // per replica, of the current call's alpha and timestep
     int* d_image = nullptr;
     int* d_accept = nullptr;
@@ -978,7 +981,7 @@ mj_status batch_energy(mj_batch* b, const DynCoef& c, double* E, cudaStream_t s)
     A.tile_e = b->d_tile_e;
     mj_status st = batch_pass(b->shape, b->variant, BPASS_ENERGY, b->zaxial, b->sp, c, A, batch_blocks(b), s);
     if (st != MJ_OK) return st;
-    k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E);
+    k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E, b->d_status);
     return cuda_status(cudaGetLastError(), "k_batch_energy");
 }
 
@@ -1013,6 +1016,7 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
                 A.step0 = step;
                 A.nsteps = n;
                 A.box = reinterpret_cast<unsigned long long*>(b->d_mid);
+                A.mute = b->mute_tiles ? 1 : 0;
                 A.status = b->d_status;
                 st = with_shape(b->shape, [&](auto sh) {
                     return batch_steps_shape<decltype(sh)>(b->zaxial, g.one, b->sp, c, A, g.count, s);
@@ -1069,7 +1073,7 @@ struct BatchFields {
         A.tile_e = b->d_tile_e;
         mj_status e = batch_pass(b->shape, b->variant, BPASS_FIELD, b->zaxial, b->sp, c, A, batch_blocks(b), s);
         if (e != MJ_OK) return e;
-        k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E);
+        k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E, b->d_status);
         return cuda_status(cudaGetLastError(), "k_batch_energy");
     }
     mj_status iterate(double* F, double* m, double* E, double* img, const GnebCtl* ctl) {
@@ -1366,7 +1370,7 @@ mj_status mj_batch_field(mj_batch* b, double* B_dev, double* E_dev, int32_t proj
     mj_status st = batch_pass(b->shape, b->variant, B_dev ? BPASS_FIELD : BPASS_ENERGY, b->zaxial, b->sp, c, A, batch_blocks(b), s);
     if (st != MJ_OK) return st;
     if (E_dev) {
-        k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E_dev);
+        k_batch_energy<<<b->nrep, 256, 0, s>>>(b->d_reps, b->nrep, b->d_tile_e, E_dev, b->d_status);
         return cuda_status(cudaGetLastError(), "k_batch_energy");
     }
     return MJ_OK;
@@ -1406,6 +1410,16 @@ static mj_status batch_configure(mj_batch* b, int32_t variant, int32_t blocks_pe
         b->graph_key.clear();
     }
     return retile ? batch_tiles(b, false) : MJ_OK;
+}
+
+mj_status mj_batch_set_option(mj_batch* b, int32_t option, int32_t value) {
+    if (!b) return set_error(MJ_ERR_ARG, "null batch");
+    switch (option) {
+        case MJ_OPT_TEST_TIMEOUT: b->mute_tiles = value != 0; break;
+        default: return set_error(MJ_ERR_ARG, "unknown batch option " + std::to_string(option));
+    }
+    b->graph_key.clear();
+    return MJ_OK;
 }
 
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm) {

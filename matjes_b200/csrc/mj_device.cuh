@@ -397,6 +397,11 @@ __device__ void grid_reduce(double (&v)[NV], double* partials, unsigned int* cou
     if (tid == 0) *counter = 0u;
 }
 
+// A timeout of a bounded wait stands in the status word: what was made of that launch's
+// results must not pass for a number.
+__device__ __forceinline__ bool timed_out(const int* status) { return (*status & kStatusTimeout) != 0; }
+__device__ __forceinline__ double no_number() { return __longlong_as_double(0x7ff8000000000000LL); }
+
 // ---------------------------------------------------------------------------
 // Squared angle between two unit vectors from u2 = |a - b|^2 = 4 sin^2(angle/2):
 // 4 arcsin^2(x) = 4 sum_n a_n x^2n at x^2 = u2 / 4, a_1 = 1, a_{n+1} = a_n 2 n^2 /

@@ -114,8 +114,8 @@ void build_noise_tables(double* tab);
 }  // namespace mj
 
 namespace mj {
-// d_aux holds at least this many doubles: the energy partials of a launch of many
-// steps, up to 8 per tile and step.
+// Where the many-step launches serve the lattice (steps_tiles > 0) d_aux holds at
+// least this many doubles: their energy partials, up to 8 per tile and step.
 constexpr int64_t kStepsAuxDoubles = 32768;
 
 // The working memory of a GNEB relaxation (mj_gneb.cuh), kept by the plan or
@@ -154,6 +154,7 @@ struct mj_plan {
     bool store_draw = true;          // SIB: the predictor stores its Philox draw for the corrector (else recomputed)
     bool steps_together = true;             // many steps in one launch where the lattice fits (off once a
                                             // program picks a kernel variant)
+    bool mute_tiles = false;                // their tiles post nothing (a test of the waits)
     unsigned long long* d_steps_box = nullptr;  // their tiles' boxes, in d_mid (null: the lattice does not fit)
     int64_t aux_doubles = 0;                    // size of d_aux
     unsigned int* d_sched = nullptr; // fused step scheduler: work counter, exit ticket, done tiles per row
@@ -318,7 +319,7 @@ struct StepsJob {
 };
 mj_status launch_steps(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warps, bool& fits, cudaStream_t s);
 // E[k] = the sum of slot k's n partials, k < slots
-mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, cudaStream_t s);
+mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, const int* status, cudaStream_t s);
 // tiles of the plan's lattice, 0 when it has more than any configuration keeps resident
 // (or no tiled kernels); words of their boxes
 int64_t steps_tiles(const mj_plan* p);

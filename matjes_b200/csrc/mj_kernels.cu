@@ -592,8 +592,13 @@ __global__ void __launch_bounds__(256) k_soa_to_aos_stream(const double* __restr
 // energy partials summed in the fixed order of ordered_sum (one block)
 __global__ void k_ordered_sum1(const double* partials, int nblocks, double* out) { ordered_sum<1>(partials, nblocks, out); }
 
-// E[slot]: a slot's energy partials in the same fixed order (mj_steps_impl.cuh)
-__global__ void __launch_bounds__(256) k_steps_energy(const double* partials, int n, double* E) {
+// E[slot]: a slot's energy partials in the same fixed order (mj_steps_impl.cuh), NaN after
+// a timeout
+__global__ void __launch_bounds__(256) k_steps_energy(const double* partials, int n, double* E, const int* status) {
+    if (timed_out(status)) {
+        if (threadIdx.x == 0) E[blockIdx.x] = no_number();
+        return;
+    }
     ordered_sum<1>(partials + static_cast<int64_t>(blockIdx.x) * n, n, E + blockIdx.x);
 }
 
@@ -942,8 +947,8 @@ mj_status launch_ordered_sum(const double* partials, int nblocks, int nthreads, 
     k_ordered_sum1<<<1, nthreads, 0, s>>>(partials, nblocks, out);
     return cuda_status(cudaGetLastError(), "k_ordered_sum1");
 }
-mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, cudaStream_t s) {
-    k_steps_energy<<<slots, 256, 0, s>>>(partials, n, E);
+mj_status launch_steps_energy(const double* partials, int n, int slots, double* E, const int* status, cudaStream_t s) {
+    k_steps_energy<<<slots, 256, 0, s>>>(partials, n, E, status);
     return cuda_status(cudaGetLastError(), "k_steps_energy");
 }
 mj_status soa_to_aos(const double* so, double* a, int64_t n, cudaStream_t s) {

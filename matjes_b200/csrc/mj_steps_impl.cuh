@@ -18,7 +18,12 @@
 // tile reads also reads it).  The thermal draw of a step is made before the wait,
 // and neither it nor m_n goes through memory between the passes.  The launch is
 // cooperative, so all blocks run at once and every wait ends; the waits are
-// bounded all the same (kStatusTimeout).
+// bounded all the same.  A tile whose wait gives up sets kStatusTimeout and returns;
+// the others, which by then wait for it or for its neighbours, follow at about the
+// same time.  The energies of such a launch become NaN (k_steps_energy,
+// k_batch_energy), and so do the adjoint's gradients; the spins stay as they are, to
+// be asked for with the status word.  (NaN spins from here, a limit in a register or a
+// look at the status word in the wait's loop cost 2 to 10 % of a step.)
 //
 // The arithmetic is the tiled passes' (mj_tiled_impl.cuh): the spins are the
 // same bit for bit.  us per SIB step at 10 K, this against two launches: square
@@ -50,9 +55,11 @@ struct StepsArgs {
     int nsteps;
     uint32_t step0;
     unsigned long long* box;  // the tiles' boxes, zero at the launch
+    int mute;                 // 1: nothing is posted, so that every wait runs out (a test)
     int* status;
 };
 
+// looks after which a wait gives up, about a second
 constexpr uint32_t kStepsWaitPolls = 1u << 20;
 
 // The halo of a block's tile (TileGeom layout) and the boxes its cells come from.  A tile's box: [parity][word][kN]
@@ -67,7 +74,7 @@ struct TileRing {
     static_assert(G::TX == 32 && G::TY == kStepsTY, "box_index");
     int hpos[KH], hsrc[KH];  // a halo cell's place in the tile, its site in the layer (-1: none, or past an open edge)
     int hbox[KH];            // its place in the boxes
-    int obox[RY];            // the thread's sites' places in the tile's box (-1: not near the edge)
+    int obox[RY];            // the thread's sites' places in the tile's box (-1: not posted)
     unsigned long long* box;
 
     // place of site (lx, ly) of a w x h tile in its box: the first R rows, the last R, then the sides; -1 inside
@@ -80,7 +87,7 @@ struct TileRing {
     }
     // tile (bx, by) of the nx tiles a row of an Lx x Ly layer whose first box is number tile0
     __device__ __forceinline__ void init(const int* periodic, int Lx, int Ly, int bx, int by, int nx, int tile0,
-                                         unsigned long long* boxes) {
+                                         unsigned long long* boxes, int mute) {
         const int tid = threadIdx.x + 32 * threadIdx.y;
         const int x0 = bx * G::TX, y0 = by * G::TY;
         const int w = min(G::TX, Lx - x0), h = min(G::TY, Ly - y0);
@@ -124,7 +131,7 @@ struct TileRing {
         for (int r = 0; r < RY; ++r) {
             const int lx = threadIdx.x, ly = threadIdx.y * RY + r;
             const int b = lx < w && ly < h ? box_index(lx, ly, w, h) : -1;
-            obox[r] = b < 0 ? -1 : base_of(bx, by) + b;
+            obox[r] = b < 0 || mute ? -1 : base_of(bx, by) + b;
         }
     }
     // the halo cells of a layer of `src` (component stride N) into the tile
@@ -173,7 +180,7 @@ struct TileRing {
                                           __hiloint2double(half(5), half(4))));
         }
         if (__syncthreads_or(bad)) {
-            if (threadIdx.x == 0 && threadIdx.y == 0 && status) atomicOr(status, kStatusTimeout);
+            if (threadIdx.x == 0 && threadIdx.y == 0) atomicOr(status, kStatusTimeout);
             return false;
         }
         return true;
@@ -210,7 +217,7 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_steps(const __grid_constant_
     // cells across an open edge stay zero
     for (int q = tid; q < 3 * G::NS; q += NT) sm[q] = 0.0;
     TileRing<S, BYT, RY> ring;
-    ring.init(P.periodic, Lx, Ly, blockIdx.x, blockIdx.y, gridDim.x, gridDim.x * gridDim.y * z, A.box);
+    ring.init(P.periodic, Lx, Ly, blockIdx.x, blockIdx.y, gridDim.x, gridDim.x * gridDim.y * z, A.box, A.mute);
     const int x = x0 + static_cast<int>(threadIdx.x), yt = y0 + static_cast<int>(threadIdx.y) * RY;
     const int64_t i0 = layer * z + x + static_cast<int64_t>(Lx) * yt;
     const int base = static_cast<int>(threadIdx.y) * RY * G::PX + static_cast<int>(threadIdx.x);
@@ -457,6 +464,7 @@ mj_status steps_run(mj_plan* p, const StepsJob* job, const DynCoef& C, int* warp
     A.nsteps = job->nsteps;
     A.step0 = job->step0;
     A.box = job->box;
+    A.mute = p->mute_tiles ? 1 : 0;
     A.status = p->d_status;
     mj_status st = cuda_status(cudaMemsetAsync(job->box, 0, sizeof(unsigned long long) * 12 * steps_box_sites(S::R) * tiles, s),
                                "step boxes");
