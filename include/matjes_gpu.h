@@ -219,8 +219,10 @@ mj_status mj_plan_autotune(mj_plan* plan, const double* m_dev_soa, const mj_dyn_
  * MJ_ERR_TIMEOUT when a bounded device wait gave up since the last check (the
  * results of that launch are invalid), else MJ_ERR_NAN when a time step wrote a
  * non-finite spin component (the state is invalid from that step on).  The
- * asynchronous step calls (mj_step, mj_step_dev, mj_graph_run) leave the report
- * to this call; mj_step_host and mj_gneb_path return it themselves.  The
+ * asynchronous calls (mj_step, mj_step_dev, mj_graph_run, mj_adjoint_forward and
+ * mj_adjoint_backward) leave the report to this call, the energies of many-step
+ * launches and the gradients being NaN after a timeout; mj_step_host and
+ * mj_gneb_path return it themselves.  The
  * reference has no such report: its only check is the energy-increase warning of
  * dynamics/spindynamics.f90:376-381. */
 mj_status mj_plan_check_status(mj_plan* plan);
@@ -544,6 +546,12 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
  * these passes, two launches a step, always.  The spins are
  * the same bit for bit. */
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
+/* As mj_plan_check_status, for a batch (synchronises, then clears the report):
+ * MJ_ERR_TIMEOUT when a wait between the tiles of its many-step launches gave up
+ * since the last report.  mj_batch_download and mj_batch_energies report it
+ * themselves; the asynchronous calls (mj_batch_step, mj_batch_graph_run,
+ * mj_batch_field) leave it to this call, their energies being NaN until then. */
+mj_status mj_batch_check_status(mj_batch* b);
 /* Options of a batch, as mj_plan_set_option's: MJ_OPT_TEST_TIMEOUT. */
 mj_status mj_batch_set_option(mj_batch* b, int32_t option, int32_t value);
 /* Times `steps` steps of every (variant, blocks per SM in {2,4,8,16,32}) on the

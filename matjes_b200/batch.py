@@ -156,6 +156,11 @@ class ReplicaBatch:
         check(lib.mj_batch_temperatures(self.handle, ptr(T), ptr(acc)))
         return T, acc
 
+    def check_status(self) -> None:
+        """Raises when a launch of the asynchronous calls above failed on the device since
+        the last report (download and energies raise by themselves); synchronises."""
+        check(lib.mj_batch_check_status(self.handle))
+
     # -- Monte Carlo -------------------------------------------------------
     def monte_carlo(self, p: _abi.McParams, nrounds: int, sweeps_per_round: int = 1, swap: bool = True,
                     record: bool = True, stream=None):

@@ -755,6 +755,7 @@ struct mj_batch {
     std::vector<StepGroup> groups;    // empty: a replica is too large
     mj::BatchStepTile* d_step_tiles = nullptr;
     int* d_status = nullptr;          // kStatusTimeout of a bounded wait
+    int* h_status = nullptr;          // its pinned mirror
     bool mute_tiles = false;          // the many-step launches' tiles post nothing (a test of the waits)
     double* d_sigma = nullptr;        // per replica, of the current call's alpha and timestep
     int* d_image = nullptr;
@@ -796,6 +797,7 @@ void batch_free(mj_batch* b) {
     cudaFree(b->d_sigma);
     cudaFree(b->d_step_tiles);
     cudaFree(b->d_status);
+    cudaFreeHost(b->h_status);
     cudaFree(b->d_image);
     cudaFree(b->d_accept);
     cudaFree(b->d_stepctr);
@@ -1047,12 +1049,14 @@ mj_status batch_sequence(mj_batch* b, const DynCoef& c0, double dt, uint32_t ste
     return MJ_OK;
 }
 
-// MJ_ERR_TIMEOUT once when a bounded wait of a many-step launch gave up (synchronous).
-mj_status batch_status(const mj_batch* b) {
-    int word = 0;
-    mj_status st = cuda_status(cudaMemcpy(&word, b->d_status, sizeof(int), cudaMemcpyDeviceToHost), "batch status");
-    if (st != MJ_OK || word == 0) return st;
-    cudaMemset(b->d_status, 0, sizeof(int));
+// MJ_ERR_TIMEOUT once when a bounded wait of a many-step launch gave up, for the work that
+// stream s has done or waits for; synchronises s and no other stream.
+mj_status batch_status(const mj_batch* b, cudaStream_t s) {
+    mj_status st = cuda_status(cudaMemcpyAsync(b->h_status, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, s), "batch status");
+    if (st == MJ_OK) st = cuda_status(cudaStreamSynchronize(s), "batch status");
+    if (st != MJ_OK || *b->h_status == 0) return st;
+    cudaMemsetAsync(b->d_status, 0, sizeof(int), s);
+    if ((st = cuda_status(cudaStreamSynchronize(s), "batch status")) != MJ_OK) return st;
     return set_error(MJ_ERR_TIMEOUT, "a bounded device wait of the batch's steps gave up; its spins are invalid");
 }
 
@@ -1183,6 +1187,7 @@ mj_status mj_batch_create(const mj_lattice_desc* cell, const mj_hamiltonian_desc
     if ((st = dal(&b->d_m, f3, "batch m")) != MJ_OK ||
         (st = dal(&b->d_mid, std::max(f3, sizeof(unsigned long long) * words), "batch mid")) != MJ_OK ||
         (st = dal(&b->d_status, sizeof(int), "batch status")) != MJ_OK ||
+        (st = cuda_status(cudaMallocHost(&b->h_status, sizeof(int)), "batch status")) != MJ_OK ||
         (st = dal(&b->d_aux, f3, "batch aux")) != MJ_OK || (st = dal(&b->d_E, sizeof(double) * nrep, "batch E")) != MJ_OK ||
         (st = dal(&b->d_slot_kT, sizeof(double) * nrep, "batch ladder")) != MJ_OK ||
         (st = dal(&b->d_noise_tab, sizeof(double) * kNoiseTabDoubles, "batch tables")) != MJ_OK ||
@@ -1264,8 +1269,7 @@ mj_status mj_batch_download(const mj_batch* bc, double* m, void* stream) {
     if ((st = cuda_status(cudaMemcpyAsync(m, b->d_stage, sizeof(double) * 3 * b->Ntot, cudaMemcpyDeviceToHost, s),
                           "batch download")) != MJ_OK)
         return st;
-    if ((st = cuda_status(cudaStreamSynchronize(s), "batch download")) != MJ_OK) return st;
-    return batch_status(b);
+    return batch_status(b, s);
 }
 
 mj_status mj_batch_step(mj_batch* b, const mj_dyn_params* p, int32_t nsteps, int32_t swap_every, double* E_dev,
@@ -1341,7 +1345,14 @@ mj_status mj_batch_energies(mj_batch* b, double* E_host) {
     if ((st = cuda_status(cudaMemcpy(E_host, b->d_E, sizeof(double) * b->nrep, cudaMemcpyDeviceToHost), "batch energies")) !=
         MJ_OK)
         return st;
-    return batch_status(b);
+    return batch_status(b, 0);
+}
+
+mj_status mj_batch_check_status(mj_batch* b) {
+    if (!b) return set_error(MJ_ERR_ARG, "null batch");
+    cudaSetDevice(b->device);
+    const mj_status st = cuda_status(cudaDeviceSynchronize(), "status sync");
+    return st != MJ_OK ? st : batch_status(b, 0);
 }
 
 mj_status mj_batch_temperatures(const mj_batch* b, double* T_host, int32_t* accepted) {

@@ -116,6 +116,12 @@ class Hamiltonian:
     def energy_distrib(self, m):
         return self.get_eff_field(m, with_energy=True)[1]
 
+    def check_status(self) -> None:
+        """Raises when a launch of an asynchronous call (steps of a CUDA tensor, a
+        trajectory's forward or backward) reported a timeout or a non-finite spin since
+        the last check; synchronises."""
+        check(lib.mj_plan_check_status(self.plan))
+
     def energy(self, m) -> float:
         st = SpinState(self, m)
         E = C.c_double()
@@ -216,8 +222,9 @@ class SpinDynamics:
 
     def run(self, m, nsteps: int, energies: bool = False, step0: Optional[int] = None):
         """Advance `m` by nsteps.  Host (N,3) arrays are updated in place through
-        mj_step_host; CUDA (3,N) tensors in place through mj_step_dev.  Returns
-        the per-step energies (after each step) when asked."""
+        mj_step_host; CUDA (3,N) tensors in place through mj_step_dev, without
+        waiting for them (Hamiltonian.check_status tells of failures on the device).
+        Returns the per-step energies (after each step) when asked."""
         if step0 is not None:
             self.p.step0 = int(step0)
         if _is_torch(m):
