@@ -139,8 +139,9 @@ mj_status mj_plan_noffsets(const mj_plan* plan, int32_t* n);
  * otherwise.  A plan left at its default runs calls of two or more steps on a
  * lattice whose tiles are all resident at once (about 300,000 sites, no dipolar
  * term) as one launch of many steps; setting a variant makes it run that
- * variant's launches, one per pass.  The spins are the same bit for bit.  No
- * counterpart in the reference (its SpMV has no tiling). */
+ * variant's launches, one per pass, until MJ_OPT_MANY_STEPS is set to 1 again.
+ * The spins are the same bit for bit.  No counterpart in the reference (its SpMV
+ * has no tiling). */
 mj_status mj_plan_set_variant(mj_plan* plan, int32_t variant);
 /* Current variant (-1 generic) and the matched compile-time shape id (0 none). */
 mj_status mj_plan_get_variant(const mj_plan* plan, int32_t* variant, int32_t* shape);
@@ -158,7 +159,9 @@ mj_status mj_plan_set_tma(mj_plan* plan, int32_t enable);
  * same bit for bit.  No counterpart in the reference. */
 mj_status mj_plan_set_fused(mj_plan* plan, int32_t enable);
 /* Kernel options of a stencil plan (none changes a result, every one only how
- * it is computed; no counterpart in the reference):
+ * it is computed; no counterpart in the reference).  The options of the passes
+ * (TMA, PDL, STORE_DRAW, BLOCKS_PER_SM) matter where passes run: not to the
+ * many-step launches, which MJ_OPT_MANY_STEPS 0 or a chosen variant turns off.
  *   MJ_OPT_TMA, MJ_OPT_FUSED   as mj_plan_set_tma / mj_plan_set_fused;
  *   MJ_OPT_PDL (default 1)     tiled passes launched as programmatic dependents
  *                              of the kernel before them: the next pass launches
@@ -188,6 +191,13 @@ mj_status mj_plan_set_fused(mj_plan* plan, int32_t enable);
  *   MJ_OPT_HOST_ZEROCOPY (default 1)  striped mj_step_host with a mapped pinned
  *                              buffer: kernels write the stepped spins into it
  *                              directly (0: device transposes and copies);
+ *   MJ_OPT_MANY_STEPS (default 1)  calls of several steps in one launch where
+ *                              all tiles are resident at once (adjoint sweeps
+ *                              too); 0: the launches of the passes.  A many-step
+ *                              launch takes the SMs that its tiles fill until it
+ *                              ends: 2 plans of 256^2 side by side on two streams
+ *                              8.3 us a step of both (passes 17.2), 8 plans 32
+ *                              (passes from graphs 27);
  *   MJ_OPT_TEST_TIMEOUT (default 0)  1: the tiles of the many-step launches post
  *                              nothing to each other, so that every wait between
  *                              them runs out (about a second a launch): a test of
@@ -204,7 +214,8 @@ enum {
     MJ_OPT_BLOCKS_PER_SM = 5,
     MJ_OPT_DIP_ZCONV = 6,
     MJ_OPT_HOST_ZEROCOPY = 7,
-    MJ_OPT_TEST_TIMEOUT = 8
+    MJ_OPT_TEST_TIMEOUT = 8,
+    MJ_OPT_MANY_STEPS = 9
 };
 mj_status mj_plan_set_option(mj_plan* plan, int32_t option, int32_t value);
 /* Autotuner: times `steps` steps of `p` for every kernel configuration of the
@@ -543,7 +554,8 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
  * resident at once (when each replica alone fits: about 300,000 sites), where there
  * are enough steps between two swap rounds to pay for the groups' launches (one to
  * five, more where the groups are half full); setting a configuration makes it run
- * these passes, two launches a step, always.  The spins are
+ * these passes, two launches a step, always (until MJ_OPT_MANY_STEPS is set to 1
+ * again).  The spins are
  * the same bit for bit. */
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
 /* As mj_plan_check_status, for a batch (synchronises, then clears the report):
@@ -552,7 +564,8 @@ mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_s
  * themselves; the asynchronous calls (mj_batch_step, mj_batch_graph_run,
  * mj_batch_field) leave it to this call, their energies being NaN until then. */
 mj_status mj_batch_check_status(mj_batch* b);
-/* Options of a batch, as mj_plan_set_option's: MJ_OPT_TEST_TIMEOUT. */
+/* Options of a batch, as mj_plan_set_option's: MJ_OPT_MANY_STEPS and
+ * MJ_OPT_TEST_TIMEOUT. */
 mj_status mj_batch_set_option(mj_batch* b, int32_t option, int32_t value);
 /* Times `steps` steps of every (variant, blocks per SM in {2,4,8,16,32}) on the
  * current state (restored afterwards), keeps the fastest; ms_table (25 doubles,

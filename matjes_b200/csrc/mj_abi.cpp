@@ -1212,6 +1212,7 @@ mj_status mj_plan_set_option(mj_plan* plan, int32_t option, int32_t value) {
         }
         case MJ_OPT_HOST_ZEROCOPY: plan->host_zerocopy = value != 0; break;
         case MJ_OPT_TEST_TIMEOUT: plan->mute_tiles = value != 0; break;
+        case MJ_OPT_MANY_STEPS: plan->steps_together = value != 0; break;
         case MJ_OPT_BLOCKS_PER_SM: {
             if (value != 0 && (value < 4 || value > 32))
                 return set_error(MJ_ERR_ARG, "blocks per SM must be 0 or in [4, 32]");

@@ -1427,6 +1427,7 @@ mj_status mj_batch_set_option(mj_batch* b, int32_t option, int32_t value) {
     if (!b) return set_error(MJ_ERR_ARG, "null batch");
     switch (option) {
         case MJ_OPT_TEST_TIMEOUT: b->mute_tiles = value != 0; break;
+        case MJ_OPT_MANY_STEPS: b->together = value != 0; break;
         default: return set_error(MJ_ERR_ARG, "unknown batch option " + std::to_string(option));
     }
     b->graph_key.clear();
