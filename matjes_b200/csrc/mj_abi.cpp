@@ -346,7 +346,6 @@ mj_status alloc_scratch(mj_plan* p) {
     if ((st = dalloc(&p->d_mid, std::max(3 * N, words), "mid")) != MJ_OK) return st;
     p->aux_doubles = std::max<int64_t>(3 * N, tiles > 0 ? kStepsAuxDoubles : 0);
     if ((st = dalloc(&p->d_aux, p->aux_doubles, "aux")) != MJ_OK) return st;
-    if ((st = dalloc(&p->d_aux2, 3 * N, "aux2")) != MJ_OK) return st;
     if (tiles > 0 && p->aux_doubles >= 2 * 8 * tiles)  // room for two slots of energies
         p->d_steps_box = reinterpret_cast<unsigned long long*>(p->d_mid);
     // generic grid, or the smallest tile of the tiled kernels (32 x 8), whichever has more blocks

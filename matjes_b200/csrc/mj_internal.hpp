@@ -184,7 +184,7 @@ struct mj_plan {
     // scratch
     double* d_mid = nullptr;         // 3N
     double* d_aux = nullptr;         // 3N (Heun: the predictor's D1/2 + DT; SIB: its draw)
-    double* d_aux2 = nullptr;        // 3N (minimisation velocities)
+    double* d_aux2 = nullptr;        // 3N (minimisation velocities; made by the first mj_minimize)
     double* d_field = nullptr;       // 3N (field scratch)
     double* d_partials = nullptr;    // per-block energy partials
     unsigned int* d_counter = nullptr;

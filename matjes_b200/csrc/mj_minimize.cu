@@ -179,6 +179,7 @@ mj_status mj_minimize(mj_plan* plan, double* m, const mj_min_params* p, int64_t 
     const size_t f3 = sizeof(double) * 3 * static_cast<size_t>(N);
     mj_status st;
     if (!plan->d_field && (st = cuda_status(cudaMalloc(&plan->d_field, f3), "field scratch")) != MJ_OK) return st;
+    if (!plan->d_aux2 && (st = cuda_status(cudaMalloc(&plan->d_aux2, f3), "velocities")) != MJ_OK) return st;
     MinState* d_S = nullptr;
     if ((st = cuda_status(cudaMalloc(&d_S, sizeof(MinState)), "minimiser state")) != MJ_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
