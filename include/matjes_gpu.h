@@ -560,8 +560,8 @@ mj_status mj_gneb_path(mj_plan* plan, double* m_dev_images, int32_t nimg, const 
 mj_status mj_batch_set_config(mj_batch* b, int32_t variant, int32_t blocks_per_sm);
 /* As mj_plan_check_status, for a batch (synchronises, then clears the report):
  * MJ_ERR_TIMEOUT when a wait between the tiles of its many-step launches gave up
- * since the last report.  mj_batch_download and mj_batch_energies report it
- * themselves; the asynchronous calls (mj_batch_step, mj_batch_graph_run,
+ * since the last report.  mj_batch_download, mj_batch_energies and
+ * mj_batch_gneb_path (before it starts) report it themselves; the asynchronous calls (mj_batch_step, mj_batch_graph_run,
  * mj_batch_field) leave it to this call, their energies being NaN until then. */
 mj_status mj_batch_check_status(mj_batch* b);
 /* Options of a batch, as mj_plan_set_option's: MJ_OPT_MANY_STEPS and

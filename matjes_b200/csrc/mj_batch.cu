@@ -288,7 +288,9 @@ __global__ void __launch_bounds__(32 * BYT, MINB) k_batch(const __grid_constant_
 // two swap rounds.  us per step, this against the passes: 4 replicas (44 k sites) 4.1 /
 // 13.5, 16 (324 k) 15.0 / 24.8, 64 (1.4 M) 53 / 72, 256 (5.07 M) 188 / 238: small
 // batches were bound by two launches a step, large ones by the corrector's HBM
-// traffic; now instruction issue (37 ps per site and step).
+// traffic; now half by instruction issue (0.48 of the schedulers' cycles), half by the
+// exchanges (per instruction 5.8 cycles waiting for memory, 3.1 at barriers): 37 ps
+// per site and step.
 struct BatchStepTile {
     int64_t off;      // first packed site of the replica
     int Lx, Ly;
@@ -1647,6 +1649,7 @@ mj_status mj_batch_gneb_path(mj_batch* b, const mj_gneb_params* p, double* rx, d
     fl.tile_g = b->d_tile_g;
     // the path as the work queued on the legacy default stream (an upload) leaves it
     st = cuda_status(cudaStreamSynchronize(0), "GNEB start");
+    if (st == MJ_OK) st = batch_status(b, 0);  // images that a timed-out launch left are no path
     if (st == MJ_OK)
         st = gneb_relax(fl, b->gneb, b->d_m, nrep, GnebIdx{n, n, Ntot}, b->num_sms, b->cap_stream, p, 32, rx, ene, dene,
                         iterations, max_force, climbing);

@@ -50,3 +50,16 @@ def test_download_reports_for_its_stream():
     assert _abi.lib.mj_batch_download(b.handle, out.ctypes.data, s.cuda_stream) == _abi.MJ_ERR_TIMEOUT
     b.check_status()
     assert _abi.lib.mj_batch_download(b.handle, out.ctypes.data, s.cuda_stream) == _abi.MJ_OK
+
+
+def test_a_path_is_not_relaxed_from_invalid_images():
+    import matjes_b200 as mj
+
+    b = mj.ReplicaBatch(mj.square_film((8, 8, 1)), [(16, 16)] * 4, np.zeros((4, 3)), [1.0] * 4)
+    m = mj.random_sphere(b.N, 2)
+    b.upload(m)
+    _time_out(b)
+    with pytest.raises(mj.MatjesError, match="bounded device wait"):
+        b.gneb_path(0.3, 0.02, 1.0, 0.0, 5, "I")
+    b.upload(m)
+    assert b.gneb_path(0.3, 0.02, 1.0, 0.0, 5, "I")[3] == 5
