@@ -261,8 +261,10 @@ __global__ void __launch_bounds__(256) k_zconv(const double2* __restrict__ in, d
 // distance dz one load of K's six components serves the pairs (z, z - dz) and
 // (z, z + dz) of all of them, the next distance's K in flight meanwhile (holding
 // a block's K in shared memory instead measured slower, 16.7 against 14.9 us at
-// 16 planes of 128 x 65 columns).  Bound by FP64 (36 fma a pair, Lz^2 pairs a
-// column) and the shared memory reads behind them.
+// 16 planes of 128 x 65 columns).  Bound by the latency of K's loads behind few warps
+// (13 planes of 128 x 65 columns: 0.34 of the issue slots, FP64 pipe 0.24, 22 % of the
+// warps, 4.3 cycles waiting for memory per instruction; 36 fma a pair, Lz^2 pairs a
+// column), on large planes by the bytes of K.
 enum ZdirMode { kZdirMirror = 0, kZdirOpen = 1, kZdirCircular = 2 };
 constexpr int kZdirMax = 16;  // planes: two per warp, the spectra in 24 KB of shared memory
 // Whether the direct sum is taken for lz planes of pc columns; `even`: K(-r) = K(r)
@@ -282,10 +284,10 @@ constexpr int kZdirMax = 16;  // planes: two per warp, the spectra in 24 KB of s
 //   open (third vector not normal), pow2: 2 planes 96^2 in x, y periodic 33 / 35, 256^2 40.4 /
 //     39.3, 4 planes 64^2 32.2 / 31.5; else: 3 planes 256^2 104 / 107, 5 planes 128^2 55 / 60,
 //     192^2 137 / 131, 7 planes 192^2 180 / 190, 9 planes 96^2 68 / 64; uneven 6 planes 256^2
-//     75 / 79, 384^2 170 / 165, 11 planes 128^2 53 / 61, 9 planes 192^2 74 / 72
+//     75 / 79, 384^2 170 / 165, 11 planes 128^2 53 / 61, 192^2 84 / 92, 9 planes 192^2 74 / 72
 //   circular, pow2: 4 planes 192^2 41.6 / 41.6, 384^2 100 / 95, 8 planes 128^2 41.5 / 39.5;
 //     else: 3 planes 384^2 84 / 86, 512^2 97.7 / 96.0, 9 planes 192^2 60.6 / 61.1,
-//     5 planes 256^2 56.8 / 54.9, 12 planes 192^2 75.5 / 71.6
+//     5 planes 256^2 56.8 / 54.9, 12 planes 192^2 75.5 / 71.6, 14 192^2 87 / 91, 256^2 132 / 124
 // One plane has no z part to transform: the real product is never slower (1024^2 open
 // 348 us, 473 by the direct sum's complex K).
 bool zdirect_pays(int mode, int lz, int64_t pc, bool even, bool pow2) {
@@ -297,10 +299,11 @@ bool zdirect_pays(int mode, int lz, int64_t pc, bool even, bool pow2) {
     }
     if (mode == kZdirOpen) {
         if (pow2) return lz <= 2 && pc <= 20000;
-        return lz == 3 || lz == 7 || (lz <= 7 && w <= (even ? 170000 : 400000)) || (lz <= 11 && pc <= 10000);
+        return lz == 3 || lz == 7 || (lz <= 7 && w <= (even ? 170000 : 400000)) || (lz <= 11 && pc <= 10000) ||
+               ((lz == 11 || lz == 13) && pc > 4000 && pc <= (even ? 20000 : 40000));
     }
     if (pow2) return lz <= 4 && pc <= 20000;
-    return lz <= 3 ? pc <= 100000 : w <= 160000;
+    return lz <= 3 ? pc <= 100000 : w <= 160000 || (lz == 14 && pc <= 20000);
 }
 
 struct KSix {
@@ -546,20 +549,25 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
     const int sel[6] = {0, 1, 2, 4, 5, 8};
     for (int c = 0; c < 6; ++c)
         for (int64_t q = 0; q < nk; ++q) k6[static_cast<size_t>(c) * nk + q] = K[static_cast<size_t>(q) * 9 + sel[c]];
-    // K's symmetries, checked value by value: the mirror in z (open axis), and K(-r) = K(r)
-    bool mirror = nz >= 2 * d->lz, even = true;
-    for (int c = 0; c < 6 && mirror; ++c) {
-        const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
-        for (int z = 1; z < d->lz && mirror; ++z) {
-            const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
-            const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
-            for (int64_t q = 0; q < d->pr && mirror; ++q) mirror = a[q] == sg * b[q];
+    // K's symmetries where the choice depends on them: the mirror in z (open axis), value by
+    // value, and K(-r) = K(r)
+    auto pays = [&](int mode, bool even) { return zdirect_pays(mode, d->lz, d->pc, even, pow2); };
+    auto mirrored = [&]() {
+        for (int c = 0; c < 6; ++c) {
+            const double sg = (c == 2 || c == 4) ? -1.0 : 1.0;
+            for (int z = 1; z < d->lz; ++z) {
+                const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr];
+                const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(nz - z) * d->pr];
+                for (int64_t q = 0; q < d->pr; ++q)
+                    if (a[q] != sg * b[q]) return false;
+            }
         }
-    }
-    if (d->lz >= 2 && d->lz <= kZdirMax) {
+        return true;
+    };
+    auto is_even = [&]() {  // (from two planes: it decides the route's speed alone)
         double top = 0.0, odd = 0.0;
         for (int c = 0; c < 6; ++c)
-            for (int z = 0; z < nz; ++z)
+            for (int z = 0; z < std::min(nz, 2); ++z)
                 for (int y = 0; y < ny; ++y) {
                     const double* a = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>(z) * d->pr + static_cast<size_t>(y) * nx];
                     const double* b = &k6[static_cast<size_t>(c) * nk + static_cast<size_t>((nz - z) % nz) * d->pr +
@@ -569,10 +577,14 @@ mj_status dipolar_create(mj_plan* p, const std::vector<double>& K, cudaStream_t 
                         odd = std::max(odd, std::fabs(a[x] - b[x == 0 ? 0 : nx - x]));
                     }
                 }
-        even = odd <= 1e-12 * top;
+        return odd <= 1e-12 * top;
+    };
+    int zmode = kZdirCircular;
+    if (nz >= 2 * d->lz) {
+        const bool either = pays(kZdirMirror, true) || pays(kZdirMirror, false) || pays(kZdirOpen, true) || pays(kZdirOpen, false);
+        zmode = either && mirrored() ? kZdirMirror : kZdirOpen;
     }
-    const int zmode = nz >= 2 * d->lz ? (mirror ? kZdirMirror : kZdirOpen) : kZdirCircular;
-    const bool direct = zdirect_pays(zmode, d->lz, d->pc, even, pow2);
+    const bool direct = pays(zmode, true) == pays(zmode, false) ? pays(zmode, true) : pays(zmode, is_even());
     const int planes = direct && zmode == kZdirMirror ? d->lz : nz;  // of K that are transformed
     {
         double* d_k6 = nullptr;
