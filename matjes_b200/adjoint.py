@@ -8,7 +8,8 @@ sign) and the per-site applied field ``bfield`` ((3, N) T, or None for the
 deck's uniform field).  The forward map is the reference's dynamics loop
 (dynamics/spindynamics.f90:282-313) with the SIB scheme of Mentink et al.
 (2010); the backward sweep is the hand-written transpose in mj_adjoint.cu,
-with checkpoints every ``checkpoint_every`` steps.
+with checkpoints every ``checkpoint_every`` steps.  Both sweeps are asynchronous:
+a device wait that ran out leaves NaN gradients, and ``ham.check_status()`` tells.
 """
 from __future__ import annotations
 

@@ -578,7 +578,7 @@ constexpr int kTBYT = 8, kTRY = 1;
 // segment to the next and reduced over the grid once, after the last (so the
 // sums do not depend on the checkpoint spacing).  m_n and mb of a step come from the recomputed segment, so
 // their tiles, the two fields and the draw are ready before the wait.
-// Bound by the chain of its two exchanges: 256^2 square, 3 terms, 7.5 us a step,
+// Bound by the chain of its two exchanges (0.34 of the issue slots): 256^2 square, 3 terms, 7.5 us a step,
 // 21.6 us with the two launches (10.9 + 10.7); a forward and backward sweep of
 // 200 steps with checkpoints every 50 10.0 -> 3.4 ms.
 struct SegArgs {

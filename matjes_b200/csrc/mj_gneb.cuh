@@ -595,12 +595,16 @@ mj_status gneb_relax(Fields& fl, GnebWork& W, double* m, int nrep, GnebIdx X, in
         // Forces and spins alternate between their two buffers (an even chunk
         // starts on F1 and mB).  Two chunks are in flight: the stop flag of one
         // is read while the next runs; after the stop every kernel returns at
-        // once, and no iteration past itrmax is queued.  A run of more than four
+        // once (but a plan's field passes that are launched image by image), and no
+        // iteration past itrmax is queued.  A run of more than four
         // chunks replays a chunk as one graph; a shorter one launches its
         // kernels directly (capturing and instantiating the graph queues as many
         // launches as the chunk has).  40 iterations of 256^2 x 16 images: 3.7 ms
         // a call, 8.8 to 12.3 ms with the graph, every buffer allocated per call
-        // and two chunks always queued.
+        // and two chunks always queued.  The line is that of a few launches an
+        // iteration; with a launch per image and forked streams the graph would pay
+        // from about two chunks (8 images of a dipolar 32^2 x 4 film, us an iteration:
+        // 40 316, 128 303, 129 by the graph 228; never above the earlier 684, 340, 390).
         // Four sites per thread once that still gives two blocks per SM: the
         // loads of four sites in flight before each block's reduction.
         const bool spt4 = Ntot >= 2LL * 1024 * num_sms;

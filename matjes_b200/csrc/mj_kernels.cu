@@ -108,8 +108,9 @@ struct StencilField {
 // SP_AXIAL (as in mj_tiled_impl.cuh): the in-plane tensors have W[0][1] = W[1][0]
 // = 0, the z bonds are isotropic, the on-site tensor is its zz entry alone.  The
 // neighbours are added in the order of the plan's offsets, so the field is the
-// offset loop's bit for bit.  Bound by instruction issue and the L2 (the
-// neighbouring rows and layers come from there).  96 x 96 x 97 periodic at 10 K:
+// offset loop's bit for bit.  Bound by instruction issue (0.66 of the
+// slots in the predictor, 0.55 in the corrector) and the latency of its loads (the
+// neighbouring rows and layers come from the L2).  96 x 96 x 97 periodic at 10 K:
 // a SIB step 47.2 us with the energy, 78.3 with the offset loop and a second draw
 // (passes 25.6 + 17.9 us against 41.9 + 31.8).  Held to 48 registers for five
 // resident blocks: 47.5 us at the four that 58 allow.
@@ -259,9 +260,10 @@ struct EllField : EllSites {
     }
 };
 
-// The entries by tensor id.  Bound by its loads: 4 bytes per entry instead of
-// the general form's 76, the tensors copied to shared memory once per block
-// (the lanes of a warp read at most one tensor per atom of the cell).
+// The entries by tensor id.  Bound by the latency of its gathers (11 to 13 cycles
+// waiting for memory per instruction, 0.42 / 0.36 of the issue slots): 4 bytes per
+// entry instead of the general form's 76, the tensors copied to shared memory once per
+// block (the lanes of a warp read at most one tensor per atom of the cell).
 // 384 x 384 cells of two atoms, 9 entries a site: a SIB step 38.9 us, 109.0 us
 // with the general form (passes 18.4 + 15.5 us against 56.7 + 42.3); 35.6 us since
 // the corrector reads the predictor's draw, 33.6 at five resident blocks.

@@ -30,8 +30,10 @@
 // 16^2 3.1 / 10.6, 64^2 3.2 / 10.3, 256^2 4.0 / 11.6, 512^2 10.3 / 15.5;
 // triangular, three shells, 64^2 3.7 / 12.6, 256^2 4.9 / 13.4, 512^2 12.2 / 18.3
 // (with a release, a counter and a load per exchange 4.9 at 64^2, 6.6 at 256^2).
-// What bounds it: up to 256^2 the chain post - poll - pass, 1.6 to 2 us a pass;
-// at 512^2 instruction issue (39 ps per site and step).
+// What bounds it: the chain post - poll - pass, 1.6 to 2 us a pass up to 256^2.  At
+// 512^2 (39 ps per site and step) still half of it: the schedulers issue in 0.51 of
+// their cycles (0.33 at 256^2), per instruction a warp waits 4.4 cycles for memory
+// (polls and halo) and 2.7 at the barriers.
 #pragma once
 
 #include "mj_tiled_impl.cuh"
